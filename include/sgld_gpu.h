@@ -165,9 +165,9 @@ int sgld_kbyu_tile(const sgld_ctx *ctx, int *tile_x, int *z_chunk);
  * (other streams, other contexts on the same device) race; serialise them.
  * The call uploads no constants: if the device holds another context's
  * element matrix, it returns SGLD_ERR_STATE, and any other call on this
- * context binds the matrix again.  Grids needing more than
- * SGLD_NOALLOC_MAX_CTAS CTAs (on the order of 1e8 nodes; each CTA covers a
- * 31 x 7 x 16 node block) are rejected with SGLD_ERR_ARG. */
+ * context binds the matrix again.  Grids of more than SGLD_NOALLOC_MAX_CTAS
+ * blocks of 31 x 7 x 16 nodes (on the order of 1e8 nodes) are rejected with
+ * SGLD_ERR_ARG. */
 #define SGLD_NOALLOC_MAX_CTAS 32768
 int sgld_kbyu_dot_noalloc(sgld_ctx *ctx, const double *d_u, double *d_y, double *d_dot, void *stream);
 

@@ -1,0 +1,397 @@
+// FP64 matrix-free K*u of the finest level in sum-factorised Hadamard form
+// (reference: src/MEXfuncs/Solving_KbyU_MatrixFree_mex.cpp:53-138).
+//
+// GB300 issues about two FP64 operations per clock and SM, so the operator is
+// bound by the number of FP64 instructions and by nothing else: 238 MB of
+// vectors on the 256 x 128 x 128 grid take 35 us of HBM time, 137 operations
+// per element 0.94 ms of FP64 time.  The kernel therefore forms every partial
+// result once and lets the elements around it share it through shared memory:
+//   * the y butterfly of an edge along y (4 elements share it): 6 operations;
+//   * the x butterfly of a face in a node layer (2 elements): 12;
+//   * per element the z butterfly (21: the three rigid translations are not
+//     needed), E * Kh in the 8-value form of a cubic-symmetric element matrix
+//     (8 + 33), the z butterfly undone and added to what the element layer
+//     below carried up (30), the x butterfly undone (12);
+//   * the two faces of an edge add (6), the y butterfly is undone (6) and the
+//     two edges of a node add (3).
+// The form before it applied the three butterflies per element: 234
+// operations, on a fixed 32 x 8 tile whose halo and ragged edges made 1.43
+// threads per node of that grid.  sgld_kbyu_device (with its scatter and
+// gather) went from 2.85 to 1.52 ms on 256 x 128 x 128 and from 302 to 71 us on
+// 64 x 32 x 32, where the fixed tile filled 60 of 152 SMs.
+//
+// A CTA owns (ye-1) x (xe-1) node columns and marches through zc node layers;
+// thread t handles the element column t % ye, t / ye of its ye x xe element
+// tile.  Any ye and xe will do, as both exchanges go through shared memory, so
+// the tile is chosen to fit the grid (kbyu64_pick_tile).
+#include "sgld_internal.cuh"
+
+namespace sgld {
+
+// Hadamard-basis element matrix (sgld_internal.cuh), and its 8-value form
+// A-B, B, C, D, E, F-G, G, H (KH_CLASS in kernels_stencil.cu)
+__constant__ double c_kh64[KH_NNZ];
+__constant__ double c_kc64[8];
+
+void upload_kh64(const double *Kh, const double *kc, cudaStream_t s) {
+    cudaMemcpyToSymbolAsync(c_kh64, Kh, sizeof(double) * KH_NNZ, 0, cudaMemcpyHostToDevice, s);
+    cudaMemcpyToSymbolAsync(c_kc64, kc, sizeof(double) * 8, 0, cudaMemcpyHostToDevice, s);
+}
+
+namespace k64 {
+constexpr int MAX_THREADS = 384;   // at 168 registers a thread
+constexpr int STAGE = 5;           // staged words per thread and node layer, at most
+constexpr int SLOTS = 3;           // node layers in shared memory
+
+__host__ __device__ constexpr int threads(int ye, int xe) { return (ye * xe + 31) & ~31; }
+constexpr int node_words(int ye, int xe) { return 3 * (ye + 1) * (xe + 1); }
+constexpr size_t smem(int ye, int xe) {   // node ring, edge, face and node exchanges
+    return sizeof(double) * ((size_t)SLOTS * node_words(ye, xe) + 6 * ye * (xe + 1) + 9 * ye * xe);
+}
+}  // namespace k64
+
+// h <- E Kh h without the translations h[0..2]; k holds E times the 8 values
+__device__ __forceinline__ void kh_cubic_f64(double (&h)[24], const double (&k)[8]) {
+#define Y3(i, j, l, a, b)                             \
+    {                                                 \
+        const double t = k[b] * ((h[i] + h[j]) + h[l]); \
+        h[i] = fma(k[a], h[i], t);                    \
+        h[j] = fma(k[a], h[j], t);                    \
+        h[l] = fma(k[a], h[l], t);                    \
+    }
+#define YC(i, j) h[i] = h[j] = k[2] * (h[i] + h[j]);
+#define YD(i, j)                             \
+    {                                        \
+        const double a = h[i], b = h[j];     \
+        h[i] = fma(k[4], b, k[3] * a);       \
+        h[j] = fma(k[4], a, k[3] * b);       \
+    }
+    Y3(3, 7, 14, 0, 1)
+    YC(4, 6)
+    YC(5, 12)
+    YC(8, 13)
+    YD(9, 20)
+    YD(10, 17)
+    Y3(11, 16, 18, 5, 6)
+    YD(15, 19)
+    h[21] *= k[7];
+    h[22] *= k[7];
+    h[23] *= k[7];
+#undef Y3
+#undef YC
+#undef YD
+}
+
+// the same for any element matrix with the hexahedral block pattern
+__device__ __forceinline__ void kh_general_f64(double (&h)[24], double e) {
+#define Z3(i, j, l, o)                                                                     \
+    {                                                                                      \
+        const double a = e * h[i], b = e * h[j], d = e * h[l];                             \
+        h[i] = fma(c_kh64[o + 2], d, fma(c_kh64[o + 1], b, c_kh64[o] * a));                \
+        h[j] = fma(c_kh64[o + 5], d, fma(c_kh64[o + 4], b, c_kh64[o + 3] * a));            \
+        h[l] = fma(c_kh64[o + 8], d, fma(c_kh64[o + 7], b, c_kh64[o + 6] * a));            \
+    }
+#define Z2(i, j, o)                                               \
+    {                                                             \
+        const double a = e * h[i], b = e * h[j];                  \
+        h[i] = fma(c_kh64[o + 1], b, c_kh64[o] * a);              \
+        h[j] = fma(c_kh64[o + 3], b, c_kh64[o + 2] * a);          \
+    }
+    Z3(3, 7, 14, 0)
+    Z2(4, 6, 9)
+    Z2(5, 12, 13)
+    Z2(8, 13, 17)
+    Z2(9, 20, 21)
+    Z2(10, 17, 25)
+    Z3(11, 16, 18, 29)
+    Z2(15, 19, 38)
+    h[21] *= c_kh64[42] * e;
+    h[22] *= c_kh64[43] * e;
+    h[23] *= c_kh64[44] * e;
+#undef Z3
+#undef Z2
+}
+
+__device__ __forceinline__ void copy_word(double *dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+// y = K u on the full grid; y is 0 at fixed DOFs and at inactive nodes.  When
+// DOT, also writes sum(u .* y) of this CTA's nodes to partial[block].
+// tiles: the CTAs' activity map for this tile (0: no active element in the
+// CTA's box, so all it owns is zero), or null.
+template <bool DOT, bool CUBIC>
+__global__ void __launch_bounds__(k64::MAX_THREADS, 1)
+    k_kbyu64(const double *__restrict__ u, double *__restrict__ y, const double *__restrict__ E,
+             const uint8_t *__restrict__ nflag, int ny, int nx, int nz, int ye, int xe, int zc,
+             double *__restrict__ partial, const uint8_t *__restrict__ tiles) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int tn = ye * xe, te = ye * (xe + 1), nw = k64::node_words(ye, xe);
+    double *su = reinterpret_cast<double *>(smem_raw);   // [SLOTS][nw] node layers
+    double *se = su + k64::SLOTS * nw;                   // [6][te] y butterflies of the edges of a node layer
+    double *sl = se + 6 * te;                            // [6][tn] left face shares of the edges
+    double *sn = sl + 6 * tn;                            // [3][tn] upper shares of the nodes
+    const int ly = tid % ye, lx = tid / ye;
+    const bool elem = tid < tn;
+    const int NY = ny + 1, NX = nx + 1, NZ = nz + 1;
+    const int y0 = blockIdx.x * (ye - 1), x0 = blockIdx.y * (xe - 1), z0 = blockIdx.z * zc;
+    const int zend = min(z0 + zc, NZ);
+    const int gy = y0 + ly, gx = x0 + lx;   // the node this thread completes: local (ly+1, lx+1)
+    const bool owner = elem && ly < ye - 1 && lx < xe - 1 && gy < NY && gx < NX;
+    const int64_t plane = (int64_t)NY * NX, slot = blockIdx.x + gridDim.x * (blockIdx.y + (int64_t)gridDim.y * blockIdx.z);
+    if (tiles && !tiles[slot]) {
+        if (owner)
+            for (int z = z0; z < zend; ++z) {
+                double *o = y + 3 * (gy + (int64_t)NY * gx + plane * z);
+                o[0] = o[1] = o[2] = 0.0;
+            }
+        if (DOT && tid == 0) partial[slot] = 0.0;
+        return;
+    }
+    // this thread's words of a node layer: offsets in the layer, -1 past the grid, -2 none
+    int off[k64::STAGE];
+#pragma unroll
+    for (int k = 0; k < k64::STAGE; ++k) {
+        const int i = tid + k * nt;
+        off[k] = -2;
+        if (i < nw) {
+            const int node = i / 3, c = i - 3 * node, ny_ = node % (ye + 1), nx_ = node / (ye + 1);
+            const int py = y0 - 1 + ny_, px = x0 - 1 + nx_;
+            off[k] = (py >= 0 && py < NY && px >= 0 && px < NX) ? 3 * (py + NY * px) + c : -1;
+        }
+    }
+    auto stage = [&](int z) {   // node layer z into slot z mod 3
+        double *dst = su + (z + 3) % k64::SLOTS * nw;
+        const double *src = u + 3 * plane * z;
+        const bool zin = z >= 0 && z < NZ;
+#pragma unroll
+        for (int k = 0; k < k64::STAGE; ++k) {
+            const int i = tid + k * nt;
+            if (off[k] == -2) continue;
+            if (zin && off[k] >= 0)
+                copy_word(dst + i, src + off[k]);
+            else
+                dst[i] = 0.0;
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    // y butterflies of the edges of node layer z: sum and u(ly) - u(ly+1)
+    auto edges = [&](int z) {
+        if (!elem) return;
+        const double *p = su + (z + 3) % k64::SLOTS * nw + 3 * (ly + (ye + 1) * lx);
+        for (int x = lx;; ++x, p += 3 * (ye + 1)) {   // the last column's threads also form the column past it
+            double *o = se + ly + ye * x;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                o[c * te] = p[c] + p[3 + c];
+                o[(3 + c) * te] = p[c] - p[3 + c];
+            }
+            if (lx < xe - 1 || x == xe) break;
+        }
+    };
+    // the 12 face coefficients (index 3 (bx | by << 1) + c) of this element column
+    auto faces = [&](double (&F)[12]) {
+        const double *p = se + tid;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const double a = p[i * te], b = p[i * te + ye];
+            const int k = i < 3 ? i : i + 3;   // by = 0: 0..2, by = 1: 6..8
+            F[k] = a + b;
+            F[k + 3] = b - a;
+        }
+    };
+    const int ey = y0 - 1 + ly, ex = x0 - 1 + lx;
+    const bool ein = elem && ey >= 0 && ey < ny && ex >= 0 && ex < nx;
+    const double *ep = E + ey + (int64_t)ny * ex;
+    const int64_t eplane = (int64_t)ny * nx;
+    auto modulus = [&](int z) { return ein && z >= 0 && z < nz ? ep[eplane * z] : 0.0; };
+
+    double Fp[12], carry[12], dot = 0.0;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) Fp[i] = carry[i] = 0.0;
+    stage(z0 - 1);
+    stage(z0);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    edges(z0 - 1);
+    __syncthreads();
+    double ev = modulus(z0 - 1), en = modulus(z0);
+    if (elem && ev != 0.0) faces(Fp);
+    __syncthreads();
+    for (int ez = z0 - 1; ez < zend; ++ez) {
+        // element layer ez between node layers ez (faces Fp) and ez + 1
+        edges(ez + 1);
+        __syncthreads();
+        if (ez + 2 <= zend) stage(ez + 2);
+        double rp[6];
+        if (elem) {
+            double Ft[12];
+            // the faces of layer ez + 1 are needed by the elements below and above them
+            if (ev != 0.0 || en != 0.0) faces(Ft);
+            double phi[12];
+            if (ev != 0.0) {
+                double h[24];
+#pragma unroll
+                for (int i = 0; i < 12; ++i) {
+                    h[i] = i < 3 ? 0.0 : Fp[i] + Ft[i];
+                    h[12 + i] = Ft[i] - Fp[i];
+                }
+                if constexpr (CUBIC) {
+                    double k[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) k[i] = c_kc64[i] * ev;
+                    kh_cubic_f64(h, k);
+                } else {
+                    kh_general_f64(h, ev);
+                }
+#pragma unroll
+                for (int i = 0; i < 12; ++i) {
+                    phi[i] = i < 3 ? carry[i] - h[12 + i] : carry[i] + (h[i] - h[12 + i]);
+                    carry[i] = i < 3 ? h[12 + i] : h[i] + h[12 + i];
+                }
+            } else {   // void: nothing is read from its nodes, whatever they hold
+#pragma unroll
+                for (int i = 0; i < 12; ++i) {
+                    phi[i] = carry[i];
+                    carry[i] = 0.0;
+                }
+            }
+            // x butterfly undone: column lx gets phi0 - phi1, column lx + 1 phi0 + phi1
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                const int k = i < 3 ? i : i + 3;
+                sl[i * tn + tid] = phi[k] - phi[k + 3];
+                rp[i] = phi[k] + phi[k + 3];
+            }
+            if (en != 0.0) {
+#pragma unroll
+                for (int i = 0; i < 12; ++i) Fp[i] = Ft[i];
+            }
+            ev = en;
+            en = modulus(ez + 2);
+        }
+        __syncthreads();
+        // edge of column lx + 1: this element's right part and the next column's left part; y
+        // butterfly undone: node ly + 1 gets t0 - t1, node ly gets t0 + t1
+        double lo[3];
+        if (elem && lx < xe - 1) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double t0 = rp[c] + sl[c * tn + tid + ye], t1 = rp[3 + c] + sl[(3 + c) * tn + tid + ye];
+                lo[c] = t0 - t1;
+                sn[c * tn + tid] = t0 + t1;
+            }
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        if (owner && ez >= z0) {
+            const int64_t node = gy + (int64_t)NY * gx + plane * ez;
+            const uint8_t f = nflag[node];
+            const double *un = su + (ez + 3) % k64::SLOTS * nw + 3 * (ly + 1 + (ye + 1) * (lx + 1));
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double o = (f & (NF_FIXX << c)) ? 0.0 : lo[c] + sn[c * tn + tid + 1];
+                y[3 * node + c] = o;
+                if (DOT) dot = fma(un[c], o, dot);
+            }
+        }
+    }
+    if (DOT) {
+        __shared__ double red[k64::MAX_THREADS / 32];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, o);
+        if ((tid & 31) == 0) red[tid >> 5] = dot;
+        __syncthreads();
+        if (tid == 0) {
+            double s = 0.0;
+            for (int i = 0; i < nt / 32; ++i) s += red[i];
+            partial[slot] = s;
+        }
+    }
+}
+
+// The tile for a grid: the FP64 pipe runs a CTA's element layers one after the
+// other, so a tile's cost is the work of the busiest SM, (CTAs / 152 rounded
+// up) x (zc + 1) layers x warps x 137 operations at 16 clocks a warp, plus the
+// barriers' latency per layer and a CTA's start.  Small grids get many small
+// CTAs that fill the SMs, large ones tiles whose ragged edge and halo are
+// small.  At most SGLD_NOALLOC_MAX_CTAS CTAs, the scratch of the
+// allocation-free call, where the grid allows it.
+void kbyu64_pick_tile(Level &l) {
+    const int NY = l.ny + 1, NX = l.nx + 1, NZ = l.nz + 1;
+    constexpr int SMS = 152, MAX_CTAS = 32768;
+    double best = 0.0;
+    l.k64_ye = 0;
+    for (int ty = 1; ty <= NY; ++ty) {   // tiles along y: the smallest ye that needs no more of them
+        const int ye = (NY + ty - 1) / ty + 1;
+        if ((NY + ye - 2) / (ye - 1) != ty) continue;
+        if (ye < 4 && ty > 1) break;
+        if (ye * 2 > k64::MAX_THREADS) continue;
+        for (int tx = 1; tx <= NX; ++tx) {
+            const int xe = (NX + tx - 1) / tx + 1;
+            if ((NX + xe - 2) / (xe - 1) != tx) continue;
+            if (xe < 4 && tx > 1) break;
+            const int nt = k64::threads(ye, xe);
+            if (nt > k64::MAX_THREADS || k64::node_words(ye, xe) > k64::STAGE * nt) continue;
+            for (int tz = 1; tz <= NZ; ++tz) {
+                const int zc = (NZ + tz - 1) / tz;
+                if ((NZ + zc - 1) / zc != tz) continue;
+                if (zc < 2 && tz > 1) break;
+                const int64_t n = (int64_t)ty * tx * tz;
+                const double layer = nt / 32 * (137.0 * 16.0) + 600.0;
+                double cost = (double)((n + SMS - 1) / SMS) * ((zc + 1) * layer + 3000.0);
+                if (n > MAX_CTAS) cost *= 1e6;
+                if (!l.k64_ye || cost < best) {
+                    best = cost;
+                    l.k64_ye = ye;
+                    l.k64_xe = xe;
+                    l.k64_zc = zc;
+                }
+            }
+        }
+    }
+}
+
+dim3 kbyu64_grid(const Level &l) {
+    return dim3((l.ny + l.k64_ye - 1) / (l.k64_ye - 1), (l.nx + l.k64_xe - 1) / (l.k64_xe - 1),
+                (l.nz + l.k64_zc) / l.k64_zc);
+}
+
+template <bool DOT, bool CUBIC>
+static void attributes() {
+    // the widest node ring any tile asks for
+    size_t most = 0;
+    for (int ye = 2; ye <= k64::MAX_THREADS / 2; ++ye)
+        for (int xe = 2; ye * xe <= k64::MAX_THREADS; ++xe)
+            if (k64::node_words(ye, xe) <= k64::STAGE * k64::threads(ye, xe) && k64::smem(ye, xe) > most)
+                most = k64::smem(ye, xe);
+    cudaFuncSetAttribute(k_kbyu64<DOT, CUBIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
+void init_kbyu64_attributes() {
+    attributes<true, true>();
+    attributes<true, false>();
+    attributes<false, true>();
+    attributes<false, false>();
+}
+
+template <bool DOT, bool CUBIC>
+static void launch(const Level &l0, const double *E, const double *u, double *y, double *partial, cudaStream_t s) {
+    const int ye = l0.k64_ye, xe = l0.k64_xe;
+    k_kbyu64<DOT, CUBIC><<<kbyu64_grid(l0), k64::threads(ye, xe), k64::smem(ye, xe), s>>>(
+        u, y, E, l0.nflag, l0.ny, l0.nx, l0.nz, ye, xe, l0.k64_zc, partial, l0.tiles64);
+}
+
+void launch_kbyu_f64(const Level &l0, const double *E, const double *u, double *y, double *partial_dot,
+                     int *nblocks_out, cudaStream_t s) {
+    const dim3 g = kbyu64_grid(l0);
+    if (nblocks_out) *nblocks_out = (int)(g.x * g.y * g.z);
+    ++g_launches;
+    if (partial_dot)
+        l0.kh_cubic64 ? launch<true, true>(l0, E, u, y, partial_dot, s) : launch<true, false>(l0, E, u, y, partial_dot, s);
+    else
+        l0.kh_cubic64 ? launch<false, true>(l0, E, u, y, nullptr, s) : launch<false, false>(l0, E, u, y, nullptr, s);
+}
+
+}  // namespace sgld

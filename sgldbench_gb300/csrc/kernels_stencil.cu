@@ -1,20 +1,9 @@
-// Element-stencil kernels on the finest level: matrix-free K*u, unit
-// compliance and the stress recovery of the solution.
-//
-// K*u (reference: src/MEXfuncs/Solving_KbyU_MatrixFree_mex.cpp:53-138) is
-// restated for a structured grid without colouring.  A CTA owns a tile of
-// (TY-1) x (TX-1) node columns and marches through z one element layer at a
-// time: the two node layers an element layer touches are staged in shared
-// memory, every thread applies E_e*Ke to one element of the (TY x TX)
-// element tile (which includes a one-element halo), writes the 24 results to
-// shared memory, and every node thread then sums the contributions of its 8
-// neighbouring elements.  No atomics, deterministic, every node written once.
+// Element-stencil kernels on the finest level: the FP32 matrix-free K*u, unit
+// compliance and the stress recovery of the solution.  (FP64 K*u:
+// kernels_kbyu64.cu; double-float K*u: kernels_df.cu.)
 //
 // The element product uses the 8-corner Hadamard basis in which the
-// isotropic hexahedral Ke has 45 nonzeros (instead of 576): forward
-// butterflies (72 adds), 45 FMAs, E scaling, inverse butterflies (72 adds).
-// FP64 arithmetic is the scarce resource on GB300, so this is the form that
-// matters for the FP64 operator.
+// isotropic hexahedral Ke has 45 nonzeros (instead of 576).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -46,14 +35,25 @@ constexpr int KH_CLASS[KH_NNZ] = {0, 1, 1, 1, 0, 1, 1, 1, 0,   // {3, 7, 14}
                                   3, 4, 4, 3,                  // {15, 19}
                                   7, 7, 7};                    // 21, 22, 23
 
-bool kh_cubic(const double *Kh) {
-    double rep[8], mx = 0.0;
-    for (int i = KH_NNZ - 1; i >= 0; --i) {
-        rep[KH_CLASS[i]] = Kh[i];   // ends with each letter's first entry
-        mx = fmax(mx, fabs(Kh[i]));
+// the letters' values, A .. H: the mean of their entries (which differ by
+// rounding when the matrix is cubic: 2.4e-16 of the largest over Poisson
+// ratios 0 to 0.49)
+static void kh_letters(const double *Kh, double rep[8]) {
+    int n[8] = {};
+    for (int k = 0; k < 8; ++k) rep[k] = 0.0;
+    for (int i = 0; i < KH_NNZ; ++i) {
+        rep[KH_CLASS[i]] += Kh[i];
+        ++n[KH_CLASS[i]];
     }
+    for (int k = 0; k < 8; ++k) rep[k] /= n[k];
+}
+
+bool kh_cubic(const double *Kh, double tol) {
+    double rep[8], mx = 0.0;
+    kh_letters(Kh, rep);
+    for (int i = 0; i < KH_NNZ; ++i) mx = fmax(mx, fabs(Kh[i]));
     for (int i = 0; i < KH_NNZ; ++i)
-        if (fabs(Kh[i] - rep[KH_CLASS[i]]) > 1e-12 * mx) return false;
+        if (!(fabs(Kh[i] - rep[KH_CLASS[i]]) <= tol * mx)) return false;
     return true;
 }
 
@@ -62,20 +62,14 @@ void upload_kh(const double *Kh, cudaStream_t s) {
     for (int i = 0; i < KH_NNZ; ++i) f[i] = (float)Kh[i];
     cudaMemcpyToSymbolAsync(c_Kh, Kh, sizeof(double) * KH_NNZ, 0, cudaMemcpyHostToDevice, s);
     cudaMemcpyToSymbolAsync(c_Kh32, f, sizeof(float) * KH_NNZ, 0, cudaMemcpyHostToDevice, s);
-    // A-B, B, C, D, E, F-G, G, H from the letters' first entries (zeros when not cubic;
-    // the 8-value kernels then never run)
-    float kc[8] = {};
-    if (kh_cubic(Kh)) {
-        kc[0] = (float)(Kh[0] - Kh[1]);
-        kc[1] = (float)Kh[1];
-        kc[2] = (float)Kh[9];
-        kc[3] = (float)Kh[21];
-        kc[4] = (float)Kh[22];
-        kc[5] = (float)(Kh[29] - Kh[30]);
-        kc[6] = (float)Kh[30];
-        kc[7] = (float)Kh[42];
-    }
+    // A-B, B, C, D, E, F-G, G, H (the 8-value kernels run only when the matrix is cubic)
+    double rep[8];
+    kh_letters(Kh, rep);
+    const double kd[8] = {rep[0] - rep[1], rep[1], rep[2], rep[3], rep[4], rep[5] - rep[6], rep[6], rep[7]};
+    float kc[8];
+    for (int i = 0; i < 8; ++i) kc[i] = (float)kd[i];
     cudaMemcpyToSymbolAsync(c_Kc32, kc, sizeof kc, 0, cudaMemcpyHostToDevice, s);
+    upload_kh64(Kh, kd, s);
     cudaStreamSynchronize(s);
 }
 
@@ -179,44 +173,8 @@ __device__ __forceinline__ T block_sum(T v, T *red) {
     return s;
 }
 
-constexpr int KT_Y = 32, KT_X = 8, KT_THREADS = KT_Y * KT_X;
-constexpr int KT_NL = (KT_Y + 1) * (KT_X + 1);   // staged nodes per layer
+constexpr int KT_Y = 32, KT_X = 8;
 constexpr int KT_ZC = 16;                        // node layers per CTA
-
-constexpr int KT_SV = (KT_NL * 3 + KT_THREADS - 1) / KT_THREADS;   // staged words per thread and layer
-
-// node layer z lives in ring slot z mod 3 (z may be -1)
-__device__ __forceinline__ int kslot(int z) { return (z + 3) % 3; }
-
-// asynchronous global -> shared word copy (cp.async, completes at async_wait_all)
-template <typename T>
-__device__ __forceinline__ void async_copy(T *dst, const T *src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    if (sizeof(T) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src));
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src));
-}
-__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// A CTA whose element box holds no active element: every node it owns is
-// inactive and its K*u is exactly zero, so it writes zeros (no loads, no
-// element work) and a zero dot partial.  The whole CTA takes this branch.
-template <typename T>
-__device__ __forceinline__ void skip_tile(T *__restrict__ y, bool owner, int gny, int gnx, int NY, int NX, int z0,
-                                          int zend, double *__restrict__ partial) {
-    if (owner) {
-        const int64_t node0 = (int64_t)gny + (int64_t)NY * gnx;
-        for (int z = z0; z < zend; ++z) {
-            T *o = y + 3 * (node0 + (int64_t)NY * NX * z);
-            o[0] = T(0);
-            o[1] = T(0);
-            o[2] = T(0);
-        }
-    }
-    if (partial && threadIdx.x == 0) partial[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = 0.0;
-}
 
 // Active-tile map of a z-marching K*u grid g whose CTAs own (TY-1) x (TX-1)
 // node columns and zc node layers: a CTA is active iff an element of its box
@@ -246,137 +204,6 @@ static void make_tile_map(const Level &l, int TY, int TX, int zc, dim3 g, uint8_
     const int64_t ntile = (int64_t)g.x * g.y * g.z;
     ++g_launches;
     k_tile_map<<<(unsigned)((ntile + 3) / 4), 128, 0, s>>>(l.eact, l.ny, l.nx, l.nz, TY, TX, zc, g, out);
-}
-
-// y = K u on the full grid; y at fixed DOFs is 0.  When DOT, also writes
-// sum(u .* y) of this CTA's nodes to partial[block].
-template <typename T, bool DOT>
-__global__ void __launch_bounds__(KT_THREADS) k_kbyu(const T *__restrict__ u, T *__restrict__ y,
-                                                     const T *__restrict__ E, const uint8_t *__restrict__ nflag,
-                                                     int ny, int nx, int nz, double *__restrict__ partial,
-                                                     const uint8_t *__restrict__ tiles) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *su = reinterpret_cast<T *>(smem_raw);      // [3][KT_NL*3] ring of node layers
-    T *so = su + 3 * KT_NL * 3;                   // [24][KT_THREADS]
-    const int tid = threadIdx.x;
-    const int ty = tid % KT_Y, tx = tid / KT_Y;
-    const int NY = ny + 1, NX = nx + 1, NZ = nz + 1;
-    const int y0 = blockIdx.x * (KT_Y - 1), x0 = blockIdx.y * (KT_X - 1), z0 = blockIdx.z * KT_ZC;
-    const int zend = min(z0 + KT_ZC, NZ);
-    const int gny = y0 + ty, gnx = x0 + tx;
-    const bool owner = (ty < KT_Y - 1) && (tx < KT_X - 1) && gny < NY && gnx < NX;
-    const int ey = y0 - 1 + ty, ex = x0 - 1 + tx;
-    const bool ein = ey >= 0 && ey < ny && ex >= 0 && ex < nx;
-    if (tiles && !tiles[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)]) {
-        skip_tile(y, owner, gny, gnx, NY, NX, z0, zend, DOT ? partial : nullptr);
-        return;
-    }
-    T acc0 = T(0), acc1 = T(0), acc2 = T(0);
-    T dot = T(0);
-
-    // staging plan: this thread copies up to KT_SV words of every node layer;
-    // the in-layer source offsets are fixed, only the layer stride changes
-    int soff[KT_SV];
-#pragma unroll
-    for (int k = 0; k < KT_SV; ++k) {
-        const int i = tid + k * KT_THREADS;
-        soff[k] = -2;
-        if (i < KT_NL * 3) {
-            const int node = i / 3, c = i - 3 * node;
-            const int ly = node % (KT_Y + 1), lx = node / (KT_Y + 1);
-            const int gy = y0 - 1 + ly, gx = x0 - 1 + lx;
-            soff[k] = (gy >= 0 && gy < NY && gx >= 0 && gx < NX) ? 3 * (gy + NY * gx) + c : -1;
-        }
-    }
-    const int64_t lstride = 3 * (int64_t)NY * NX;
-    auto stage = [&](int z) {
-        T *dst = su + kslot(z) * KT_NL * 3;
-        const bool zin = z >= 0 && z < NZ;
-#pragma unroll
-        for (int k = 0; k < KT_SV; ++k) {
-            const int i = tid + k * KT_THREADS;
-            if (soff[k] == -2) continue;
-            if (zin && soff[k] >= 0)
-                async_copy(dst + i, u + ((int64_t)z * lstride + soff[k]));
-            else
-                dst[i] = T(0);
-        }
-        async_commit();
-    };
-
-    stage(z0 - 1);
-    stage(z0);
-    async_wait_all();
-    __syncthreads();
-    for (int ez = z0 - 1; ez < zend; ++ez) {
-        const int s0 = kslot(ez), s1 = kslot(ez + 1);
-        if (ez + 2 <= zend) stage(ez + 2);   // prefetch, overlaps the element work below
-        T ev = T(0);
-        if (ein && ez >= 0 && ez < nz) ev = E[(int64_t)ey + (int64_t)ny * (ex + (int64_t)nx * ez)];
-        T ue[24];
-        if (ev != T(0)) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int dx = k & 1, dy = 1 - ((k >> 1) & 1), kp = k >> 2;
-                const T *src = su + (kp ? s1 : s0) * KT_NL * 3 + 3 * ((ty + dy) + (KT_Y + 1) * (tx + dx));
-                ue[3 * k + 0] = src[0];
-                ue[3 * k + 1] = src[1];
-                ue[3 * k + 2] = src[2];
-            }
-            hex_apply<T>(ue, ev);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 24; ++i) ue[i] = T(0);
-        }
-#pragma unroll
-        for (int i = 0; i < 24; ++i) so[i * KT_THREADS + tid] = ue[i];
-        __syncthreads();
-        if (owner) {
-            // lower corners (kp = 0) of element layer ez complete node layer ez
-#pragma unroll
-            for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-                for (int dx = 0; dx < 2; ++dx) {
-                    const int k = dx | ((1 - dy) << 1);
-                    const int t = (ty + 1 - dy) + KT_Y * (tx + 1 - dx);
-                    acc0 += so[(3 * k + 0) * KT_THREADS + t];
-                    acc1 += so[(3 * k + 1) * KT_THREADS + t];
-                    acc2 += so[(3 * k + 2) * KT_THREADS + t];
-                }
-            if (ez >= z0) {
-                const int64_t node = (int64_t)gny + (int64_t)NY * (gnx + (int64_t)NX * ez);
-                const uint8_t f = nflag[node];
-                const T o0 = (f & NF_FIXX) ? T(0) : acc0;
-                const T o1 = (f & NF_FIXY) ? T(0) : acc1;
-                const T o2 = (f & NF_FIXZ) ? T(0) : acc2;
-                y[3 * node + 0] = o0;
-                y[3 * node + 1] = o1;
-                y[3 * node + 2] = o2;
-                if (DOT) {
-                    const T *un = su + s0 * KT_NL * 3 + 3 * ((ty + 1) + (KT_Y + 1) * (tx + 1));
-                    dot += un[0] * o0 + un[1] * o1 + un[2] * o2;
-                }
-            }
-            acc0 = acc1 = acc2 = T(0);
-#pragma unroll
-            for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-                for (int dx = 0; dx < 2; ++dx) {
-                    const int k = 4 | dx | ((1 - dy) << 1);
-                    const int t = (ty + 1 - dy) + KT_Y * (tx + 1 - dx);
-                    acc0 += so[(3 * k + 0) * KT_THREADS + t];
-                    acc1 += so[(3 * k + 1) * KT_THREADS + t];
-                    acc2 += so[(3 * k + 2) * KT_THREADS + t];
-                }
-        }
-        async_wait_all();
-        __syncthreads();
-    }
-    if (DOT) {
-        __shared__ double red[KT_THREADS / 32];
-        const double s = block_sum_to_double<T>(dot, red);
-        if (tid == 0) partial[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = s;
-    }
 }
 
 // ---- paired FP32 arithmetic -----------------------------------------------------
@@ -803,11 +630,6 @@ static dim3 kbyu_grid(const Level &l) {
     return dim3((l.ny + 1 + KT_Y - 2) / (KT_Y - 1), (l.nx + 1 + KT_X - 2) / (KT_X - 1), (l.nz + 1 + KT_ZC - 1) / KT_ZC);
 }
 
-template <typename T>
-static constexpr size_t kbyu_smem() {
-    return sizeof(T) * (3 * KT_NL * 3 + 24 * KT_THREADS);
-}
-
 template <int TX, bool DOT, bool CUBIC>
 static void tma_attributes() {
     cudaFuncSetAttribute(k_kbyu_tma<TX, DOT, CUBIC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -817,8 +639,7 @@ static void tma_attributes() {
 // opt-in shared memory sizes; called once per context before any launch or
 // graph capture
 void init_kernel_attributes() {
-    cudaFuncSetAttribute(k_kbyu<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kbyu_smem<double>());
-    cudaFuncSetAttribute(k_kbyu<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kbyu_smem<double>());
+    init_kbyu64_attributes();
     tma_attributes<8, true, false>();
     tma_attributes<8, false, false>();
     tma_attributes<16, true, false>();
@@ -857,23 +678,6 @@ static int vector_tensor_map(CUtensorMap *m, const float *u, int64_t n) {
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : -1;
-}
-
-template <typename T, bool DOT>
-static void kbyu_launch(const Level &l0, const T *E, const T *u, T *y, double *partial, int *nb, cudaStream_t s) {
-    const size_t smem = kbyu_smem<T>();
-    dim3 g = kbyu_grid(l0);
-    if (nb) *nb = (int)(g.x * g.y * g.z);
-    ++g_launches;
-    k_kbyu<T, DOT><<<g, KT_THREADS, smem, s>>>(u, y, E, l0.nflag, l0.ny, l0.nx, l0.nz, partial, l0.tiles16);
-}
-
-void launch_kbyu_f64(const Level &l0, const double *E, const double *u, double *y, double *partial_dot,
-                     int *nblocks_out, cudaStream_t s) {
-    if (partial_dot)
-        kbyu_launch<double, true>(l0, E, u, y, partial_dot, nblocks_out, s);
-    else
-        kbyu_launch<double, false>(l0, E, u, y, nullptr, nblocks_out, s);
 }
 
 template <int TX, bool DOT, bool CUBIC>
@@ -924,6 +728,12 @@ int update_kbyu_tiles(Level &l0, cudaStream_t s) {
         if (e != cudaSuccess) return (int)e;
         make_tile_map(l0, KT_Y, KT_X, KT_ZC, g16, l0.tiles16, s);
     }
+    if (!l0.tiles64) {
+        const dim3 g = kbyu64_grid(l0);
+        e = cudaMalloc((void **)&l0.tiles64, (size_t)g.x * g.y * g.z);
+        if (e != cudaSuccess) return (int)e;
+        make_tile_map(l0, l0.k64_ye, l0.k64_xe, l0.k64_zc, g, l0.tiles64, s);
+    }
     if (!l0.kerr) {
         e = cudaMalloc((void **)&l0.kerr, sizeof(int));
         if (e != cudaSuccess) return (int)e;
@@ -948,10 +758,6 @@ int update_kbyu_tiles(Level &l0, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
-int kbyu_num_blocks(const Level &l0) {
-    dim3 g = kbyu_grid(l0);
-    return (int)(g.x * g.y * g.z);
-}
 
 // ---------------------------------------------------------------------------
 // unit compliance ce_e = u_e' Ke u_e (TopOpti_CmptUnitCompliance_mex.cpp:40-107)

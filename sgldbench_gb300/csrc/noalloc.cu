@@ -7,14 +7,11 @@
 // scratch (one partial sum per CTA of the K*u grid) lives in the file-scope
 // device array below, which every GPU that loads this library holds until the
 // process exits.  The call itself allocates nothing.
+#include <algorithm>
 #include <atomic>
 
 #include "../../include/sgld_gpu.h"
 #include "sgld_internal.cuh"
-
-namespace sgld {
-int kbyu_num_blocks(const Level &l0);
-}
 
 using namespace sgld;
 
@@ -37,9 +34,13 @@ extern "C" int sgld_kbyu_dot_noalloc(sgld_ctx *ctx, const double *d_u, double *d
         return SGLD_ERR_STATE;
     }
     const Level &l0 = c.lv[0];
-    const int nb = kbyu_num_blocks(l0);
+    // grids of more than 32768 blocks of 31 x 7 x 16 nodes are refused; the tile's choice
+    // keeps every smaller grid within the scratch (checked all the same)
+    const dim3 g = kbyu64_grid(l0);
+    const int64_t nb = std::max((int64_t)(l0.ny / 31 + 1) * (l0.nx / 7 + 1) * (l0.nz / 16 + 1),
+                                (int64_t)g.x * g.y * g.z);
     if (nb > SGLD_NOALLOC_MAX_CTAS) {
-        c.err = "sgld_kbyu_dot_noalloc: grid of " + std::to_string(nb) + " CTAs exceeds the scratch limit of " +
+        c.err = "sgld_kbyu_dot_noalloc: grid of " + std::to_string(nb) + " blocks exceeds the scratch limit of " +
                 std::to_string(SGLD_NOALLOC_MAX_CTAS) + " (use sgld_kbyu_device for larger grids)";
         return SGLD_ERR_ARG;
     }

@@ -708,7 +708,7 @@ bool g_kh_stale[kMaxDevices] = {};      // upload again even if the record match
 double g_kh_held[kMaxDevices][KH_NNZ];   // the element matrix in each device's constants
 }  // namespace
 
-// the FP32 K*u's 45-value form even for a cubic element matrix (environment
+// the K*u's 45-value form even for a cubic element matrix (environment
 // SGLD_KH_GENERAL=1, read once; for comparisons)
 static bool kh_general_forced() {
     static const bool v = [] {
@@ -723,7 +723,10 @@ int bind_ctx(sgld_ctx *ctx) {
     int dev = -1;
     CK(cudaGetDevice(&dev));
     if (dev != c.device) CK(cudaSetDevice(c.device));
-    if (!c.lv.empty()) c.lv[0].kh_cubic = !kh_general_forced() && kh_cubic(c.Kh);
+    if (!c.lv.empty()) {
+        c.lv[0].kh_cubic = !kh_general_forced() && kh_cubic(c.Kh, 1e-12);
+        c.lv[0].kh_cubic64 = !kh_general_forced() && kh_cubic(c.Kh, 1e-15);
+    }
     std::lock_guard<std::mutex> lock(g_bind_mu);
     const bool same = g_kh_valid[c.device] && memcmp(g_kh_held[c.device], c.Kh, sizeof c.Kh) == 0;
     if (same && !g_kh_stale[c.device]) return SGLD_OK;
@@ -918,9 +921,11 @@ int sgld_create(int resY, int resX, int resZ, const uint8_t *solid, const sgld_o
     CK(dalloc(&c.d_isc, 16));
     init_kernel_attributes();
     init_kbyu_df_attributes();
+    kbyu64_pick_tile(c.lv[0]);
+    const dim3 g64 = kbyu64_grid(l0);
     // partial-sum slots: the largest grid of any kernel that writes per-CTA partials
     // (prolongation: ceil(NY*NX/256) CTAs per node plane)
-    c.npart = (int)std::max<int64_t>({(int64_t)152 * 8, (l0.nel + 255) / 256 + 1,
+    c.npart = (int)std::max<int64_t>({(int64_t)152 * 8, (l0.nel + 255) / 256 + 1, (int64_t)g64.x * g64.y * g64.z,
                                       (int64_t)(((l0.ny + 1) * (l0.nx + 1) + 255) / 256) * (l0.nz + 1),
                                       (int64_t)((l0.ny + 31) / 31 + 1) * ((l0.nx + 7) / 7 + 1) * ((l0.nz + 16) / 16 + 1)});
     CK(dalloc(&c.d_part, c.npart));
@@ -942,7 +947,7 @@ void sgld_destroy(sgld_ctx *ctx) {
         cudaSetDevice(c.device);
     for (Level &l : c.lv) {
         for (void *p : {(void *)l.eact, (void *)l.nflag, (void *)l.diag, (void *)l.idiag, (void *)l.idiag32, (void *)l.Ks, (void *)l.r,
-                        (void *)l.x, (void *)l.r32, (void *)l.x32, (void *)l.tiles16, (void *)l.tiles_f32,
+                        (void *)l.x, (void *)l.r32, (void *)l.x32, (void *)l.tiles64, (void *)l.tiles16, (void *)l.tiles_f32,
                         (void *)l.runs, (void *)l.kerr})
             if (p) cudaFree(p);
     }

@@ -45,15 +45,17 @@ struct Level {
     int kx_tx = 0;                // x width of the FP32 K*u tile, 8 or 16 (0 = 8; set by the tuner)
     bool kh_cubic = false;        // finest level: the bound element matrix has the hexahedron's
                                   // cubic symmetry (kh_cubic), so the FP32 K*u takes its 8-value form
+    bool kh_cubic64 = false;      // ... to rounding (kh_cubic at 1e-15), so the FP64 K*u takes it too
+    int k64_ye = 0, k64_xe = 0, k64_zc = 0;   // finest level: tile of the FP64 K*u (kbyu64_pick_tile)
     int64_t nel = 0, nnode = 0;   // full-grid counts
     int64_t nel_active = 0, nnode_active = 0;
     uint8_t *eact = nullptr;      // [nel] element non-empty
     // active-tile maps of the finest level's K*u launches (one byte per CTA:
     // 0 = no active element in the CTA's element box, so every node it owns
-    // is inactive and its result is zero): the 32 x 8 x 16-layer grid of the
-    // FP64 and double-float kernels, and the FP32 kernel's grid for the tile
-    // (tiles_f32_tx, tiles_f32_zc) it was made for
-    uint8_t *tiles16 = nullptr, *tiles_f32 = nullptr;
+    // is inactive and its result is zero): the FP64 kernel's grid, the 32 x 8 x
+    // 16-layer grid of the double-float kernel, and the FP32 kernel's grid for
+    // the tile (tiles_f32_tx, tiles_f32_zc) it was made for
+    uint8_t *tiles64 = nullptr, *tiles16 = nullptr, *tiles_f32 = nullptr;
     // finest level: the words of the active nodes as chunks of contiguous
     // floats (runs of active nodes along y, gaps of a few nodes bridged), each
     // first DOF | floats << 40, in address order; empty when nearly every node
@@ -182,8 +184,14 @@ extern thread_local int64_t g_launches;
 // ---- launchers (kernels_*.cu) ------------------------------------------------
 void upload_kh(const double *Kh, cudaStream_t s);
 // true when the 45 Hadamard-basis values take the 8 distinct values that the cubic
-// symmetry of an isotropic hexahedral element gives them (to 1e-12 of the largest)
-bool kh_cubic(const double *Kh);
+// symmetry of an isotropic hexahedral element gives them (to tol of the largest)
+bool kh_cubic(const double *Kh, double tol);
+// FP64 K*u (kernels_kbyu64.cu): the element matrix (kc: A-B, B, C, D, E, F-G, G, H, used
+// when kh_cubic64), the tile for a level's grid, the launch
+void upload_kh64(const double *Kh, const double *kc, cudaStream_t s);
+void kbyu64_pick_tile(Level &l0);
+dim3 kbyu64_grid(const Level &l0);
+void init_kbyu64_attributes();
 void launch_kbyu_f64(const Level &l0, const double *E, const double *u, double *y, double *partial_dot,
                      int *nblocks_out, cudaStream_t s);
 // (re)makes l0's active-tile maps for its current FP32 tile; 0 or a CUDA error
