@@ -57,7 +57,7 @@ __global__ void k_restrict(const T *__restrict__ rf, T *__restrict__ rc, int nyc
     rc[3 * n + 2] = a2;
 }
 
-// The same restriction with the span S a compile-time constant: the
+// The same restriction with the span S a compile-time constant (2): the
 // (2S-1)^3 taps unroll, the weights are constants and the indices stay 32-bit
 // (grids below 2^31 / 3 nodes).  Lanes hold consecutive coarse y, so for one
 // (dx, dz) a warp's taps cover a contiguous run of fine nodes.
@@ -112,6 +112,45 @@ __global__ void __launch_bounds__(128) k_restrict_s(const T *__restrict__ rf, T 
     rc[n + 2] = a2;
 }
 
+// Span 4: a warp per coarse node, whose lanes share the 7^3 taps (consecutive
+// lanes along fine y).  A non-dyadic hierarchy's first coarse level has 1/64 of
+// the fine nodes: a thread per coarse node left a 64 x 32 x 32 grid with 18
+// CTAs, each thread walking 343 taps (71 us in FP64, 36 us in FP32 there).  With
+// k_prolong_rows4 the FP64 analysis of that grid went from 23.9 to 16.0 ms, the
+// mixed one from 10.5 to 6.9 ms.
+template <typename T>
+__global__ void __launch_bounds__(256) k_restrict4(const T *__restrict__ rf, T *__restrict__ rc,
+                                                   const uint8_t *__restrict__ cflag, int nyc, int nxc, int nzc,
+                                                   int keep_zeros) {
+    constexpr int S = 4, W = 2 * S - 1;
+    const int NYc = nyc + 1, NXc = nxc + 1;
+    const int NYf = S * nyc + 1, NXf = S * nxc + 1, NZf = S * nzc + 1;
+    const int pl = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (pl >= NYc * NXc) return;
+    const int I = pl % NYc, J = pl / NYc, Kz = blockIdx.y, n = 3 * (pl + NYc * NXc * Kz);
+    if (!(cflag[n / 3] & NF_ACTIVE)) {
+        if (!keep_zeros && lane < 3) rc[n + lane] = T(0);
+        return;
+    }
+    T a[3] = {T(0), T(0), T(0)};
+#pragma unroll
+    for (int k = 0; k < (W * W * W + 31) / 32; ++k) {
+        const int t = lane + 32 * k, dy = t % W - (S - 1), dx = t / W % W - (S - 1), dz = t / (W * W) - (S - 1);
+        const int fy = S * I + dy, fx = S * J + dx, fz = S * Kz + dz;
+        if (t < W * W * W && fy >= 0 && fy < NYf && fx >= 0 && fx < NXf && fz >= 0 && fz < NZf) {
+            const T w = T((S - abs(dy)) * (S - abs(dx)) * (S - abs(dz))) * (T(1) / T(S * S * S));
+            const T *r = rf + 3 * (fy + NYf * (fx + NXf * fz));
+#pragma unroll
+            for (int c = 0; c < 3; ++c) a[c] += w * r[c];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
+    if (lane < 3) rc[n + lane] = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];
+}
+
 template <typename T>
 void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *rc, cudaStream_t st) {
     ++g_launches;
@@ -123,7 +162,8 @@ void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *rc,
     if (small && coarse.span == 2)
         k_restrict_s<T, 2><<<g, 128, 0, st>>>(rf, rc, coarse.nflag, coarse.ny, coarse.nx, coarse.nz, keep);
     else if (small && coarse.span == 4)
-        k_restrict_s<T, 4><<<g, 128, 0, st>>>(rf, rc, coarse.nflag, coarse.ny, coarse.nx, coarse.nz, keep);
+        k_restrict4<T><<<dim3((unsigned)(((coarse.ny + 1) * (coarse.nx + 1) + 7) / 8), g.y), 256, 0, st>>>(
+            rf, rc, coarse.nflag, coarse.ny, coarse.nx, coarse.nz, keep);
     else
         k_restrict<T><<<g, 128, 0, st>>>(rf, rc, coarse.ny, coarse.nx, coarse.nz, coarse.span);
 }
@@ -330,6 +370,81 @@ __global__ void __launch_bounds__(128) k_prolong_cells(const T *__restrict__ xc,
     }
 }
 
+// Span 4: a thread per fine column (fx, fz) and coarse cell along y, writing
+// the cell's 4 fine nodes of that column.  Same operator as k_prolong_cells, whose
+// thread per coarse cell walks 64 fine nodes and left a 64 x 32 x 32 grid with 18
+// CTAs (73 us in FP64, 28 us in FP32 there).
+// keep_zeros: inactive nodes of xf hold 0 and are not written.
+template <typename T, bool FINAL>
+__global__ void __launch_bounds__(128) k_prolong_rows4(const T *__restrict__ xc, const T *__restrict__ rf,
+                                                       const T *__restrict__ D, const uint8_t *__restrict__ nflag,
+                                                       T omega, T *__restrict__ xf, int nyc, int nxc, int nzc,
+                                                       int keep_zeros, double *__restrict__ partial) {
+    constexpr int S = 4;
+    const int NYc = nyc + 1, NXc = nxc + 1, NYf = S * nyc + 1, NXf = S * nxc + 1;
+    const int pl = blockIdx.x * blockDim.x + threadIdx.x;
+    T dot = T(0);
+    if (pl < NYc * NXf) {
+        const int I = pl % NYc, fx = pl / NYc, fz = blockIdx.y;
+        const int J = fx / S, rx = fx % S, K = fz / S, rz = fz % S;
+        const int f0 = S * I + NYf * (fx + NXf * fz), ly = I < nyc ? S : 1;
+        uint8_t fl[S];
+        T r[S][3], dg[S][3];
+        bool any = false;
+        // r and D are loaded whatever the flags say, so that they do not wait for them
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            fl[k] = k < ly ? nflag[f0 + k] : 0;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                r[k][q] = k < ly ? rf[3 * (f0 + k) + q] : T(0);
+                dg[k][q] = k < ly ? D[3 * (f0 + k) + q] : T(0);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < S; ++k) any |= (fl[k] & NF_ACTIVE) != 0;
+        T qa[2][3] = {};
+        if (any) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    if ((c && rz == 0) || (b && rx == 0)) continue;
+                    const T w = T((c ? rz : S - rz) * (b ? rx : S - rx)) * (T(1) / T(S * S));
+#pragma unroll
+                    for (int a = 0; a < 2; ++a) {
+                        if (a && I == nyc) continue;
+                        const T *x = xc + 3 * ((I + a) + NYc * ((J + b) + NXc * (K + c)));
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) qa[a][q] += w * x[q];
+                    }
+                }
+        }
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            if (k >= ly) break;
+            const bool act = (fl[k] & NF_ACTIVE) != 0;
+            T o[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const T t = (omega * r[k][q]) * dg[k][q];
+                o[q] = act ? (t + (T(S - k) / T(S) * qa[0][q] + T(k) / T(S) * qa[1][q])) + t : T(0);
+                if (FINAL && (fl[k] & (NF_FIXX << q))) o[q] = T(0);
+            }
+            if (FINAL && act) dot += o[0] * r[k][0] + o[1] * r[k][1] + o[2] * r[k][2];
+            if (act || !keep_zeros) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) xf[3 * (f0 + k) + q] = o[q];
+            }
+        }
+    }
+    if (FINAL && partial) {
+        __shared__ double red[4];
+        const double sum = warp_block_sum<T>(dot, red);
+        if (threadIdx.x == 0) partial[blockIdx.x + gridDim.x * blockIdx.y] = sum;
+    }
+}
+
 template <typename T>
 void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, const T *rf, const T *diag, T omega,
                            T *xf, bool final_level, double *partial_dot, int *nblocks_out, cudaStream_t st) {
@@ -337,7 +452,19 @@ void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, 
     // empty cells are skipped in FP32 only: the FP32 V-cycle's outputs (d_z32 and the
     // levels' x32) are zeroed at allocation, so their inactive nodes hold 0 throughout
     const bool skip_inactive = sizeof(T) == sizeof(float);
-    if (small && (coarse.span == 2 || coarse.span == 4)) {
+    if (small && coarse.span == 4) {
+        const dim3 g((unsigned)(((coarse.ny + 1) * (int64_t)(fine.nx + 1) + 127) / 128), (unsigned)(fine.nz + 1));
+        if (nblocks_out) *nblocks_out = (int)(g.x * g.y);
+        ++g_launches;
+        if (final_level)
+            k_prolong_rows4<T, true><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, omega, xf, coarse.ny, coarse.nx,
+                                                        coarse.nz, skip_inactive, partial_dot);
+        else
+            k_prolong_rows4<T, false><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, omega, xf, coarse.ny, coarse.nx,
+                                                         coarse.nz, skip_inactive, nullptr);
+        return;
+    }
+    if (small && coarse.span == 2) {
         // 8 (else 4) coarse planes per CTA while that keeps at least 8 CTAs per SM
         const int64_t plane_ctas = ((coarse.ny + 1) * (int64_t)(coarse.nx + 1) + 127) / 128;
         int zp = 8;
@@ -345,22 +472,13 @@ void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, 
         const dim3 g((unsigned)plane_ctas, (unsigned)((coarse.nz + zp) / zp));
         if (nblocks_out) *nblocks_out = (int)(g.x * g.y);
         ++g_launches;
-#define PCELLS(S, F)                                                                                              \
-    k_prolong_cells<T, S, F><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, skip_inactive ? coarse.nflag : nullptr, \
-                                                omega, xf, coarse.ny, coarse.nx, coarse.nz, zp,                  \
-                                                F ? partial_dot : nullptr)
-        if (coarse.span == 2) {
-            if (final_level)
-                PCELLS(2, true);
-            else
-                PCELLS(2, false);
-        } else {
-            if (final_level)
-                PCELLS(4, true);
-            else
-                PCELLS(4, false);
-        }
-#undef PCELLS
+        const uint8_t *cflag = skip_inactive ? coarse.nflag : nullptr;
+        if (final_level)
+            k_prolong_cells<T, 2, true><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, cflag, omega, xf, coarse.ny,
+                                                           coarse.nx, coarse.nz, zp, partial_dot);
+        else
+            k_prolong_cells<T, 2, false><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, cflag, omega, xf, coarse.ny,
+                                                            coarse.nx, coarse.nz, zp, nullptr);
         return;
     }
     const dim3 nb((unsigned)(((fine.ny + 1) * (fine.nx + 1) + 255) / 256), (unsigned)(fine.nz + 1));
