@@ -587,23 +587,18 @@ __global__ void k_scatter_nodes(const int64_t *__restrict__ map, int64_t n, cons
     const int c = (int)(i - 3 * node);
     dst[3 * map[node] + c] = src[i];
 }
-__global__ void k_gather_nodes(const int64_t *__restrict__ map, int64_t n, const double *__restrict__ src,
-                               double *__restrict__ dst) {
+template <int PER>
+__global__ void k_gather_rows(const int64_t *__restrict__ map, int64_t n, const double *__restrict__ src,
+                              double *__restrict__ dst) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= 3 * n) return;
-    const int64_t node = i / 3;
-    const int c = (int)(i - 3 * node);
-    dst[i] = src[3 * map[node] + c];
+    if (i >= PER * n) return;
+    const int64_t row = i / PER;
+    dst[i] = src[PER * map[row] + (i - PER * row)];
 }
 __global__ void k_scatter_elems(const int64_t *__restrict__ map, int64_t n, const double *__restrict__ src,
                                 double *__restrict__ dst) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n) dst[map[i]] = src[i];
-}
-__global__ void k_gather_elems(const int64_t *__restrict__ map, int64_t n, const double *__restrict__ src,
-                               double *__restrict__ dst) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[map[i]];
 }
 
 void launch_scatter_nodes(const int64_t *map, int64_t n, const double *compact, double *full, cudaStream_t s) {
@@ -612,11 +607,19 @@ void launch_scatter_nodes(const int64_t *map, int64_t n, const double *compact, 
         k_scatter_nodes<<<(unsigned)((3 * n + 255) / 256), 256, 0, s>>>(map, n, compact, full);
     }
 }
-void launch_gather_nodes(const int64_t *map, int64_t n, const double *full, double *compact, cudaStream_t s) {
-    if (n > 0) {
-        ++g_launches;
-        k_gather_nodes<<<(unsigned)((3 * n + 255) / 256), 256, 0, s>>>(map, n, full, compact);
+void launch_gather_rows(const int64_t *map, int64_t n, int per, const double *src, double *dst, cudaStream_t s) {
+    if (n <= 0) return;
+    const unsigned nb = (unsigned)((per * n + 255) / 256);
+    ++g_launches;
+    switch (per) {
+        case 1: k_gather_rows<1><<<nb, 256, 0, s>>>(map, n, src, dst); break;
+        case 3: k_gather_rows<3><<<nb, 256, 0, s>>>(map, n, src, dst); break;
+        case 6: k_gather_rows<6><<<nb, 256, 0, s>>>(map, n, src, dst); break;
+        default: k_gather_rows<12><<<nb, 256, 0, s>>>(map, n, src, dst); break;
     }
+}
+void launch_gather_nodes(const int64_t *map, int64_t n, const double *full, double *compact, cudaStream_t s) {
+    launch_gather_rows(map, n, 3, full, compact, s);
 }
 void launch_scatter_elems(const int64_t *map, int64_t n, const double *compact, double *full, cudaStream_t s) {
     if (n > 0) {
@@ -625,10 +628,7 @@ void launch_scatter_elems(const int64_t *map, int64_t n, const double *compact, 
     }
 }
 void launch_gather_elems(const int64_t *map, int64_t n, const double *full, double *compact, cudaStream_t s) {
-    if (n > 0) {
-        ++g_launches;
-        k_gather_elems<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(map, n, full, compact);
-    }
+    launch_gather_rows(map, n, 1, full, compact, s);
 }
 
 // ---- fixed-DOF bookkeeping (src/FEA_SetupVoxelBased.m:13-26) ----------------

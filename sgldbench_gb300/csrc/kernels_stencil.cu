@@ -812,88 +812,182 @@ void launch_unit_compliance(const Level &l0, const double *u, const double *E, d
 // stress recovery (src/FEA_StressAnalysis.m:29-60): per element, corner
 // stresses = E_e * inv(sFM) * D * B * u_e (48 values); nodal stress = sum
 // over the elements sharing the node / their count; nodal von Mises.
-// Node-centric gather: each node thread recomputes the corner stresses of its
-// (at most 8) elements restricted to its own corner -> deterministic.
+// Node-centric gather over the active nodes (map), deterministic.
+//
+// The strains of a trilinear element lie in the span of its shape functions, so
+// extrapolating them from the Gauss points gives the strains at the corner
+// itself, whose derivatives are the differences along the corner's three edges.
+// The 4 elements on one side of a node share that side's difference, so
+//   sum_e E_e du/dx = EX+ (u(n+x) - u(n)) + EX- (u(n) - u(n-x)),
+// EX+- the sums of the moduli on that side: about 70 operations per node instead
+// of 8 products with 6 rows of M (1152).  On the 192 x 96 x 96 blob shape the
+// launch went from 2.70 to 0.105 ms, still bound by the FP64 pipe; the whole call
+// from 12.6 to 1.2 ms, as its results are now gathered on the device.
+//
+// A displacement that is not finite at some node spoils all corner stresses of
+// its elements in the reference's product, those of the opposite corners too; the
+// edge form would leave them out.  So when any displacement is not finite
+// (*nonfinite, k_any_nonfinite), the product with M is taken.
 // ---------------------------------------------------------------------------
-__global__ void k_nodal_stress(const double *__restrict__ u, const double *__restrict__ E,
-                               const uint8_t *__restrict__ nflag, const uint8_t *__restrict__ eact, int ny, int nx,
-                               int nz, double *__restrict__ s6,
-                               double *__restrict__ vm) {
-    const int NY = ny + 1, NX = nx + 1, NZ = nz + 1;
-    const int64_t nn = (int64_t)NY * NX * NZ;
-    const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (n >= nn) return;
-    const int iy = (int)(n % NY), ix = (int)((n / NY) % NX), iz = (int)(n / ((int64_t)NY * NX));
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    int cnt = 0;
-    if (nflag[n] & NF_ACTIVE) {
-        // reference corner order j: offsets (dy, dx, dz)
-        const int cdy[8] = {1, 1, 0, 0, 1, 1, 0, 0}, cdx[8] = {0, 1, 1, 0, 0, 1, 1, 0},
-                  cdz[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-        for (int j = 0; j < 8; ++j) {
-            const int ey = iy - cdy[j], ex = ix - cdx[j], ez = iz - cdz[j];
-            if (ey < 0 || ex < 0 || ez < 0 || ey >= ny || ex >= nx || ez >= nz) continue;
-            const int64_t eidx = (int64_t)ey + (int64_t)ny * (ex + (int64_t)nx * ez);
-            if (!eact[eidx]) continue;
-            const double ev = E[eidx];
-            ++cnt;
-            double ue[24];
-            for (int k = 0; k < 8; ++k) {
-                const int64_t m = (int64_t)(ey + cdy[k]) + (int64_t)NY * ((ex + cdx[k]) + (int64_t)NX * (ez + cdz[k]));
-                ue[3 * k] = u[3 * m];
-                ue[3 * k + 1] = u[3 * m + 1];
-                ue[3 * k + 2] = u[3 * m + 2];
-            }
-            for (int c = 0; c < 6; ++c) {
-                const double *row = c_M + (6 * j + c);   // column-major 48 x 24
-                double sacc = 0.0;
-                for (int i = 0; i < 24; ++i) sacc += row[48 * i] * ue[i];
-                acc[c] += sacc * ev;
-            }
-        }
-    }
-    double v[6];
-    for (int c = 0; c < 6; ++c) v[c] = cnt ? acc[c] / (double)cnt : 0.0;
-    for (int c = 0; c < 6; ++c) s6[6 * n + c] = v[c];
-    const double a = v[0] - v[1], b = v[1] - v[2], d = v[2] - v[0];
-    vm[n] = cnt ? sqrt(0.5 * (a * a + b * b + d * d) + 3.0 * (v[5] * v[5] + v[3] * v[3] + v[4] * v[4])) : 0.0;
+__global__ void k_any_nonfinite(const double *__restrict__ u, int64_t n, int *__restrict__ flag) {
+    bool bad = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        bad |= (__double2hiint(u[i]) & 0x7ff00000) == 0x7ff00000;
+    if (bad) *flag = 1;
 }
 
-void launch_stress(const Level &l0, const double *E, const double *u, const double *M48x24, double *nodal6,
-                   double *vm_node, cudaStream_t s) {
+// sum over the node's elements of E_e M u_e, restricted to the node's corner; returns their number
+__device__ __noinline__ int corner_products(const double *__restrict__ u, const double *__restrict__ E,
+                                            const uint8_t *__restrict__ eact, int ny, int nx, int nz, int iy, int ix,
+                                            int iz, double *acc) {
+    // reference corner order j: offsets (dy, dx, dz)
+    const int cdy[8] = {1, 1, 0, 0, 1, 1, 0, 0}, cdx[8] = {0, 1, 1, 0, 0, 1, 1, 0}, cdz[8] = {0, 0, 0, 0, 1, 1, 1, 1};
+    const int NY = ny + 1, NX = nx + 1;
+    int cnt = 0;
+    for (int j = 0; j < 8; ++j) {
+        const int ey = iy - cdy[j], ex = ix - cdx[j], ez = iz - cdz[j];
+        if (ey < 0 || ex < 0 || ez < 0 || ey >= ny || ex >= nx || ez >= nz) continue;
+        const int64_t eidx = (int64_t)ey + (int64_t)ny * (ex + (int64_t)nx * ez);
+        if (!eact[eidx]) continue;
+        const double ev = E[eidx];
+        ++cnt;
+        for (int c = 0; c < 6; ++c) {
+            const double *row = c_M + (6 * j + c);   // column-major 48 x 24
+            double sacc = 0.0;
+            for (int i = 0; i < 24; ++i) {
+                const int k = i / 3;
+                const int64_t m = (int64_t)(ey + cdy[k]) + (int64_t)NY * ((ex + cdx[k]) + (int64_t)NX * (ez + cdz[k]));
+                sacc += row[48 * i] * u[3 * m + i % 3];
+            }
+            acc[c] += sacc * ev;
+        }
+    }
+    return cnt;
+}
+
+struct StressScale {
+    double c1, c2, c3;   // Hooke's law at E = 1: (1-nu) / .., nu / .., 1 / (2 (1 + nu))
+    double rc[9];        // 1 / (cell size * element count)
+};
+
+__global__ void __launch_bounds__(128) k_nodal_stress(const double *__restrict__ u, const double *__restrict__ E,
+                                                      const int64_t *__restrict__ map, int64_t nact,
+                                                      const uint8_t *__restrict__ eact, int ny, int nx, int nz,
+                                                      const __grid_constant__ StressScale sc,
+                                                      const int *__restrict__ nonfinite,
+                                                      double *__restrict__ s6, double *__restrict__ vm) {
+    const int NY = ny + 1, NX = nx + 1;
+    const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i0 >= nact) return;
+    const int64_t n = map[i0];
+    const int64_t row = n / NY;
+    const int iy = (int)(n - row * NY), ix = (int)(row % NX), iz = (int)(row / NX);
+    double v[6] = {0, 0, 0, 0, 0, 0};
+    if (*nonfinite) {
+        const int cnt = corner_products(u, E, eact, ny, nx, nz, iy, ix, iz, v);
+        for (int c = 0; c < 6; ++c) v[c] /= (double)cnt;
+    } else {
+        // moduli and activity of the 8 elements; index bit 0 = +row (y), 1 = +x, 2 = +z side
+        double e[8];
+        unsigned act = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int ey = iy - 1 + (k & 1), ex = ix - 1 + ((k >> 1) & 1), ez = iz - 1 + (k >> 2);
+            e[k] = 0.0;
+            if (ey < 0 || ex < 0 || ez < 0 || ey >= ny || ex >= nx || ez >= nz) continue;
+            const int64_t i = (int64_t)ey + (int64_t)ny * (ex + (int64_t)nx * ez);
+            if (!eact[i]) continue;
+            act |= 1u << k;
+            e[k] = E[i];
+        }
+        double un[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) un[c] = u[3 * n + c];
+        // g[ax][c] = sum_e E_e du_c/d(axis), axes x, y (against the rows), z, times the cell size
+        double g[3][3] = {};
+        auto side = [&](int ax, unsigned mask, int64_t m, double sign) {
+            if (!(act & mask)) return;   // no solid element on this side
+            double es = 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (mask >> k & 1) es += e[k];
+            es *= sign;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) g[ax][c] = fma(es, u[3 * m + c] - un[c], g[ax][c]);
+        };
+        const int64_t dx = NY, dz = (int64_t)NY * NX;
+        side(0, 0xccu, n + dx, 1.0);
+        side(0, 0x33u, n - dx, -1.0);
+        side(1, 0xaau, n + 1, -1.0);
+        side(1, 0x55u, n - 1, 1.0);
+        side(2, 0xf0u, n + dz, 1.0);
+        side(2, 0x0fu, n - dz, -1.0);
+        const double r = sc.rc[__popc(act)], a1 = sc.c1 * r, a2 = sc.c2 * r, a3 = sc.c3 * r;
+        v[0] = a1 * g[0][0] + a2 * (g[1][1] + g[2][2]);
+        v[1] = a1 * g[1][1] + a2 * (g[0][0] + g[2][2]);
+        v[2] = a1 * g[2][2] + a2 * (g[0][0] + g[1][1]);
+        v[3] = a3 * (g[2][1] + g[1][2]);
+        v[4] = a3 * (g[2][0] + g[0][2]);
+        v[5] = a3 * (g[1][0] + g[0][1]);
+    }
+    double2 *o = reinterpret_cast<double2 *>(s6 + 6 * n);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[c] = make_double2(v[2 * c], v[2 * c + 1]);
+    const double a = v[0] - v[1], b = v[1] - v[2], d = v[2] - v[0];
+    vm[i0] = sqrt(0.5 * (a * a + b * b + d * d) + 3.0 * (v[5] * v[5] + v[3] * v[3] + v[4] * v[4]));
+}
+
+// map: the nact active nodes; nodal6 (full grid) is written at active nodes, vm_node is compact;
+// flag: a device int
+void launch_stress(const Level &l0, const double *E, const double *u, const double *M48x24, double nu, double cell,
+                   const int64_t *map, int64_t nact, int *flag, double *nodal6, double *vm_node, cudaStream_t s) {
     cudaMemcpyToSymbolAsync(c_M, M48x24, sizeof(double) * 48 * 24, 0, cudaMemcpyHostToDevice, s);
-    const int64_t nn = l0.nnode;
-    ++g_launches;
-    k_nodal_stress<<<(unsigned)((nn + 127) / 128), 128, 0, s>>>(u, E, l0.nflag, l0.eact, l0.ny, l0.nx, l0.nz, nodal6, vm_node);
+    cudaMemsetAsync(flag, 0, sizeof(int), s);
+    StressScale sc;
+    const double c = (1 + nu) * (1 - 2 * nu);
+    sc.c1 = (1 - nu) / c;
+    sc.c2 = nu / c;
+    sc.c3 = 1.0 / (2 * (1 + nu));
+    sc.rc[0] = 0.0;
+    for (int k = 1; k <= 8; ++k) sc.rc[k] = 1.0 / (cell * k);
+    g_launches += 2;
+    k_any_nonfinite<<<reduce_blocks(3 * l0.nnode), 256, 0, s>>>(u, 3 * l0.nnode, flag);
+    k_nodal_stress<<<(unsigned)((nact + 127) / 128), 128, 0, s>>>(u, E, map, nact, l0.eact, l0.ny, l0.nx, l0.nz, sc,
+                                                                  flag, nodal6, vm_node);
 }
 
 // per-element: centroid stress = mean of the 8 nodal stresses, von Mises,
 // then the reference's extra square root (FEA_ComputePerElementVonMisesStress.m:10-19).
-__global__ void k_elem_vm(const double *__restrict__ s6, const uint8_t *__restrict__ eact, int ny, int nx, int nz,
+// A thread per solid element (map), result compact: the FP64 pipe bounds it, and lanes
+// of void elements would take their share.
+__global__ void k_elem_vm(const double *__restrict__ s6, const int64_t *__restrict__ map, int64_t nact, int ny, int nx,
                           double *__restrict__ vme) {
-    const int64_t nel = (int64_t)ny * nx * nz;
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= nel) return;
-    if (!eact[e]) {
-        vme[e] = 0.0;
-        return;
-    }
-    const int ey = (int)(e % ny), ex = (int)((e / ny) % nx), ez = (int)(e / ((int64_t)ny * nx));
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= nact) return;
+    const int64_t e = map[i], row = e / ny;
+    const int ey = (int)(e - row * ny), ex = (int)(row % nx), ez = (int)(row / nx);
     const int NY = ny + 1, NX = nx + 1;
     const int cdy[8] = {1, 1, 0, 0, 1, 1, 0, 0}, cdx[8] = {0, 1, 1, 0, 0, 1, 1, 0}, cdz[8] = {0, 0, 0, 0, 1, 1, 1, 1};
     double v[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
     for (int k = 0; k < 8; ++k) {
         const int64_t m = (int64_t)(ey + cdy[k]) + (int64_t)NY * ((ex + cdx[k]) + (int64_t)NX * (ez + cdz[k]));
-        for (int c = 0; c < 6; ++c) v[c] += 0.125 * s6[6 * m + c];
+        const double2 *sm = reinterpret_cast<const double2 *>(s6 + 6 * m);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double2 t = sm[c];
+            v[2 * c] += 0.125 * t.x;
+            v[2 * c + 1] += 0.125 * t.y;
+        }
     }
     const double a = v[0] - v[1], b = v[1] - v[2], d = v[2] - v[0];
-    vme[e] = sqrt(sqrt(0.5 * (a * a + b * b + d * d) + 3.0 * (v[5] * v[5] + v[3] * v[3] + v[4] * v[4])));
+    vme[i] = sqrt(sqrt(0.5 * (a * a + b * b + d * d) + 3.0 * (v[5] * v[5] + v[3] * v[3] + v[4] * v[4])));
 }
 
-void launch_elem_vm(const Level &l0, const double *nodal6, double *vm_elem_full, cudaStream_t s) {
-    const int64_t nel = l0.nel;
+void launch_elem_vm(const Level &l0, const double *nodal6, const int64_t *map, int64_t nact, double *vm_elem,
+                    cudaStream_t s) {
     ++g_launches;
-    k_elem_vm<<<(unsigned)((nel + 255) / 256), 256, 0, s>>>(nodal6, l0.eact, l0.ny, l0.nx, l0.nz, vm_elem_full);
+    k_elem_vm<<<(unsigned)((nact + 127) / 128), 128, 0, s>>>(nodal6, map, nact, l0.ny, l0.nx, vm_elem);
 }
 
 }  // namespace sgld

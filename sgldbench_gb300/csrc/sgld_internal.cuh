@@ -304,9 +304,10 @@ void launch_set_passive_x(const Level &l0, double *x, int nb, cudaStream_t s);
 void launch_mark_passive(const Level &l0, const int64_t *full, int64_t np, int nb, cudaStream_t s);
 void launch_unit_compliance(const Level &l0, const double *u, const double *E, double *ce_full,
                             double *partial, int *nblocks_out, cudaStream_t s);
-void launch_stress(const Level &l0, const double *E, const double *u, const double *M48x24,
-                   double *nodal6, double *vm_node, cudaStream_t s);
-void launch_elem_vm(const Level &l0, const double *nodal6, double *vm_elem_full, cudaStream_t s);
+void launch_stress(const Level &l0, const double *E, const double *u, const double *M48x24, double nu, double cell,
+                   const int64_t *map, int64_t nact, int *flag, double *nodal6, double *vm_node, cudaStream_t s);
+void launch_elem_vm(const Level &l0, const double *nodal6, const int64_t *map, int64_t nact, double *vm_elem,
+                    cudaStream_t s);
 void launch_principal(const Level &l0, const double *s6, double *ps_node, double *dir_elem, cudaStream_t s);
 // PDE density filter (kernels_pde.cu)
 void upload_kpde(const double *K, double *d_kp, cudaStream_t s);
@@ -333,6 +334,8 @@ void launch_diag_from_Ks(const Level &l, double *diag, cudaStream_t s);
 void launch_inverse_diag(const Level &l, cudaStream_t s);   // l.idiag, l.idiag32 from l.diag
 void launch_scatter_nodes(const int64_t *map, int64_t n, const double *compact, double *full, cudaStream_t s);
 void launch_gather_nodes(const int64_t *map, int64_t n, const double *full, double *compact, cudaStream_t s);
+// dst[per * i + c] = src[per * map[i] + c]; per in {1, 3, 6, 12}
+void launch_gather_rows(const int64_t *map, int64_t n, int per, const double *src, double *dst, cudaStream_t s);
 void launch_scatter_elems(const int64_t *map, int64_t n, const double *compact, double *full, cudaStream_t s);
 void launch_gather_elems(const int64_t *map, int64_t n, const double *full, double *compact, cudaStream_t s);
 void launch_fixed_indicator(const Level &l, double *v, cudaStream_t s);
