@@ -14,9 +14,11 @@
 //    applies its sparse Cholesky factor with two triangular solves
 //    (src/Solving_Vcycle.m:116-118); M' M gives the same numbers to rounding
 //    and turns two sequential solves into parallel mat-vecs.
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <atomic>
+#include <utility>
 #include <vector>
 
 #include "sgld_internal.cuh"
@@ -789,78 +791,82 @@ int coarse_factor_invert(Ctx &c) {
 // ---- coarse apply: x_L[free] = A^-1 r_L[free] = M' (M r) -------------------------
 // The inverse factor is stored square: M (lower triangle, column-major) and
 // its transpose in the upper triangle, so that both products are column-major
-// GEMVs with coalesced loads.  A CTA covers 32 output rows and one of CSPLIT
-// column chunks; each warp takes 32-column blocks of the chunk, lane l holding
-// row i0 + l: its 32 loads of a block (one coalesced row segment per column)
-// are independent and in flight together.  The 8 warps' sums meet in shared
-// memory and the chunk's partial goes to part[chunk * n + row].
+// GEMVs with coalesced loads.
 //   lower (UPPER = false): y_i = sum_{j <= i} M[i + n j] v[rows[j]]
-//   upper (UPPER = true):  x_j = sum_{i >= j} M[j + n i] v[i]   (= (M' v)_j)
-constexpr int CL_WARPS = 8;
+//   upper (UPPER = true):  x[rows[j]] = sum_{i >= j} M[j + n i] v[i]   (= (M' v)_j)
+// A cluster of CL_CTAS CTAs covers 32 output rows.  Their columns are dealt to the
+// cluster's 64 warps in blocks of 32, so the triangle's short and long rows
+// load all of them alike; lane l holds row i0 + l, and the 32 loads of a block
+// (one coalesced row segment per column) are in flight together.  The warps' sums
+// meet in shared memory, the CTAs' sums in the first CTA's through distributed
+// shared memory, where they are added in a fixed order.  Chunk partials in global
+// memory cost two more launches and a memset of x per apply: the FP32 V-cycle of
+// 384 x 192 x 192 blobs (1300 rows) went from 214 to 193 us, of 256 x 128 x 128
+// (3888 rows) from 151 to 136, of 96 x 48 x 48 from 63 to 53.
+constexpr int CL_WARPS = 8, CL_CTAS = 8;
 
 template <typename T, bool UPPER>
-__global__ void __launch_bounds__(32 * CL_WARPS) k_coarse_gemv(const T *__restrict__ M, const int *__restrict__ rows,
-                                                              const T *__restrict__ v, int n,
-                                                              double *__restrict__ part) {
+__global__ void __cluster_dims__(1, CL_CTAS, 1) __launch_bounds__(32 * CL_WARPS)
+    k_coarse_gemv(const T *__restrict__ M, const int *__restrict__ rows, const int *__restrict__ pos, int ndof,
+                  const T *__restrict__ v, int n, T *__restrict__ y) {
+    namespace cg = cooperative_groups;
     __shared__ T red[CL_WARPS][32];
+    __shared__ double sums[CL_CTAS][32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = blockIdx.x * 32, i = i0 + lane;
-    const int chunk = ((n + CSPLIT - 1) / CSPLIT + 31) & ~31;
-    int j0 = blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-    if (UPPER)
-        j0 = max(j0, i0);
-    else
-        j1 = min(j1, i0 + 32);
-    const int ii = min(i, n - 1);
+    const int i0 = blockIdx.x * 32, i = i0 + lane, ii = min(i, n - 1);
+    auto cluster = cg::this_cluster();
+    auto started = cluster.barrier_arrive();   // every CTA of the cluster runs before its memory is written
+    const int first = UPPER ? i0 : 0, last = UPPER ? n : min(n, i0 + 32);
     T acc = T(0);
-    for (int jb = j0 + 32 * w; jb < j1; jb += 32 * CL_WARPS) {
+    for (int jb = first + 32 * (w + CL_WARPS * (int)blockIdx.y); jb < last; jb += 32 * CL_WARPS * CL_CTAS) {
         const int jl = jb + lane;
         const T vl = (jl < n) ? (UPPER ? v[jl] : v[rows[jl]]) : T(0);
-        T a0 = T(0), a1 = T(0);
+        T m[32];
 #pragma unroll
-        for (int q = 0; q < 32; q += 2) {
-            const int ja = jb + q, jc = jb + q + 1;
-            const T ma = (ja < n) ? M[(int64_t)ja * n + ii] : T(0);
-            const T mc = (jc < n) ? M[(int64_t)jc * n + ii] : T(0);
-            const T va = __shfl_sync(0xffffffffu, vl, q), vc = __shfl_sync(0xffffffffu, vl, q + 1);
-            a0 += (UPPER ? ja >= i : ja <= i) ? ma * va : T(0);
-            a1 += (UPPER ? jc >= i : jc <= i) ? mc * vc : T(0);
+        for (int q = 0; q < 32; ++q) m[q] = (jb + q < n) ? M[(int64_t)(jb + q) * n + ii] : T(0);
+        T a[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            const T vq = __shfl_sync(0xffffffffu, vl, q);
+            // the other triangle holds the transpose
+            if (UPPER ? jb + q >= i : jb + q <= i) a[q & 3] += m[q] * vq;
         }
-        acc += a0 + a1;
+        acc += (a[0] + a[1]) + (a[2] + a[3]);
     }
     red[w][lane] = acc;
     __syncthreads();
-    if (w == 0 && i < n) {
+    cluster.barrier_wait(std::move(started));
+    if (w == 0) {
         double sum = 0.0;
 #pragma unroll
         for (int k = 0; k < CL_WARPS; ++k) sum += (double)red[k][lane];
-        part[(int64_t)blockIdx.y * n + i] = sum;
+        cluster.map_shared_rank(&sums[0][0], 0)[32 * blockIdx.y + lane] = sum;
     }
-}
-
-// y_i = sum of the chunk partials (compact), or x[rows[i]] = that sum (scatter)
-template <typename T, bool SCATTER>
-__global__ void k_coarse_sum(const double *__restrict__ part, int n, const int *__restrict__ rows,
-                             T *__restrict__ y) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = 0.0;
-    for (int k = 0; k < CSPLIT; ++k) s += part[(int64_t)k * n + i];
-    y[SCATTER ? rows[i] : i] = (T)s;
+    cluster.sync();
+    if (blockIdx.y == 0 && w == 0 && i < n) {
+        double sum = 0.0;
+#pragma unroll
+        for (int k = 0; k < CL_CTAS; ++k) sum += sums[k][lane];
+        y[UPPER ? rows[i] : i] = (T)sum;
+    }
+    // x is zero off the free DOFs
+    if (UPPER && blockIdx.x == 0 && blockIdx.y == 1)
+        for (int d = threadIdx.x; d < ndof; d += 32 * CL_WARPS)
+            if (pos[d] < 0) y[d] = T(0);
 }
 
 template <typename T>
 static void coarse_apply(const Ctx &c, const T *M, const T *rc, T *xc, T *ybuf, cudaStream_t s) {
-    const Level &lc = c.lv[c.L - 1];
-    cudaMemsetAsync(xc, 0, sizeof(T) * 3 * lc.nnode, s);
-    if (c.ncf == 0) return;
-    const dim3 g((c.ncf + 31) / 32, CSPLIT);
-    const unsigned gs = (unsigned)((c.ncf + 127) / 128);
-    g_launches += 4;
-    k_coarse_gemv<T, false><<<g, 32 * CL_WARPS, 0, s>>>(M, c.d_cfree, rc, c.ncf, c.d_cpart);
-    k_coarse_sum<T, false><<<gs, 128, 0, s>>>(c.d_cpart, c.ncf, c.d_cfree, ybuf);
-    k_coarse_gemv<T, true><<<g, 32 * CL_WARPS, 0, s>>>(M, c.d_cfree, ybuf, c.ncf, c.d_cpart);
-    k_coarse_sum<T, true><<<gs, 128, 0, s>>>(c.d_cpart, c.ncf, c.d_cfree, xc);
+    const int ndof = (int)(3 * c.lv[c.L - 1].nnode);
+    if (c.ncf == 0) {
+        cudaMemsetAsync(xc, 0, sizeof(T) * ndof, s);
+        return;
+    }
+    const dim3 g((c.ncf + 31) / 32, CL_CTAS);
+    const int *pos = c.d_cfree + c.ncf;
+    g_launches += 2;
+    k_coarse_gemv<T, false><<<g, 32 * CL_WARPS, 0, s>>>(M, c.d_cfree, pos, ndof, rc, c.ncf, ybuf);
+    k_coarse_gemv<T, true><<<g, 32 * CL_WARPS, 0, s>>>(M, c.d_cfree, pos, ndof, ybuf, c.ncf, xc);
 }
 
 void launch_coarse_apply_f64(const Ctx &c, const double *rc, double *xc, cudaStream_t s) {

@@ -981,7 +981,7 @@ void sgld_destroy(sgld_ctx *ctx) {
     for (void *p : {(void *)c.d_nodemap, (void *)c.d_elemap, (void *)c.E, (void *)c.d_E32, (void *)c.d_b,
                     (void *)c.d_x, (void *)c.d_r, (void *)c.d_z, (void *)c.d_p, (void *)c.d_q, (void *)c.d_tmp,
                     (void *)c.d_r32, (void *)c.d_z32, (void *)c.d_part, (void *)c.d_scal, (void *)c.d_iflag,
-                    (void *)c.d_Ac, (void *)c.d_Ainv, (void *)c.d_Ainv32, (void *)c.d_cpart, (void *)c.d_cfree,
+                    (void *)c.d_Ac, (void *)c.d_Ainv, (void *)c.d_Ainv32, (void *)c.d_cfree,
                     (void *)c.d_H, (void *)ctx->d_s6, (void *)ctx->d_vmn, (void *)ctx->d_vme, (void *)c.d_e32,
                     (void *)c.d_s32, (void *)c.d_d32, (void *)c.d_t32, (void *)c.d_isc, (void *)c.d_part2, (void *)c.d_LB,
                     (void *)c.d_cy})
@@ -1144,10 +1144,10 @@ int sgld_set_fixed_dofs(sgld_ctx *ctx, const uint8_t *fixed) {
             }
     ctx->h_rows = rows;
     if (ncf != c.ncf || band != c.cband || !c.d_cfree) {
-        for (void *p : {(void *)c.d_Ac, (void *)c.d_Ainv, (void *)c.d_Ainv32, (void *)c.d_cpart, (void *)c.d_cfree,
+        for (void *p : {(void *)c.d_Ac, (void *)c.d_Ainv, (void *)c.d_Ainv32, (void *)c.d_cfree,
                         (void *)c.d_LB, (void *)c.d_cy})
             if (p) cudaFree(p);
-        c.d_Ac = c.d_Ainv = c.d_LB = c.d_cy = c.d_cpart = nullptr;
+        c.d_Ac = c.d_Ainv = c.d_LB = c.d_cy = nullptr;
         c.d_Ainv32 = nullptr;
         c.d_cfree = nullptr;
         c.ncf = ncf;
@@ -1155,7 +1155,6 @@ int sgld_set_fixed_dofs(sgld_ctx *ctx, const uint8_t *fixed) {
         CK(dalloc(&c.d_Ac, (size_t)ncf * ncf));
         CK(dalloc(&c.d_Ainv, (size_t)ncf * ncf));
         CK(dalloc(&c.d_Ainv32, (size_t)ncf * ncf));
-        CK(dalloc(&c.d_cpart, (size_t)CSPLIT * ncf));
         // band + 1/diag + inverses of the 32 x 32 diagonal blocks, as float pairs
         CK(dalloc(&c.d_LB, (size_t)ncf * (band + 1) + ncf + (size_t)((ncf + 31) / 32) * 1024));
         CK(dalloc(&c.d_cy, 2 * (size_t)ncf));

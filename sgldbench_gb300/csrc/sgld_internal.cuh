@@ -114,7 +114,6 @@ struct Ctx {
     int trinv_g = 16;               // columns per CTA of the L^-1 sweeps (narrower for wide bands)
     size_t trinv_smem = 0;
     bool m64_valid = false;         // d_Ainv holds L^-1 of the current factorization (made on first use)
-    double *d_cpart = nullptr;      // [CSPLIT*ncf] GEMV partials
     // templates for the level-2 Galerkin assembly
     double *d_H = nullptr;          // [2 (8 + 64) * 576] templates for span 2, span 4, then both as
                                     // (hi, lo) float pairs
@@ -166,8 +165,6 @@ struct sgld_ctx {
 };
 
 namespace sgld {
-
-constexpr int CSPLIT = 16;   // column chunks of the coarse GEMV
 
 // learned warm start of the SIMP loop (sgld_learned.cu)
 void learned_free(LearnedWS *w);
