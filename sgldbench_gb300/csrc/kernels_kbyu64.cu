@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
     auto modulus = [&](int z) { return ein && z >= 0 && z < nz ? ep[eplane * z] : 0.0; };
 
     double Fp[12], carry[12], dot = 0.0;
+    bool live = false;   // carry is not zero
 #pragma unroll
     for (int i = 0; i < 12; ++i) Fp[i] = carry[i] = 0.0;
     stage(z0 - 1);
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
             // the faces of layer ez + 1 are needed by the elements below and above them
             if (ev != 0.0 || en != 0.0) faces(Ft);
             double phi[12];
+            live |= ev != 0.0;
             if (ev != 0.0) {
                 double h[24];
 #pragma unroll
@@ -258,12 +260,18 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
                 }
             }
             // x butterfly undone: column lx gets phi0 - phi1, column lx + 1 phi0 + phi1
+            if (live) {
 #pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                const int k = i < 3 ? i : i + 3;
-                sl[i * tn + tid] = phi[k] - phi[k + 3];
-                rp[i] = phi[k] + phi[k + 3];
+                for (int i = 0; i < 6; ++i) {
+                    const int k = i < 3 ? i : i + 3;
+                    sl[i * tn + tid] = phi[k] - phi[k + 3];
+                    rp[i] = phi[k] + phi[k + 3];
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 6; ++i) sl[i * tn + tid] = rp[i] = 0.0;
             }
+            live = ev != 0.0;   // carried up
             if (en != 0.0) {
 #pragma unroll
                 for (int i = 0; i < 12; ++i) Fp[i] = Ft[i];
@@ -316,11 +324,16 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
 // up) x (zc + 1) layers x warps x 137 operations at 16 clocks a warp, plus the
 // barriers' latency per layer and a CTA's start.  Small grids get many small
 // CTAs that fill the SMs, large ones tiles whose ragged edge and halo are
-// small.  At most SGLD_NOALLOC_MAX_CTAS CTAs, the scratch of the
+// small.  On a grid with void regions the CTAs' work differs from tile to tile, and
+// the last one to start decides: there the cost is the active share of the work,
+// spread evenly, plus one whole CTA.  (With the solid grid's rule the 384 x 192 x 192
+// blob shape took 3.69 ms, with this one 2.01; the fixed 32 x 8 x 16 tile 3.28.)  At most SGLD_NOALLOC_MAX_CTAS CTAs, the scratch of the
 // allocation-free call, where the grid allows it.
 void kbyu64_pick_tile(Level &l) {
     const int NY = l.ny + 1, NX = l.nx + 1, NZ = l.nz + 1;
     constexpr int SMS = 152, MAX_CTAS = 32768;
+    const double fill = (double)l.nnode_active / (double)l.nnode;
+    const bool solid = fill > 0.85;
     double best = 0.0;
     l.k64_ye = 0;
     for (int ty = 1; ty <= NY; ++ty) {   // tiles along y: the smallest ye that needs no more of them
@@ -340,7 +353,8 @@ void kbyu64_pick_tile(Level &l) {
                 if (zc < 2 && tz > 1) break;
                 const int64_t n = (int64_t)ty * tx * tz;
                 const double layer = nt / 32 * (137.0 * 16.0) + 600.0;
-                double cost = (double)((n + SMS - 1) / SMS) * ((zc + 1) * layer + 3000.0);
+                const double rounds = solid ? (double)((n + SMS - 1) / SMS) : fill * (double)n / SMS + 1.0;
+                double cost = rounds * ((zc + 1) * layer + 3000.0);
                 if (n > MAX_CTAS) cost *= 1e6;
                 if (!l.k64_ye || cost < best) {
                     best = cost;
