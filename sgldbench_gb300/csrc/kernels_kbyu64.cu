@@ -41,7 +41,7 @@ void upload_kh64(const double *Kh, const double *kc, cudaStream_t s) {
 namespace k64 {
 constexpr int MAX_THREADS = 384;   // at 168 registers a thread
 constexpr int STAGE = 5;           // staged words per thread and node layer, at most
-constexpr int SLOTS = 3;           // node layers in shared memory
+constexpr int SLOTS = 4;           // node layers in shared memory
 
 __host__ __device__ constexpr int threads(int ye, int xe) { return (ye * xe + 31) & ~31; }
 constexpr int node_words(int ye, int xe) { return 3 * (ye + 1) * (xe + 1); }
@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
             off[k] = (py >= 0 && py < NY && px >= 0 && px < NX) ? 3 * (py + NY * px) + c : -1;
         }
     }
-    auto stage = [&](int z) {   // node layer z into slot z mod 3
-        double *dst = su + (z + 3) % k64::SLOTS * nw;
+    auto stage = [&](int z) {   // node layer z into its slot
+        double *dst = su + ((z + k64::SLOTS) % k64::SLOTS) * nw;
         const double *src = u + 3 * plane * z;
         const bool zin = z >= 0 && z < NZ;
 #pragma unroll
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
     // y butterflies of the edges of node layer z: sum and u(ly) - u(ly+1)
     auto edges = [&](int z) {
         if (!elem) return;
-        const double *p = su + (z + 3) % k64::SLOTS * nw + 3 * (ly + (ye + 1) * lx);
+        const double *p = su + ((z + k64::SLOTS) % k64::SLOTS) * nw + 3 * (ly + (ye + 1) * lx);
         for (int x = lx;; ++x, p += 3 * (ye + 1)) {   // the last column's threads also form the column past it
             double *o = se + ly + ye * x;
 #pragma unroll
@@ -220,10 +220,27 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
     double ev = modulus(z0 - 1), en = modulus(z0);
     if (elem && ev != 0.0) faces(Fp);
     __syncthreads();
+    edges(z0);
+    // node layer ez, one barrier after its shares were written
+    double lo[3] = {0.0, 0.0, 0.0};
+    auto output = [&](int ez) {
+        if (!owner || ez < z0) return;
+        const int64_t node = gy + (int64_t)NY * gx + plane * ez;
+        const uint8_t f = nflag[node];
+        const double *un = su + ((ez + k64::SLOTS) % k64::SLOTS) * nw + 3 * (ly + 1 + (ye + 1) * (lx + 1));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double o = (f & (NF_FIXX << c)) ? 0.0 : lo[c] + sn[c * tn + tid + 1];
+            y[3 * node + c] = o;
+            if (DOT) dot = fma(un[c], o, dot);
+        }
+    };
+    // two barriers per element layer: the edges of the next node layer are formed with the
+    // undone edges of this one, a node layer is written a barrier later
     for (int ez = z0 - 1; ez < zend; ++ez) {
         // element layer ez between node layers ez (faces Fp) and ez + 1
-        edges(ez + 1);
         __syncthreads();
+        output(ez - 1);
         if (ez + 2 <= zend) stage(ez + 2);
         double rp[6];
         if (elem) {
@@ -279,10 +296,10 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
             ev = en;
             en = modulus(ez + 2);
         }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
         // edge of column lx + 1: this element's right part and the next column's left part; y
         // butterfly undone: node ly + 1 gets t0 - t1, node ly gets t0 + t1
-        double lo[3];
         if (elem && lx < xe - 1) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -291,20 +308,10 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
                 sn[c * tn + tid] = t0 + t1;
             }
         }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();
-        if (owner && ez >= z0) {
-            const int64_t node = gy + (int64_t)NY * gx + plane * ez;
-            const uint8_t f = nflag[node];
-            const double *un = su + (ez + 3) % k64::SLOTS * nw + 3 * (ly + 1 + (ye + 1) * (lx + 1));
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const double o = (f & (NF_FIXX << c)) ? 0.0 : lo[c] + sn[c * tn + tid + 1];
-                y[3 * node + c] = o;
-                if (DOT) dot = fma(un[c], o, dot);
-            }
-        }
+        if (ez + 1 < zend) edges(ez + 2);
     }
+    __syncthreads();
+    output(zend - 1);
     if (DOT) {
         __shared__ double red[k64::MAX_THREADS / 32];
 #pragma unroll
@@ -319,16 +326,18 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
     }
 }
 
-// The tile for a grid: the FP64 pipe runs a CTA's element layers one after the
-// other, so a tile's cost is the work of the busiest SM, (CTAs / 152 rounded
-// up) x (zc + 1) layers x warps x 137 operations at 16 clocks a warp, plus the
-// barriers' latency per layer and a CTA's start.  Small grids get many small
-// CTAs that fill the SMs, large ones tiles whose ragged edge and halo are
-// small.  On a grid with void regions the CTAs' work differs from tile to tile, and
-// the last one to start decides: there the cost is the active share of the work,
-// spread evenly, plus one whole CTA.  (With the solid grid's rule the 384 x 192 x 192
-// blob shape took 3.69 ms, with this one 2.01; the fixed 32 x 8 x 16 tile 3.28.)  At most SGLD_NOALLOC_MAX_CTAS CTAs, the scratch of the
-// allocation-free call, where the grid allows it.
+// The tile for a grid, by the FP64 work of the busiest SM.  Its CTAs, (CTAs / 152
+// rounded up), run as many at a time as fit into 384 threads; each of the SM's four
+// schedulers takes a quarter of their warps, rounded up, and needs 64 clocks per
+// FP64 instruction and warp, 137 instructions per element layer; a layer costs
+// about 2000 clocks of latency and barriers besides, a CTA's start 6000.  Small grids
+// get many small CTAs that fill the SMs, large ones tiles whose ragged edge and
+// halo are small.  On a grid with void regions the CTAs' work differs from tile to
+// tile, and the last one to start decides: there the cost is the active share of
+// the work, spread evenly, plus one whole CTA.  (With the solid grid's rule the 384 x
+// 192 x 192 blob shape took 3.69 ms, with this one 2.01; the fixed 32 x 8 x 16 tile
+// 3.28.)  At most SGLD_NOALLOC_MAX_CTAS CTAs, the scratch of the allocation-free
+// call, where the grid allows it.
 void kbyu64_pick_tile(Level &l) {
     const int NY = l.ny + 1, NX = l.nx + 1, NZ = l.nz + 1;
     constexpr int SMS = 152, MAX_CTAS = 32768;
@@ -352,9 +361,17 @@ void kbyu64_pick_tile(Level &l) {
                 if ((NZ + zc - 1) / zc != tz) continue;
                 if (zc < 2 && tz > 1) break;
                 const int64_t n = (int64_t)ty * tx * tz;
-                const double layer = nt / 32 * (137.0 * 16.0) + 600.0;
-                const double rounds = solid ? (double)((n + SMS - 1) / SMS) : fill * (double)n / SMS + 1.0;
-                double cost = rounds * ((zc + 1) * layer + 3000.0);
+                // clocks per layer of k CTAs together, and of a CTA's share of that
+                const int w = nt / 32, fit = k64::MAX_THREADS / nt;
+                auto layer = [&](int k) { return (k * w + 3) / 4 * 64.0 * 137.0 + 2000.0; };
+                auto clocks = [&](double per_layer) { return (zc + 1) * per_layer + 6000.0; };
+                double cost;
+                if (solid) {
+                    const int64_t r = (n + SMS - 1) / SMS;   // CTAs of the busiest SM
+                    cost = (double)(r / fit) * clocks(layer(fit)) + (r % fit ? clocks(layer((int)(r % fit))) : 0.0);
+                } else {
+                    cost = (fill * (double)n / SMS + 1.0) * clocks(layer(fit) / fit);
+                }
                 if (n > MAX_CTAS) cost *= 1e6;
                 if (!l.k64_ye || cost < best) {
                     best = cost;
