@@ -13,10 +13,10 @@
 //
 // The additive V-cycle of the reference (src/Solving_Vcycle.m:12-50) is
 //   r_l = R r_{l-1};  x_L = A_L^-1 r_L;
-//   x_{l} = t_l + P x_{l+1} + t_l  with t_l = (omega r_l) ./ D_l,
-// summed in that order.  1 ./ D_l is formed once per assembly (the division
-// is the most expensive FP64 operation of the cycle), so t_l may differ from
-// the reference's (omega r_l) ./ D_l in the last bit.
+//   x_{l} = t_l + P x_{l+1} + t_l  with t_l = (omega r_l) ./ D_l.
+// 2 omega ./ D_l is formed once per assembly, so a fine node takes one
+// multiply-add, x_l = r_l (2 omega / D_l) + P x_{l+1}, which may differ from the
+// reference's sum in the last bit.
 #include "sgld_internal.cuh"
 
 namespace sgld {
@@ -57,59 +57,122 @@ __global__ void k_restrict(const T *__restrict__ rf, T *__restrict__ rc, int nyc
     rc[3 * n + 2] = a2;
 }
 
-// The same restriction with the span S a compile-time constant (2): the
-// (2S-1)^3 taps unroll, the weights are constants and the indices stay 32-bit
-// (grids below 2^31 / 3 nodes).  Lanes hold consecutive coarse y, so for one
-// (dx, dz) a warp's taps cover a contiguous run of fine nodes.
-// A coarse node outside the active domain (cflag) gets 0 without reading the
-// fine grid: all 8 coarse elements around it are empty, so every fine node
-// strictly inside their union -- the tent's support -- is inactive and holds 0.
-// With keep_zeros (the FP32 V-cycle, whose coarse vectors are zeroed when
-// allocated) an inactive coarse node is not written at all: it holds 0 already.
-template <typename T, int S>
-__global__ void __launch_bounds__(128) k_restrict_s(const T *__restrict__ rf, T *__restrict__ rc,
-                                                    const uint8_t *__restrict__ cflag, int nyc, int nxc, int nzc,
-                                                    int keep_zeros) {
+// Span 2: lanes along y, 32-bit indices (grids below 2^31 / 3 nodes).  A coarse
+// node outside the active domain (cflag) gets 0 without reading the fine grid: all
+// 8 coarse elements around it are empty, so every fine node strictly inside
+// their union -- the tent's support -- is inactive and holds 0.
+//
+// FP32: a thread per coarse node.  Taps are read at clamped positions, those past
+// the grid with weight 0, so that no branch stands between the 81 loads: with one
+// per tap row they went out row by row, nine memory latencies one after the other
+// (384 x 192 x 192 blobs, finest level: 29.6 -> 25.0 us).  Inactive coarse nodes
+// are not written: the FP32 V-cycle's coarse vectors are zeroed when allocated.
+__global__ void __launch_bounds__(128) k_restrict2_f32(const float *__restrict__ rf, float *__restrict__ rc,
+                                                       const uint8_t *__restrict__ cflag, int nyc, int nxc, int nzc,
+                                                       int keep_zeros) {
     const int NYc = nyc + 1, NXc = nxc + 1;
-    const int NYf = S * nyc + 1, NXf = S * nxc + 1, NZf = S * nzc + 1;
+    const int NYf = 2 * nyc + 1, NXf = 2 * nxc + 1;
     const int pl = blockIdx.x * blockDim.x + threadIdx.x;
     if (pl >= NYc * NXc) return;
-    const int I = pl % NYc, J = pl / NYc, Kz = blockIdx.y;
-    if (!(cflag[pl + NYc * NXc * Kz] & NF_ACTIVE)) {
-        if (keep_zeros) return;
-        const int n = 3 * (pl + NYc * NXc * Kz);
-        rc[n] = rc[n + 1] = rc[n + 2] = T(0);
+    const int n = 3 * (pl + NYc * NXc * blockIdx.y);
+    if (!(cflag[n / 3] & NF_ACTIVE)) {
+        if (!keep_zeros) rc[n] = rc[n + 1] = rc[n + 2] = 0.f;
         return;
     }
-    const T inv = T(1) / T(S);
-    T a0 = T(0), a1 = T(0), a2 = T(0);
+    // offsets and weights of the three taps of each axis
+    int o[3][3];
+    float w[3][3];
+    const int c[3] = {pl % NYc, pl / NYc, (int)blockIdx.y}, m[3] = {nyc, nxc, nzc}, st[3] = {3, 3 * NYf, 3 * NYf * NXf};
 #pragma unroll
-    for (int dz = -S + 1; dz < S; ++dz) {
-        const int fz = S * Kz + dz;
-        if (fz < 0 || fz >= NZf) continue;
-        const T wz = T(S - (dz < 0 ? -dz : dz)) * inv;
-#pragma unroll
-        for (int dx = -S + 1; dx < S; ++dx) {
-            const int fx = S * J + dx;
-            if (fx < 0 || fx >= NXf) continue;
-            const T wxz = T(S - (dx < 0 ? -dx : dx)) * inv * wz;
-            const int base = NYf * (fx + NXf * fz);
-#pragma unroll
-            for (int dy = -S + 1; dy < S; ++dy) {
-                const int fy = S * I + dy;
-                if (fy < 0 || fy >= NYf) continue;
-                const T w = T(S - (dy < 0 ? -dy : dy)) * inv * wxz;
-                const int f = 3 * (fy + base);
-                a0 += w * rf[f];
-                a1 += w * rf[f + 1];
-                a2 += w * rf[f + 2];
-            }
-        }
+    for (int ax = 0; ax < 3; ++ax) {
+        o[ax][1] = st[ax] * 2 * c[ax];
+        o[ax][0] = c[ax] > 0 ? o[ax][1] - st[ax] : o[ax][1];
+        o[ax][2] = c[ax] < m[ax] ? o[ax][1] + st[ax] : o[ax][1];
+        w[ax][1] = 1.f;
+        w[ax][0] = c[ax] > 0 ? 0.5f : 0.f;
+        w[ax][2] = c[ax] < m[ax] ? 0.5f : 0.f;
     }
-    const int n = 3 * (pl + NYc * NXc * Kz);
-    rc[n] = a0;
-    rc[n + 1] = a1;
-    rc[n + 2] = a2;
+    float a[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int dz = 0; dz < 3; ++dz) {
+        float v[3][3][3];
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) v[dx][dy][q] = rf[o[0][dy] + o[1][dx] + o[2][dz] + q];
+        // y, then x, then z
+        float p[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                p[q] += w[1][dx] * (v[dx][1][q] + (w[0][0] * v[dx][0][q] + w[0][2] * v[dx][2][q]));
+#pragma unroll
+        for (int q = 0; q < 3; ++q) a[q] += w[2][dz] * p[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) rc[n + q] = a[q];
+}
+
+// FP64 is bound by its operations: a thread takes zp coarse planes of a column and
+// forms the sum over a fine plane's 9 taps once, as the plane between two coarse
+// planes serves both: 54 operations and 18 taps per node instead of 81 and 27
+// (256 x 128 x 128, finest level: 89 -> 75 us).
+__global__ void __launch_bounds__(128) k_restrict2_f64(const double *__restrict__ rf, double *__restrict__ rc,
+                                                       const uint8_t *__restrict__ cflag, int nyc, int nxc, int nzc,
+                                                       int zp) {
+    using T = double;
+    const int NYc = nyc + 1, NXc = nxc + 1;
+    const int NYf = 2 * nyc + 1, NXf = 2 * nxc + 1;
+    const int pl = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pl >= NYc * NXc) return;
+    const int I = pl % NYc, J = pl / NYc;
+    const bool y0 = I > 0, y1 = I < nyc, x0 = J > 0, x1 = J < nxc;
+    const int oy[3] = {y0 ? -3 : 0, 0, y1 ? 3 : 0}, ox[3] = {x0 ? -3 * NYf : 0, 0, x1 ? 3 * NYf : 0};
+    const int base = 3 * (2 * I + NYf * 2 * J), fplane = 3 * NYf * NXf;
+    // half-weighted neighbours along y and x of fine plane z
+    auto plane = [&](int z, T (&p)[3]) {
+        const T *r = rf + base + fplane * z;
+        T v[3][3][3];
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) v[dx][dy][q] = r[oy[dy] + ox[dx] + q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            T s[3];
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx)
+                s[dx] = v[dx][1][q] + T(0.5) * ((y0 ? v[dx][0][q] : T(0)) + (y1 ? v[dx][2][q] : T(0)));
+            p[q] = s[1] + T(0.5) * ((x0 ? s[0] : T(0)) + (x1 ? s[2] : T(0)));
+        }
+    };
+    const int K0 = blockIdx.y * zp, K1 = min(nzc + 1, K0 + zp);
+    T lo[3] = {T(0), T(0), T(0)};
+    bool have = K0 == 0;   // lo holds fine plane 2 K - 1
+    for (int K = K0; K < K1; ++K) {
+        const int n = 3 * (pl + NYc * NXc * K);
+        if (!(cflag[n / 3] & NF_ACTIVE)) {
+            rc[n] = rc[n + 1] = rc[n + 2] = T(0);
+            have = false;
+            continue;
+        }
+        T mid[3], up[3];
+        if (!have && K > 0) plane(2 * K - 1, lo);
+        plane(2 * K, mid);
+        plane(min(2 * K + 1, 2 * nzc), up);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            if (K == nzc) up[q] = T(0);
+            rc[n + q] = mid[q] + T(0.5) * ((K > 0 ? lo[q] : T(0)) + up[q]);
+            lo[q] = up[q];
+        }
+        have = true;
+    }
 }
 
 // Span 4: a warp per coarse node, whose lanes share the 7^3 taps (consecutive
@@ -159,9 +222,17 @@ void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *rc,
     // FP32: the coarse vectors (the levels' r32) are zeroed at allocation and keep zeros at
     // inactive nodes
     const int keep = sizeof(T) == sizeof(float) && static_cast<const void *>(rc) == coarse.r32;
-    if (small && coarse.span == 2)
-        k_restrict_s<T, 2><<<g, 128, 0, st>>>(rf, rc, coarse.nflag, coarse.ny, coarse.nx, coarse.nz, keep);
-    else if (small && coarse.span == 4)
+    if (small && coarse.span == 2) {
+        if constexpr (sizeof(T) == sizeof(float)) {
+            k_restrict2_f32<<<g, 128, 0, st>>>(rf, rc, coarse.nflag, coarse.ny, coarse.nx, coarse.nz, keep);
+        } else {
+            // 8 (else 4, 2, 1) coarse planes per CTA while that keeps 8 CTAs per SM
+            int zp = 8;
+            while (zp > 1 && (int64_t)g.x * ((coarse.nz + zp) / zp) < 152 * 8) zp >>= 1;
+            k_restrict2_f64<<<dim3(g.x, (unsigned)((coarse.nz + zp) / zp)), 128, 0, st>>>(
+                rf, rc, coarse.nflag, coarse.ny, coarse.nx, coarse.nz, zp);
+        }
+    } else if (small && coarse.span == 4)
         k_restrict4<T><<<dim3((unsigned)(((coarse.ny + 1) * (coarse.nx + 1) + 7) / 8), g.y), 256, 0, st>>>(
             rf, rc, coarse.nflag, coarse.ny, coarse.nx, coarse.nz, keep);
     else
@@ -184,12 +255,12 @@ __device__ __forceinline__ double warp_block_sum(T v, double *red) {
     return s;
 }
 
-// x_f = t + P x_c + t, t = (omega r_f) .* D on active fine nodes, 0 elsewhere,
-// where D holds the reciprocal Jacobi diagonal.
+// x_f = r_f .* D + P x_c on active fine nodes, 0 elsewhere, where D holds 2 omega
+// over the Jacobi diagonal.
 // FINAL (finest level): fixed DOFs set to 0 and partial sums of x_f . r_f.
 template <typename T, bool FINAL>
 __global__ void k_prolong_smooth(const T *__restrict__ xc, const T *__restrict__ rf, const T *__restrict__ D,
-                                 const uint8_t *__restrict__ nflag, T omega, T *__restrict__ xf, int nyc, int nxc,
+                                 const uint8_t *__restrict__ nflag, T *__restrict__ xf, int nyc, int nxc,
                                  int nzc, int s, double *__restrict__ partial) {
     const int NYc = nyc + 1, NXc = nxc + 1;
     const int NYf = s * nyc + 1, NXf = s * nxc + 1, NZf = s * nzc + 1;
@@ -228,10 +299,9 @@ __global__ void k_prolong_smooth(const T *__restrict__ xc, const T *__restrict__
                 }
             }
             const T r0 = rf[3 * n], r1 = rf[3 * n + 1], r2 = rf[3 * n + 2];
-            const T t0 = (omega * r0) * D[3 * n], t1 = (omega * r1) * D[3 * n + 1], t2 = (omega * r2) * D[3 * n + 2];
-            o0 = (t0 + p0) + t0;
-            o1 = (t1 + p1) + t1;
-            o2 = (t2 + p2) + t2;
+            o0 = r0 * D[3 * n] + p0;
+            o1 = r1 * D[3 * n + 1] + p1;
+            o2 = r2 * D[3 * n + 2] + p2;
             if (FINAL) {
                 if (f & NF_FIXX) o0 = T(0);
                 if (f & NF_FIXY) o1 = T(0);
@@ -250,118 +320,134 @@ __global__ void k_prolong_smooth(const T *__restrict__ xc, const T *__restrict__
     }
 }
 
-// The same operator with a thread per coarse node (I, J, K) writing the
-// fine nodes (S I + ry, S J + rx, S K + rz), 0 <= ry, rx, rz < S (only 0
-// past the last coarse cell of an axis): the 8 coarse corners are loaded once
-// per S^3 fine nodes instead of once per fine node, and the interpolation is
-// done axis by axis (z, then x, then y).  Span S is a compile-time constant,
-// indices are 32-bit.  Same result as k_prolong_smooth up to the order of the
-// interpolation sums.
+// Span 2: a thread per coarse node (I, J, K) writing the fine nodes (2 I + ry, 2 J +
+// rx, 2 K + rz), 0 <= ry, rx, rz < 2 (only 0 past the last coarse cell of an
+// axis): the 8 coarse corners are loaded once per 8 fine nodes, the upper 4 of
+// a plane are the lower 4 of the next (a CTA marches through zp planes), and the
+// interpolation is sums of 1, 2, 4 or 8 corners, axis by axis, scaled once.
+// Indices are 32-bit.  Same result as k_prolong_smooth up to the order of the sums.
+// All of a batch's loads (r, 1/D and flags of the cell's 8 fine nodes in FP32, of
+// 4 in FP64) are issued before the first is used, at clamped positions for the
+// nodes past the grid; with a branch around each fine node they went out node by
+// node, eight memory latencies per cell.  Finest level: FP32 384 x 192 x 192 blobs 76 ->
+// 53 us, FP64 (bound by its operations, 13.5 per node instead of 33) 256 x 128 x 128
+// 247 -> 131 us.
 // With cflag (the coarse node flags; passed for the FP32 V-cycle, whose output
 // vectors are zeroed when allocated), a thread whose 8 coarse corners are all
 // inactive writes nothing: every fine element touching one of its fine nodes
 // lies in a coarse element sharing a corner with the cell, and an active
 // coarse element makes all 8 of its corners active, so those fine nodes are
 // inactive and already hold 0.
-template <typename T, int S, bool FINAL>
+template <typename T, bool FINAL>
 __global__ void __launch_bounds__(128) k_prolong_cells(const T *__restrict__ xc, const T *__restrict__ rf,
                                                        const T *__restrict__ D, const uint8_t *__restrict__ nflag,
-                                                       const uint8_t *__restrict__ cflag, T omega,
+                                                       const uint8_t *__restrict__ cflag,
                                                        T *__restrict__ xf, int nyc, int nxc, int nzc, int zp,
                                                        double *__restrict__ partial) {
+    constexpr int BZ = sizeof(T) == 4 ? 2 : 1;   // fine planes per batch of loads
     const int NYc = nyc + 1, NXc = nxc + 1;
-    const int NYf = S * nyc + 1, NXf = S * nxc + 1;
+    const int NYf = 2 * nyc + 1, NXf = 2 * nxc + 1;
     const int pl = blockIdx.x * blockDim.x + threadIdx.x;
     T dot = T(0);
-    // coarse planes K = blockIdx.y * zp .. + zp - 1 (fewer CTAs, so fewer partial sums)
-    for (int K = blockIdx.y * zp; K < min(nzc + 1, (int)(blockIdx.y + 1) * zp); ++K) {
-    bool live = pl < NYc * NXc;
-    if (live && cflag) {
+    if (pl < NYc * NXc) {
         const int I = pl % NYc, J = pl / NYc;
-        bool any = false;
+        const int ly = I < nyc, lx = J < nxc;   // the cell has fine nodes at ry = 1, rx = 1
+        const int cpl = NYc * NXc, fpl = NYf * NXf;
+        // coarse corners of the cell's column: index b (x) 2 + a (y)
+        const int co[4] = {pl, pl + ly, pl + (lx ? NYc : 0), pl + ly + (lx ? NYc : 0)};
+        auto plane_active = [&](int K) {
+            bool any = false;
+            if (K <= nzc)
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
+                for (int k = 0; k < 4; ++k) any |= (cflag[co[k] + cpl * K] & NF_ACTIVE) != 0;
+            return any;
+        };
+        const int K0 = blockIdx.y * zp, K1 = min(nzc + 1, K0 + zp);
+        bool act0 = cflag ? plane_active(K0) : true, act1 = cflag ? plane_active(K0 + 1) : true;
+        T c0[4][3], c1[4][3];
+        bool have = false;   // c0 holds plane K
+        for (int K = K0; K < K1; ++K) {
+            const bool live = act0 || act1;
+            act0 = act1;
+            if (cflag) act1 = plane_active(K + 2);
+            if (!live) {
+                have = false;
+                continue;
+            }
+            const int lz = K < nzc, up = lz ? cpl : 0;
 #pragma unroll
-            for (int b = 0; b < 2; ++b)
+            for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int a = 0; a < 2; ++a)
-                    if (!((a && I == nyc) || (b && J == nxc) || (c && K == nzc)))
-                        any |= (cflag[(I + a) + NYc * ((J + b) + NXc * (K + c))] & NF_ACTIVE) != 0;
-        live = any;
-    }
-    if (live) {
-        const int I = pl % NYc, J = pl / NYc;
-        const int ly = I < nyc ? S : 1, lx = J < nxc ? S : 1, lz = K < nzc ? S : 1;
-        T cv[2][2][2][3];   // [c (z)][b (x)][a (y)][component]
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int b = 0; b < 2; ++b)
-#pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    const bool in = !((a && I == nyc) || (b && J == nxc) || (c && K == nzc));
-                    const int m = 3 * ((I + a) + NYc * ((J + b) + NXc * (K + c)));
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) cv[c][b][a][q] = in ? xc[m + q] : T(0);
+                for (int q = 0; q < 3; ++q) {
+                    if (!have) c0[k][q] = xc[3 * (co[k] + cpl * K) + q];
+                    c1[k][q] = xc[3 * (co[k] + cpl * K + up) + q];
                 }
-        const T inv = T(1) / T(S);
+            const int f00 = 2 * I + NYf * 2 * J + fpl * 2 * K;
 #pragma unroll
-        for (int rz = 0; rz < S; ++rz) {
-            if (rz >= lz) break;
-            const T wz1 = T(rz) * inv, wz0 = T(S - rz) * inv;
-            T qz[2][2][3];
+            for (int z0 = 0; z0 < 2; z0 += BZ) {
+                T r[BZ][2][2][3], dg[BZ][2][2][3];
+                uint8_t fl[BZ][2][2];
 #pragma unroll
-            for (int b = 0; b < 2; ++b)
+                for (int z = 0; z < BZ; ++z)
 #pragma unroll
-                for (int a = 0; a < 2; ++a)
+                    for (int x = 0; x < 2; ++x)
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) qz[b][a][q] = wz0 * cv[0][b][a][q] + wz1 * cv[1][b][a][q];
+                        for (int y = 0; y < 2; ++y) {
+                            const int f = f00 + (y && ly ? 1 : 0) + (x && lx ? NYf : 0) + (z0 + z && lz ? fpl : 0);
+                            fl[z][x][y] = nflag[f];
 #pragma unroll
-            for (int rx = 0; rx < S; ++rx) {
-                if (rx >= lx) break;
-                const T wx1 = T(rx) * inv, wx0 = T(S - rx) * inv;
-                T qx[2][3];
+                            for (int q = 0; q < 3; ++q) {
+                                r[z][x][y][q] = rf[3 * f + q];
+                                dg[z][x][y][q] = D[3 * f + q];
+                            }
+                        }
 #pragma unroll
-                for (int a = 0; a < 2; ++a)
+                for (int z = 0; z < BZ; ++z) {
+                    const int rz = z0 + z;
+                    if (rz && !lz) break;
+                    T qz[4][3];
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) qx[a][q] = wx0 * qz[0][a][q] + wx1 * qz[1][a][q];
-                const int rowbase = NYf * ((S * J + rx) + NXf * (S * K + rz)) + S * I;
+                    for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int ry = 0; ry < S; ++ry) {
-                    if (ry >= ly) break;
-                    const T wy1 = T(ry) * inv, wy0 = T(S - ry) * inv;
-                    const int f = rowbase + ry;
-                    const uint8_t fl = nflag[f];
-                    const bool act = (fl & NF_ACTIVE) != 0;
-                    // r and D are loaded whatever the flag says, so that these loads do not
-                    // wait for the flag load (one round trip per fine node, not two); what
-                    // an inactive node holds is discarded by the selects below
-                    T r[3], dg[3], o[3];
+                        for (int q = 0; q < 3; ++q) qz[k][q] = rz ? c0[k][q] + c1[k][q] : c0[k][q];
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) {
-                        r[q] = rf[3 * f + q];
-                        dg[q] = D[3 * f + q];
-                    }
+                    for (int x = 0; x < 2; ++x) {
+                        if (x && !lx) break;
+                        T qx[2][3];
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) {
-                        const T t = (omega * r[q]) * dg[q];
-                        o[q] = act ? (t + (wy0 * qx[0][q] + wy1 * qx[1][q])) + t : T(0);
-                    }
-                    if (FINAL) {
+                        for (int a = 0; a < 2; ++a)
 #pragma unroll
-                        for (int q = 0; q < 3; ++q)
-                            if (fl & (NF_FIXX << q)) o[q] = T(0);
-                        if (act) dot += o[0] * r[0] + o[1] * r[1] + o[2] * r[2];
-                    }
-                    // inactive nodes of an output that keeps zeros there (cflag set) are not rewritten
-                    if (act || !cflag) {
+                            for (int q = 0; q < 3; ++q) qx[a][q] = x ? qz[a][q] + qz[2 + a][q] : qz[a][q];
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) xf[3 * f + q] = o[q];
+                        for (int y = 0; y < 2; ++y) {
+                            if (y && !ly) break;
+                            const int f = f00 + y + NYf * x + fpl * rz;
+                            const T scale = T(1) / T((1 + rz) * (1 + x) * (1 + y));
+                            const bool act = (fl[z][x][y] & NF_ACTIVE) != 0;
+                            T o[3];
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) {
+                                const T p = y ? qx[0][q] + qx[1][q] : qx[0][q];
+                                o[q] = act ? r[z][x][y][q] * dg[z][x][y][q] + scale * p : T(0);
+                                if (FINAL && (fl[z][x][y] & (NF_FIXX << q))) o[q] = T(0);
+                            }
+                            if (FINAL && act)
+                                dot += o[0] * r[z][x][y][0] + o[1] * r[z][x][y][1] + o[2] * r[z][x][y][2];
+                            // inactive nodes of an output that keeps zeros there (cflag set) are not rewritten
+                            if (act || !cflag) {
+#pragma unroll
+                                for (int q = 0; q < 3; ++q) xf[3 * f + q] = o[q];
+                            }
+                        }
                     }
                 }
             }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) c0[k][q] = c1[k][q];
+            have = true;
         }
-    }
     }
     if (FINAL && partial) {
         __shared__ double red[4];
@@ -378,7 +464,7 @@ __global__ void __launch_bounds__(128) k_prolong_cells(const T *__restrict__ xc,
 template <typename T, bool FINAL>
 __global__ void __launch_bounds__(128) k_prolong_rows4(const T *__restrict__ xc, const T *__restrict__ rf,
                                                        const T *__restrict__ D, const uint8_t *__restrict__ nflag,
-                                                       T omega, T *__restrict__ xf, int nyc, int nxc, int nzc,
+                                                       T *__restrict__ xf, int nyc, int nxc, int nzc,
                                                        int keep_zeros, double *__restrict__ partial) {
     constexpr int S = 4;
     const int NYc = nyc + 1, NXc = nxc + 1, NYf = S * nyc + 1, NXf = S * nxc + 1;
@@ -427,8 +513,7 @@ __global__ void __launch_bounds__(128) k_prolong_rows4(const T *__restrict__ xc,
             T o[3];
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-                const T t = (omega * r[k][q]) * dg[k][q];
-                o[q] = act ? (t + (T(S - k) / T(S) * qa[0][q] + T(k) / T(S) * qa[1][q])) + t : T(0);
+                o[q] = act ? r[k][q] * dg[k][q] + (T(S - k) / T(S) * qa[0][q] + T(k) / T(S) * qa[1][q]) : T(0);
                 if (FINAL && (fl[k] & (NF_FIXX << q))) o[q] = T(0);
             }
             if (FINAL && act) dot += o[0] * r[k][0] + o[1] * r[k][1] + o[2] * r[k][2];
@@ -446,7 +531,7 @@ __global__ void __launch_bounds__(128) k_prolong_rows4(const T *__restrict__ xc,
 }
 
 template <typename T>
-void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, const T *rf, const T *diag, T omega,
+void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, const T *rf, const T *diag,
                            T *xf, bool final_level, double *partial_dot, int *nblocks_out, cudaStream_t st) {
     const bool small = 3 * (int64_t)fine.nnode < (int64_t)INT32_MAX;
     // empty cells are skipped in FP32 only: the FP32 V-cycle's outputs (d_z32 and the
@@ -457,10 +542,10 @@ void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, 
         if (nblocks_out) *nblocks_out = (int)(g.x * g.y);
         ++g_launches;
         if (final_level)
-            k_prolong_rows4<T, true><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, omega, xf, coarse.ny, coarse.nx,
+            k_prolong_rows4<T, true><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, xf, coarse.ny, coarse.nx,
                                                         coarse.nz, skip_inactive, partial_dot);
         else
-            k_prolong_rows4<T, false><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, omega, xf, coarse.ny, coarse.nx,
+            k_prolong_rows4<T, false><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, xf, coarse.ny, coarse.nx,
                                                          coarse.nz, skip_inactive, nullptr);
         return;
     }
@@ -474,10 +559,10 @@ void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, 
         ++g_launches;
         const uint8_t *cflag = skip_inactive ? coarse.nflag : nullptr;
         if (final_level)
-            k_prolong_cells<T, 2, true><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, cflag, omega, xf, coarse.ny,
+            k_prolong_cells<T, true><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, cflag, xf, coarse.ny,
                                                            coarse.nx, coarse.nz, zp, partial_dot);
         else
-            k_prolong_cells<T, 2, false><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, cflag, omega, xf, coarse.ny,
+            k_prolong_cells<T, false><<<g, 128, 0, st>>>(xc, rf, diag, fine.nflag, cflag, xf, coarse.ny,
                                                             coarse.nx, coarse.nz, zp, nullptr);
         return;
     }
@@ -485,16 +570,16 @@ void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, 
     if (nblocks_out) *nblocks_out = (int)(nb.x * nb.y);
     ++g_launches;
     if (final_level)
-        k_prolong_smooth<T, true><<<nb, 256, 0, st>>>(xc, rf, diag, fine.nflag, omega, xf, coarse.ny, coarse.nx,
+        k_prolong_smooth<T, true><<<nb, 256, 0, st>>>(xc, rf, diag, fine.nflag, xf, coarse.ny, coarse.nx,
                                                       coarse.nz, coarse.span, partial_dot);
     else
-        k_prolong_smooth<T, false><<<nb, 256, 0, st>>>(xc, rf, diag, fine.nflag, omega, xf, coarse.ny, coarse.nx,
+        k_prolong_smooth<T, false><<<nb, 256, 0, st>>>(xc, rf, diag, fine.nflag, xf, coarse.ny, coarse.nx,
                                                        coarse.nz, coarse.span, nullptr);
 }
 template void launch_prolong_smooth<double>(const Level &, const Level &, const double *, const double *,
-                                            const double *, double, double *, bool, double *, int *, cudaStream_t);
+                                            const double *, double *, bool, double *, int *, cudaStream_t);
 template void launch_prolong_smooth<float>(const Level &, const Level &, const float *, const float *, const float *,
-                                           float, float *, bool, double *, int *, cudaStream_t);
+                                           float *, bool, double *, int *, cudaStream_t);
 
 // ---- Jacobi diagonals (src/Solving_AssembleFEAstencil.m:82-121) -------------
 // reference corner order j = 1..8 as offsets (dy, dx, dz)
@@ -565,17 +650,18 @@ void launch_diag_from_Ks(const Level &l, double *diag, cudaStream_t s) {
 }
 
 __global__ void k_inverse_diag(const double *__restrict__ D, const uint8_t *__restrict__ nflag, int64_t nn,
-                               double *__restrict__ iD, float *__restrict__ iD32) {
+                               double omega2, double *__restrict__ iD, float *__restrict__ iD32) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= 3 * nn) return;
-    const double v = (nflag[i / 3] & NF_ACTIVE) ? 1.0 / D[i] : 0.0;
+    const double v = (nflag[i / 3] & NF_ACTIVE) ? omega2 / D[i] : 0.0;
     iD[i] = v;
     iD32[i] = (float)v;
 }
 
-void launch_inverse_diag(const Level &l, cudaStream_t s) {
+void launch_inverse_diag(const Level &l, double omega, cudaStream_t s) {
     ++g_launches;
-    k_inverse_diag<<<(unsigned)((3 * l.nnode + 255) / 256), 256, 0, s>>>(l.diag, l.nflag, l.nnode, l.idiag, l.idiag32);
+    k_inverse_diag<<<(unsigned)((3 * l.nnode + 255) / 256), 256, 0, s>>>(l.diag, l.nflag, l.nnode, 2.0 * omega, l.idiag,
+                                                                      l.idiag32);
 }
 
 // ---- compact <-> full conversions -------------------------------------------

@@ -345,7 +345,7 @@ int vcycle_dev(sgld_ctx *ctx, const double *r, double *z, double *partial, int *
     for (int l = L - 2; l >= 0; --l) {
         const double *rl = (l == 0) ? r : c.lv[l].r;
         double *xl = (l == 0) ? z : c.lv[l].x;
-        launch_prolong_smooth<double>(c.lv[l], c.lv[l + 1], c.lv[l + 1].x, rl, c.lv[l].idiag, c.omega, xl, l == 0,
+        launch_prolong_smooth<double>(c.lv[l], c.lv[l + 1], c.lv[l + 1].x, rl, c.lv[l].idiag, xl, l == 0,
                                       l == 0 ? partial : nullptr, l == 0 ? nb : nullptr, c.stream);
     }
     CKL();
@@ -366,7 +366,7 @@ int vcycle_dev32(sgld_ctx *ctx, const float *r, float *z, double *partial, int *
     for (int l = L - 2; l >= 0; --l) {
         const float *rl = (l == 0) ? r : c.lv[l].r32;
         float *xl = (l == 0) ? z : c.lv[l].x32;
-        launch_prolong_smooth<float>(c.lv[l], c.lv[l + 1], c.lv[l + 1].x32, rl, c.lv[l].idiag32, (float)c.omega, xl,
+        launch_prolong_smooth<float>(c.lv[l], c.lv[l + 1], c.lv[l + 1].x32, rl, c.lv[l].idiag32, xl,
                                      l == 0, l == 0 ? partial : nullptr, l == 0 ? nb : nullptr, st);
     }
     return SGLD_OK;
@@ -1297,7 +1297,7 @@ int sgld_assemble(sgld_ctx *ctx) {
     if (info != 0)
         return fail(ctx, SGLD_ERR_NUMERIC,
                     "coarsest-level matrix is not positive definite (pivot " + std::to_string(info) + ")");
-    for (int l = 0; l < L - 1; ++l) launch_inverse_diag(c.lv[l], c.stream);
+    for (int l = 0; l < L - 1; ++l) launch_inverse_diag(c.lv[l], c.omega, c.stream);
     launch_cast_f32(c.E, c.d_E32, c.lv[0].nel, c.stream);
     CKL();
     CK(cudaStreamSynchronize(c.stream));
@@ -1449,7 +1449,7 @@ int sgld_interpolate(sgld_ctx *ctx, int ii, const double *xc, double *xf) {
     CK(cudaMemsetAsync(rzero, 0, sizeof(double) * 3 * f.nnode, c.stream));
     std::vector<double> one(3 * f.nnode, 1.0);
     CK(cudaMemcpy(ones, one.data(), sizeof(double) * one.size(), cudaMemcpyHostToDevice));
-    launch_prolong_smooth<double>(f, c.lv[l], c.lv[l].x, rzero, ones, 0.0, out, false, nullptr, nullptr, c.stream);
+    launch_prolong_smooth<double>(f, c.lv[l], c.lv[l].x, rzero, ones, out, false, nullptr, nullptr, c.stream);
     CKL();
     return level_vec_to_host(ctx, l - 1, out, xf);
 }

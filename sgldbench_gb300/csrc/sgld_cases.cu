@@ -223,7 +223,7 @@ int net_correction(sgld_cases *cs, sgld_cases_stats *st) {
     CCK(cudaMemsetAsync(c.d_tmp, 0, sizeof(double) * nv, s));
     for (int i = cs->level - 1; i >= 0; --i) {
         double *out = (i == 0) ? c.d_p : c.lv[i].x;
-        launch_prolong_smooth<double>(c.lv[i], c.lv[i + 1], c.lv[i + 1].x, c.d_tmp, c.lv[i].idiag, 0.0, out, false,
+        launch_prolong_smooth<double>(c.lv[i], c.lv[i + 1], c.lv[i + 1].x, c.d_tmp, c.lv[i].idiag, out, false,
                                       nullptr, nullptr, s);
     }
     launch_mask_fixed(l0, c.d_p, s);

@@ -69,7 +69,7 @@ struct Level {
     int64_t tiles_f32_cap = 0;
     uint8_t *nflag = nullptr;     // [nnode] NF_* bits
     double *diag = nullptr;       // [3*nnode] Jacobi diagonal (levels 1..L-1)
-    double *idiag = nullptr;      // [3*nnode] 1 / diag on active nodes, 0 elsewhere
+    double *idiag = nullptr;      // [3*nnode] 2 omega / diag on active nodes, 0 elsewhere
     float *idiag32 = nullptr;
     double *Ks = nullptr;         // [576*nel] Galerkin element matrices (coarse levels)
     double *r = nullptr, *x = nullptr;      // [3*nnode] V-cycle work (coarse levels)
@@ -324,11 +324,11 @@ template <typename T>
 void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *rc, cudaStream_t s);
 template <typename T>
 void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, const T *rf, const T *diag,
-                           T omega, T *xf, bool final_level, double *partial_dot, int *nblocks_out,
+                           T *xf, bool final_level, double *partial_dot, int *nblocks_out,
                            cudaStream_t s);
 void launch_diag_finest(const Level &l0, const double *E, const double *Ke, double *diag, cudaStream_t s);
 void launch_diag_from_Ks(const Level &l, double *diag, cudaStream_t s);
-void launch_inverse_diag(const Level &l, cudaStream_t s);   // l.idiag, l.idiag32 from l.diag
+void launch_inverse_diag(const Level &l, double omega, cudaStream_t s);   // l.idiag, l.idiag32 from l.diag
 void launch_scatter_nodes(const int64_t *map, int64_t n, const double *compact, double *full, cudaStream_t s);
 void launch_gather_nodes(const int64_t *map, int64_t n, const double *full, double *compact, cudaStream_t s);
 // dst[per * i + c] = src[per * map[i] + c]; per in {1, 3, 6, 12}

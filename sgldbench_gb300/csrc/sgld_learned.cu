@@ -214,7 +214,7 @@ int learned_before_solve(sgld_ctx *ctx, LearnedWS *w, int mode, double E0, int *
         LCK(cudaMemsetAsync(c.d_tmp, 0, sizeof(double) * nv, s));
         for (int i = w->level - 1; i >= 0; --i) {
             double *out = (i == 0) ? c.d_p : c.lv[i].x;
-            launch_prolong_smooth<double>(c.lv[i], c.lv[i + 1], c.lv[i + 1].x, c.d_tmp, c.lv[i].idiag, 0.0, out,
+            launch_prolong_smooth<double>(c.lv[i], c.lv[i + 1], c.lv[i + 1].x, c.d_tmp, c.lv[i].idiag, out,
                                           false, nullptr, nullptr, s);
         }
         launch_mask_fixed(l0, c.d_p, s);
