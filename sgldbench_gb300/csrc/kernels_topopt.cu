@@ -12,6 +12,8 @@
 
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "sgld_internal.cuh"
 
 namespace sgld {
@@ -150,56 +152,98 @@ __device__ __forceinline__ double oc_new(double xe, double qe, double rs, double
     return fmax(0.0, fmax(xe - move, fmin(1.0, fmin(xe + move, qe * rs))));
 }
 
+// The same with the comparisons on the bit patterns: all operands are >= 0 (or NaN, which
+// is above every number in both forms), so the order of the unsigned patterns is the
+// order of the numbers and no FP64 operation is spent on it.
+__device__ __forceinline__ double bits_min(double a, double b) {
+    return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b) ? a : b;
+}
+__device__ __forceinline__ double bits_max(double a, double b) {
+    return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;   // negative numbers lose to 0
+}
+__device__ __forceinline__ double oc_new_bits(double xe, double qe, double rs, double move) {
+    return bits_max(0.0, bits_max(xe - move, bits_min(1.0, bits_min(xe + move, qe * rs))));
+}
+
 // element flags of level 1: bit 0 active, bit 1 passive (kept solid by the
 // SIMP loop; TopOpti_GlobalVolumeConstraint.m:162,179)
 constexpr uint8_t EF_PASSIVE = 2;
 
-__global__ void k_oc_step(const double *__restrict__ x, const double *__restrict__ q, const double *__restrict__ dv,
-                          const uint8_t *__restrict__ eact, int64_t n, double move, const double *__restrict__ st,
-                          double *__restrict__ part) {
-    if (st[OC_DONE] != 0.0) return;
-    const double lmid = 0.5 * (st[OC_HI] + st[OC_LO]);
-    const double rs = 1.0 / sqrt(lmid);
-    double s = 0.0;
-    for (int64_t e = blockIdx.x * (int64_t)TB + threadIdx.x; e < n; e += (int64_t)gridDim.x * TB) {
-        if (!eact[e]) continue;
-        const double xn = (eact[e] & EF_PASSIVE) ? 1.0 : oc_new(x[e], q[e], rs, move);
-        s += dv[e] * (xn - x[e]);
-    }
-    s = tblock_sum(s);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-__device__ double tsum_partials(const double *__restrict__ part, int nb) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += TB) s += part[i];
-    return tblock_sum(s);
-}
-
-// op 0: init (g = sum_v / n - V, lo = 0, hi = 1e9); op 1: bisection update (:88-89)
-__global__ void k_oc_scalar(int op, double *__restrict__ st, const double *__restrict__ part, int nb, double nact,
-                            double volfrac) {
-    const double s = tsum_partials(part, nb);
+// g = sum_v / n - V (:83), the bisection's bounds
+__global__ void k_oc_init(double *__restrict__ st, const double *__restrict__ sum_v, double nact, double volfrac) {
     if (threadIdx.x != 0) return;
-    if (op == 0) {
-        st[OC_G] = s / nact - volfrac;
-        st[OC_LO] = 0.0;
-        st[OC_HI] = 1e9;
-        st[OC_DONE] = 0.0;
-        st[OC_STEPS] = 0.0;
-        st[OC_MID] = 0.5e9;
-        return;
+    st[OC_G] = sum_v[0] / nact - volfrac;
+    st[OC_LO] = 0.0;
+    st[OC_HI] = 1e9;
+    st[OC_DONE] = 0.0;
+    st[OC_STEPS] = 0.0;
+    st[OC_MID] = 0.5e9;
+}
+
+// The bisection on the volume multiplier (:85-90), all of its steps (about 50) in one
+// cooperative launch: per step every CTA sums dv (xnew - x) over its elements, the
+// grid meets, and every CTA adds the partials and takes the step for itself.
+// As a launch per step every thread formed 1 / sqrt(lmid) (40 FP64 operations
+// for 13 per element) and a second launch added the partials: 1.33 ms on 96 x 48 x
+// 48, now 0.45.  Bound by the FP64 pipe and a step's serial part (the sums, 1 /
+// sqrt(lmid), the meeting).
+// part0, part1: gridDim.x partials each, used in turn.
+__global__ void __launch_bounds__(TB) k_oc_bisect(const double *__restrict__ x, const double *__restrict__ q,
+                                                  const double *__restrict__ dv, const uint8_t *__restrict__ eact,
+                                                  int64_t n, double move, double *st, double *part0, double *part1,
+                                                  int max_steps) {
+    auto grid = cooperative_groups::this_grid();
+    __shared__ double lo, hi, mid, next, rs, steps;
+    __shared__ bool done;
+    const int tid = threadIdx.x;
+    const double g = st[OC_G];
+    if (tid == 0) {
+        lo = st[OC_LO];
+        hi = st[OC_HI];
+        mid = st[OC_MID];
+        steps = 0.0;
+        done = false;
     }
-    if (st[OC_DONE] != 0.0) return;
-    const double lmid = 0.5 * (st[OC_HI] + st[OC_LO]);
-    st[OC_MID] = lmid;
-    const double gt = st[OC_G] + s;
-    if (gt > 0.0)
-        st[OC_LO] = lmid;
-    else
-        st[OC_HI] = lmid;
-    st[OC_STEPS] += 1.0;
-    if (!((st[OC_HI] - st[OC_LO]) / (st[OC_LO] + st[OC_HI]) > 1e-6)) st[OC_DONE] = 1.0;
+    for (int k = 0; k < max_steps; ++k) {
+        // the next multiplier and the stopping test, by two threads side by side
+        if (tid == 0) {
+            next = 0.5 * (hi + lo);
+            rs = 1.0 / sqrt(next);
+        } else if (tid == 32) {
+            done = k > 0 && !((hi - lo) / (lo + hi) > 1e-6);
+        }
+        __syncthreads();
+        if (done) break;
+        double *part = k & 1 ? part1 : part0;
+        double s = 0.0;
+        for (int64_t e = blockIdx.x * (int64_t)TB + tid; e < n; e += (int64_t)gridDim.x * TB) {
+            const uint8_t f = eact[e];   // all four loads go out together
+            const double xe = x[e], qe = q[e], de = dv[e];
+            if (f) s += de * (((f & EF_PASSIVE) ? 1.0 : oc_new_bits(xe, qe, rs, move)) - xe);
+        }
+        s = tblock_sum(s);
+        if (tid == 0) part[blockIdx.x] = s;
+        grid.sync();
+        s = 0.0;   // read past L1: the buffer held another step's partials before
+        for (int i = tid; i < (int)gridDim.x; i += TB) s += __ldcg(part + i);
+        s = tblock_sum(s);
+        if (tid == 0) {
+            mid = next;
+            if (g + s > 0.0)
+                lo = mid;
+            else
+                hi = mid;
+            steps += 1.0;
+        }
+        __syncthreads();
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        st[OC_LO] = lo;
+        st[OC_HI] = hi;
+        st[OC_MID] = mid;
+        st[OC_STEPS] = steps;
+        st[OC_DONE] = done ? 1.0 : 0.0;
+    }
 }
 
 // x <- xnew(lmid of the last bisection step); partial max |xnew - x| (:91-92)
@@ -298,14 +342,26 @@ void launch_topo_q(const Level &l0, const double *x, const double *dc, const dou
     ++g_launches;
     k_topo_q<<<nb, TB, 0, s>>>(x, dc, dv, l0.eact, l0.nel, q);
 }
-void launch_oc_step(const Level &l0, const double *x, const double *q, const double *dv, double move,
-                    const double *st, double *part, int nb, cudaStream_t s) {
+void launch_oc_init(double *st, const double *sum_v, double nact, double volfrac, cudaStream_t s) {
     ++g_launches;
-    k_oc_step<<<nb, TB, 0, s>>>(x, q, dv, l0.eact, l0.nel, move, st, part);
+    k_oc_init<<<1, 32, 0, s>>>(st, sum_v, nact, volfrac);
 }
-void launch_oc_scalar(int op, double *st, const double *part, int nb, double nact, double volfrac, cudaStream_t s) {
+// 0 or a CUDA error
+int launch_oc_bisect(const Level &l0, const double *x, const double *q, const double *dv, double move, double *st,
+                     double *part0, double *part1, int nb, int max_steps, cudaStream_t s) {
+    // two CTAs per SM: a step takes as long with one, and with more of them the grid's meeting
+    // and the partials cost more than the elements save (96 x 48 x 48: 443, 445, 516, 607 us
+    // with 1 to 4)
+    int dev = 0, sms = 0, fit = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_oc_bisect, TB, 0);
+    const int grid = std::min(nb, std::max(1, sms * std::min(fit, 2)));
+    const uint8_t *eact = l0.eact;
+    int64_t n = l0.nel;
+    void *args[] = {&x, &q, &dv, &eact, &n, &move, &st, &part0, &part1, &max_steps};
     ++g_launches;
-    k_oc_scalar<<<1, TB, 0, s>>>(op, st, part, nb, nact, volfrac);
+    return (int)cudaLaunchCooperativeKernel((const void *)k_oc_bisect, dim3(grid), dim3(TB), args, 0, s);
 }
 void launch_oc_apply(const Level &l0, double *x, const double *q, double move, const double *st, double *part,
                      int nb, cudaStream_t s) {

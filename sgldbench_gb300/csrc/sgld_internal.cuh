@@ -274,9 +274,9 @@ void launch_topo_sens(const Level &l0, const double *xp, const double *ce, const
                       double Emin, double *dcs, double *dvs, int nb, cudaStream_t s);
 void launch_topo_q(const Level &l0, const double *x, const double *dc, const double *dv, double *q, int nb,
                    cudaStream_t s);
-void launch_oc_step(const Level &l0, const double *x, const double *q, const double *dv, double move,
-                    const double *st, double *part, int nb, cudaStream_t s);
-void launch_oc_scalar(int op, double *st, const double *part, int nb, double nact, double volfrac, cudaStream_t s);
+void launch_oc_init(double *st, const double *sum_v, double nact, double volfrac, cudaStream_t s);
+int launch_oc_bisect(const Level &l0, const double *x, const double *q, const double *dv, double move, double *st,
+                     double *part0, double *part1, int nb, int max_steps, cudaStream_t s);
 void launch_oc_apply(const Level &l0, double *x, const double *q, double move, const double *st, double *part,
                      int nb, cudaStream_t s);
 void launch_max_partials(const double *part, int nb, double *out, cudaStream_t s);

@@ -432,7 +432,7 @@ extern "C" int sgld_topopt(sgld_ctx *ctx, const sgld_topopt_opts *opts, const do
         NvtxRange iter_range("SIMP iteration");
         double vol = 0.0;
         TCK(cudaMemcpyAsync(&vol, c.t_st + T_VOL, sizeof(double), cudaMemcpyDeviceToHost, s));
-        launch_oc_scalar(0, c.t_st, c.t_st + T_VOL, 1, nact, o.volfrac, s);        // g (:83), bisection bounds
+        launch_oc_init(c.t_st, c.t_st + T_VOL, nact, o.volfrac, s);        // g (:83), bisection bounds
         TCK(cudaEventRecord(ev[0], s));
         if ((rc = sgld_assemble(ctx))) return rc;                                  // :54
         int net_used = 0, net_acc = 0;
@@ -472,15 +472,8 @@ extern "C" int sgld_topopt(sgld_ctx *ctx, const sgld_topopt_opts *opts, const do
             launch_max_partials(c.d_part, nbm, c.t_st + T_CHANGE, s);
         } else {
             launch_topo_q(l0, c.t_x, c.t_dc, c.t_dv, c.t_q, nb, s);
-            double done = 0.0;
-            for (int round = 0; round < 8 && done == 0.0; ++round) {               // :85-90
-                for (int k = 0; k < 32; ++k) {
-                    launch_oc_step(l0, c.t_x, c.t_q, c.t_dv, o.move, c.t_st, c.d_part, nb, s);
-                    launch_oc_scalar(1, c.t_st, c.d_part, nb, nact, o.volfrac, s);
-                }
-                TCK(cudaMemcpyAsync(&done, c.t_st + OC_DONE, sizeof(double), cudaMemcpyDeviceToHost, s));
-                TCK(cudaStreamSynchronize(s));
-            }
+            // :85-90
+            TCK((cudaError_t)launch_oc_bisect(l0, c.t_x, c.t_q, c.t_dv, o.move, c.t_st, c.d_part, c.d_part2, nb, 256, s));
             launch_oc_apply(l0, c.t_x, c.t_q, o.move, c.t_st, c.d_part, nb, s);   // :91-92
             launch_max_partials(c.d_part, nb, c.t_st + T_CHANGE, s);
         }
