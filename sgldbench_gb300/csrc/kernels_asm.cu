@@ -313,13 +313,27 @@ __device__ __forceinline__ df df_rsqrt(df d) {
     return y;
 }
 
+// 1/d in double-float: FP32 reciprocal y and its Newton correction y (1 - d y), whose
+// factor 1 - d y (about 2^-24) is needed to FP32 accuracy only
+__device__ __forceinline__ df df_rcp(df d) {
+    const float y = __frcp_rn(d.hi);
+    return quick_two_sum(y, __fmul_rn(y, __fmaf_rn(-d.lo, y, __fmaf_rn(-d.hi, y, 1.f))));
+}
+
 // One block column of the band Cholesky (4 warps per CTA), in double-float
 // arithmetic: GB300's FP64 pipe would serialise the pivot chain (a warp-wide
 // FP64 instruction occupies its sub-partition for many cycles).  The matrix
 // stays FP64 in memory; tiles are split into (hi, lo) on load.
-//   * every CTA factors the 32 x 32 diagonal tile in shared memory (row = lane,
-//     the rank-1 update of step j split over the 4 warps by column mod 4; the
-//     pivot 1/sqrt(d) is formed by every thread, so it needs no broadcast);
+//   * every CTA factors the 32 x 32 diagonal tile as L D L': row = lane, column
+//     4 k + w in register k of warp w.  A step's only exchange is the pivot column,
+//     through shared memory: its owner updates the next pivot column first and
+//     publishes it, then one barrier.  The registers move down by one every four
+//     steps, so the loop stays rolled (unrolled, its code is read once and from
+//     far away: 51 us a launch).  A step's serial chain is a reciprocal and two
+//     products; the square roots that turn L D L' into the Cholesky factor are
+//     taken for all columns at once afterwards.  (With the tile in shared memory, a
+//     square root in the chain, branches around the updates and two barriers a step
+//     the launch took 30 us; now 15);
 //   * CTA 0 writes the factored tile back;
 //   * CTA b > 0 solves CP_RS rows of the band below against it (X = A L^-T):
 //     16 lanes per row, two columns per lane in registers, x_q broadcast by a
@@ -328,42 +342,70 @@ constexpr int CP_THREADS = 128;
 constexpr int CP_RS = 8;
 
 __global__ void __launch_bounds__(CP_THREADS) k_chol_panel(double *A, int n, int k0, int rend, int *info) {
-    __shared__ df T[NB][NB + 1];
-    __shared__ df rd[NB], ld[NB];
+    __shared__ float2 T[NB][NB + 1];     // the factor
+    __shared__ float2 rd[NB], ld[NB];    // 1 / L[j][j], L[j][j]
     const int t = threadIdx.x, r = t & 31, w = t >> 5;
     const int m = min(NB, n - k0);
-    for (int idx = t; idx < NB * NB; idx += CP_THREADS) {
-        const int rr = idx & 31, cc = idx >> 5;
-        T[rr][cc] = (rr < m && cc < m && cc <= rr) ? df_from(A[(int64_t)(k0 + rr) + (int64_t)n * (k0 + cc)])
-                                                   : df{rr == cc ? 1.f : 0.f, 0.f};
+    auto get = [](float2 v) -> df { return {v.x, v.y}; };
+    df a[NB / 4];
+#pragma unroll
+    for (int k = 0; k < NB / 4; ++k) {
+        const int c = 4 * k + w;
+        a[k] = (r < m && c < m && c <= r) ? df_from(A[(int64_t)(k0 + r) + (int64_t)n * (k0 + c)])
+                                          : df{r == c ? 1.f : 0.f, 0.f};
+    }
+    if (w == 0) T[r][0] = make_float2(a[0].hi, a[0].lo);
+    __syncthreads();
+#pragma unroll 1
+    for (int j0 = 0; j0 < NB; j0 += 4) {
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+            const int j = j0 + jj;
+            df d = get(T[j][j]);
+            const bool bad = !(d.hi > 0.f);
+            if (bad) d = {1.f, 0.f};
+            if (bad && t == 0 && blockIdx.x == 0 && info) atomicExch(info, k0 + j + 1);
+            // row r's multiplier; its column q loses f * (column j's row q)
+            const df f = df_mul(get(T[r][j]), df_rcp(d));
+            // no condition on q: columns that are done and rows above the diagonal take values
+            // that nothing reads, and the eight updates run side by side
+            auto update = [&](int k) {
+                a[k] = df_sub(a[k], df_mul(f, get(T[min(j0 + 4 * k + w, NB - 1)][j])));
+            };
+            const int kn = jj < 3 ? 0 : 1;   // the next pivot column's register, in warp (jj + 1) & 3
+            update(kn);
+            if (w == ((jj + 1) & 3) && j + 1 < NB) T[r][j + 1] = make_float2(a[kn].hi, a[kn].lo);
+#pragma unroll
+            for (int k = 0; k < NB / 4; ++k)
+                if (k != kn) update(k);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int k = 0; k + 1 < NB / 4; ++k) a[k] = a[k + 1];
+    }
+    // L = (L D) D^-1/2, columns over the warps
+    df y = {0.f, 0.f}, d = get(T[r][r]);
+    if (!(d.hi > 0.f)) d = {1.f, 0.f};
+    y = df_rsqrt(d);
+    if (w == 0) {
+        const df l = df_mul(d, y);
+        rd[r] = make_float2(y.hi, y.lo);
+        ld[r] = make_float2(l.hi, l.lo);
     }
     __syncthreads();
-    for (int j = 0; j < NB; ++j) {
-        // T[j][j] is read here and never written in the loop (the factor's
-        // diagonal goes to ld[]), so no thread can overwrite it early
-        df d = T[j][j];
-        const bool bad = !(d.hi > 0.f);
-        if (bad) d = {1.f, 0.f};
-        const df y = df_rsqrt(d);
-        if (w == 0 && r > j) T[r][j] = df_mul(T[r][j], y);
-        if (t == 0) {
-            rd[j] = y;
-            ld[j] = df_mul(d, y);
-            if (bad && blockIdx.x == 0 && info) atomicExch(info, k0 + j + 1);
-        }
-        __syncthreads();
-        if (r > j) {
-            const df lrj = T[r][j];
-            for (int q = j + 1 + ((w - j - 1) & 3); q <= r; q += 4) T[r][q] = df_sub(T[r][q], df_mul(lrj, T[q][j]));
-        }
-        __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NB / 4; ++k) {
+        const int c = 4 * k + w;
+        const df x = df_mul(get(T[r][c]), get(rd[c]));
+        T[r][c] = make_float2(x.hi, x.lo);
     }
+    __syncthreads();
     if (blockIdx.x == 0) {
         for (int idx = t; idx < NB * NB; idx += CP_THREADS) {
             const int rr = idx & 31, cc = idx >> 5;
             if (rr < m && cc < m)
                 A[(int64_t)(k0 + rr) + (int64_t)n * (k0 + cc)] =
-                    rr > cc ? df_to(T[rr][cc]) : (rr == cc ? df_to(ld[rr]) : 0.0);
+                    rr > cc ? df_to(get(T[rr][cc])) : (rr == cc ? df_to(get(ld[rr])) : 0.0);
         }
         return;
     }
@@ -377,15 +419,11 @@ __global__ void __launch_bounds__(CP_THREADS) k_chol_panel(double *A, int n, int
     }
 #pragma unroll 4
     for (int q = 0; q < NB; ++q) {
-        const df xq = df_shfl(df_mul(q < 16 ? a0 : a1, rd[q]), q & 15, 16);
-        if (g == (q & 15)) {
-            if (q < 16)
-                a0 = xq;
-            else
-                a1 = xq;
-        }
-        if (g > q) a0 = df_sub(a0, df_mul(xq, T[g][q]));
-        if (g + 16 > q) a1 = df_sub(a1, df_mul(xq, T[g + 16][q]));
+        const df xq = df_shfl(df_mul(q < 16 ? a0 : a1, get(rd[q])), q & 15, 16);
+        // selects, so that no branch stands in the chain
+        const df b0 = df_sub(a0, df_mul(xq, get(T[g][q]))), b1 = df_sub(a1, df_mul(xq, get(T[g + 16][q])));
+        a0 = g > q ? b0 : (g == q ? xq : a0);
+        a1 = g + 16 > q ? b1 : (g + 16 == q ? xq : a1);
     }
     if (live) {
         if (g < m) A[(int64_t)row + (int64_t)n * (k0 + g)] = df_to(a0);
