@@ -5,8 +5,8 @@
 //
 //  * level 2:  Ks_E = sum_q E_q H_q, H_q = P_q' Ke P_q (templates built on the
 //    host, q = child position, s^3 of them);
-//  * level l>2: Ks_E = sum_q P_q' Ks_q P_q with P_q = W_q (x) I3, W_q the 8x8
-//    trilinear weights of the parent's corners at child q's corners;
+//  * level l>2: Ks_E = sum_q P_q' Ks_q P_q, P_q the trilinear interpolation from
+//    the parent's corners to child q's, applied axis by axis;
 //  * coarsest: dense K on the free DOFs (in a bandwidth-reducing order),
 //    blocked band Cholesky K = L L' and the explicit triangular inverse
 //    M = L^-1, captured once into a CUDA graph; each V-cycle applies
@@ -30,8 +30,8 @@ namespace sgld {
 // upper triangle (row <= col) and mirror them.
 __constant__ unsigned char c_pr[300], c_pc[300];
 
-// The tables below are the same for every context; each device gets them once.
-static std::atomic<bool> g_pairs_done[kMaxDevices], g_weights_done[kMaxDevices];
+// The table is the same for every context; each device gets it once.
+static std::atomic<bool> g_pairs_done[kMaxDevices];
 
 static int current_device() {
     int dev = 0;
@@ -39,10 +39,7 @@ static int current_device() {
     return dev;
 }
 
-void forget_asm_tables(int dev) {
-    g_pairs_done[dev] = false;
-    g_weights_done[dev] = false;
-}
+void forget_asm_tables(int dev) { g_pairs_done[dev] = false; }
 
 static void upload_pairs(cudaStream_t s) {
     std::atomic<bool> &done = g_pairs_done[current_device()];
@@ -170,124 +167,124 @@ void launch_diag_templates(const Level &coarse, const double *E, const double *H
 }
 
 // ---- deeper levels: P_q' Ks_q P_q ---------------------------------------------
-// W_q[i][a] = trilinear weight of parent corner a at child q's corner i
-// (span 2, reference corner order, child q = oy + 2 ox + 4 oz).  Only 27 of
-// its 64 entries are nonzero; the kernel walks the nonzeros of each column.
-__constant__ unsigned char c_wn[8][8];      // nonzeros in column a of W_q
-__constant__ unsigned char c_wi[8][8][8];   // their row indices i
-__constant__ double c_ww[8][8][8];          // and weights
-
-__global__ void __launch_bounds__(320) k_asm_coarse(const double *__restrict__ Kf, const uint8_t *__restrict__ eact_f,
+// P_q interpolates trilinearly from the parent's corners to child q's (q = oy + 2 ox
+// + 4 oz), so it is a product of three 1D steps.  Along an axis, child and parent share
+// one corner ("near"); the far corners' values are f_near = a_near, f_far = (a_near +
+// a_far) / 2.  Transposed and doubled, a pair gives (2 f_near + f_far, f_far): one
+// operation per pair and axis, and 2^-6 at the end for both sides.
+// A warp takes a child: lane = row of its symmetric matrix, the three steps along
+// the row in registers, a transpose through shared memory, the three steps along
+// the column; the 8 children add in a fixed order.  Bound by the FP64 pipe: 72
+// operations per lane and child (the walk over W_q's nonzeros by tables in constant
+// memory, read at different places by a warp's lanes, took 1.04 ms for the 8192
+// elements of level 4 of 256 x 128 x 128; now 0.35).
+__global__ void __launch_bounds__(256) k_asm_coarse(const double *__restrict__ Kf, const uint8_t *__restrict__ eact_f,
                                                     const uint8_t *__restrict__ eact_c, int nyc, int nxc, int nzc,
                                                     double *__restrict__ Ks) {
     const int64_t e = blockIdx.x + (int64_t)gridDim.x * blockIdx.y;
     const int64_t nel = (int64_t)nyc * nxc * nzc;
     if (e >= nel || !eact_c[e]) return;
-    __shared__ double sk[576], st[576];
+    __shared__ double st[8][24][25];
+    const int q = threadIdx.x >> 5, r = threadIdx.x & 31;
+    const int o[3] = {(q >> 1) & 1, q & 1, q >> 2};   // the child's half along x, y (rows), z
     const int cy = (int)(e % nyc), cx = (int)((e / nyc) % nxc), cz = (int)(e / ((int64_t)nyc * nxc));
-    const int nyf = 2 * nyc, nxf = 2 * nxc;
-    const int t = threadIdx.x;
-    double acc = 0.0;
-    for (int q = 0; q < 8; ++q) {
-        const int oy = q & 1, ox = (q >> 1) & 1, oz = q >> 2;
-        const int64_t f = (int64_t)(2 * cy + oy) + (int64_t)nyf * ((2 * cx + ox) + (int64_t)nxf * (2 * cz + oz));
-        if (!eact_f[f]) continue;   // uniform per CTA
-        const double *src = Kf + 576 * f;
-        for (int i = t; i < 576; i += blockDim.x) sk[i] = src[i];
-        __syncthreads();
-        // st[r + 24*(3a+d)] = sum_i sk[r + 24*(3i+d)] W[i][a]
-        for (int idx = t; idx < 576; idx += blockDim.x) {
-            const int r = idx % 24, col = idx / 24, a = col / 3, d = col % 3;
-            double v = 0.0;
-            const int nz = c_wn[q][a];
-            for (int k = 0; k < nz; ++k) v += sk[r + 24 * (3 * c_wi[q][a][k] + d)] * c_ww[q][a][k];
-            st[idx] = v;
-        }
-        __syncthreads();
-        // upper triangle of W' st: out[(3b+e), col] = sum_j W[j][b] st[(3j+e) + 24 col]
-        if (t < 300) {
-            const int row = c_pr[t], col = c_pc[t], b = row / 3, ec = row % 3;
-            double v = 0.0;
-            const int nz = c_wn[q][b];
-            for (int k = 0; k < nz; ++k) v += c_ww[q][b][k] * st[(3 * c_wi[q][b][k] + ec) + 24 * col];
-            acc += v;
-        }
-        __syncthreads();
+    const int64_t f = (int64_t)(2 * cy + o[1]) + 2 * (int64_t)nyc * ((2 * cx + o[0]) + 2 * (int64_t)nxc * (2 * cz + o[2]));
+    const bool on = eact_f[f];   // the warp's child
+    // corner near | far: bit 0 = x, 1 = rows, 2 = z (0 = near) -> reference corner j
+    auto corner = [&](int k) {
+        const int x = (k & 1) ^ o[0], y = ((k >> 1) & 1) ^ o[1], z = (k >> 2) ^ o[2];
+        return 4 * z + (y ? x : 3 - x);
+    };
+    int dofs[8];   // first DOF of the 8 corners in that order
+#pragma unroll
+    for (int k = 0; k < 8; ++k) dofs[k] = 3 * corner(k);
+    auto steps = [](double (&v)[24]) {
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (!(k >> ax & 1))
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) v[3 * k + c] = fma(2.0, v[3 * k + c], v[3 * (k | 1 << ax) + c]);
+    };
+    const int mine = r < 24 ? 3 * corner(r / 3) + r % 3 : 0;   // this lane's row, and later column
+    double v[24];
+    if (on && r < 24) {
+        const double *src = Kf + 576 * f + 24 * mine;
+#pragma unroll
+        for (int i = 0; i < 24; ++i) v[i] = src[dofs[i / 3] + i % 3];
+        steps(v);
+#pragma unroll
+        for (int i = 0; i < 24; ++i) st[q][r][i] = v[i];
     }
-    if (t < 300) {
-        double *o = Ks + 576 * e;
-        o[c_pr[t] + 24 * c_pc[t]] = acc;
-        o[c_pc[t] + 24 * c_pr[t]] = acc;
+    __syncwarp();
+    if (r < 24) {
+#pragma unroll
+        for (int i = 0; i < 24; ++i) v[i] = on ? st[q][i][r] : 0.0;
+        if (on) steps(v);
+    }
+    __syncwarp();
+    if (r < 24)
+#pragma unroll
+        for (int i = 0; i < 24; ++i) st[q][dofs[i / 3] + i % 3][mine] = v[i];
+    __syncthreads();
+    for (int t = threadIdx.x; t < 300; t += 256) {
+        const int row = c_pr[t], col = c_pc[t];
+        double sum = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sum += st[k][row][col];
+        sum *= 1.0 / 64.0;
+        double *out = Ks + 576 * e;
+        out[row + 24 * col] = sum;
+        out[col + 24 * row] = sum;
     }
 }
 
 void launch_asm_coarse(const Level &coarse, const Level &fine, double *Ks, cudaStream_t s) {
-    std::atomic<bool> &uploaded = g_weights_done[current_device()];
     upload_pairs(s);
-    if (!uploaded) {
-        const int cdy[8] = {1, 1, 0, 0, 1, 1, 0, 0}, cdx[8] = {0, 1, 1, 0, 0, 1, 1, 0}, cdz[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-        unsigned char wn[8][8] = {}, wi[8][8][8] = {};
-        double ww[8][8][8] = {};
-        for (int q = 0; q < 8; ++q) {
-            const int oy = q & 1, ox = (q >> 1) & 1, oz = q >> 2;
-            for (int i = 0; i < 8; ++i) {
-                // child corner position in parent units: natural coordinates
-                const double sn = -1.0 + (ox + cdx[i]), tn = 1.0 - (oy + cdy[i]), pn = -1.0 + (oz + cdz[i]);
-                const double N[8] = {(1 - sn) * (1 - tn) * (1 - pn), (1 + sn) * (1 - tn) * (1 - pn),
-                                     (1 + sn) * (1 + tn) * (1 - pn), (1 - sn) * (1 + tn) * (1 - pn),
-                                     (1 - sn) * (1 - tn) * (1 + pn), (1 + sn) * (1 - tn) * (1 + pn),
-                                     (1 + sn) * (1 + tn) * (1 + pn), (1 - sn) * (1 + tn) * (1 + pn)};
-                for (int a = 0; a < 8; ++a) {
-                    const double w = 0.125 * N[a];
-                    if (w != 0.0) {
-                        const int k = wn[q][a]++;
-                        wi[q][a][k] = (unsigned char)i;
-                        ww[q][a][k] = w;
-                    }
-                }
-            }
-        }
-        cudaMemcpyToSymbolAsync(c_wn, wn, sizeof wn, 0, cudaMemcpyHostToDevice, s);
-        cudaMemcpyToSymbolAsync(c_wi, wi, sizeof wi, 0, cudaMemcpyHostToDevice, s);
-        cudaMemcpyToSymbolAsync(c_ww, ww, sizeof ww, 0, cudaMemcpyHostToDevice, s);
-        uploaded = true;
-    }
     const int64_t nel = coarse.nel;
     const unsigned gx = (unsigned)(nel < 65535 ? nel : 65535);
     const unsigned gy = (unsigned)((nel + gx - 1) / gx);
     ++g_launches;
-    k_asm_coarse<<<dim3(gx, gy), 320, 0, s>>>(fine.Ks, fine.eact, coarse.eact, coarse.ny, coarse.nx, coarse.nz, Ks);
+    k_asm_coarse<<<dim3(gx, gy), 256, 0, s>>>(fine.Ks, fine.eact, coarse.eact, coarse.ny, coarse.nx, coarse.nz, Ks);
 }
 
 // ---- coarsest level: dense matrix on the free DOFs ---------------------------
-__constant__ int c_ady[8] = {1, 1, 0, 0, 1, 1, 0, 0};
-__constant__ int c_adx[8] = {0, 1, 1, 0, 0, 1, 1, 0};
-__constant__ int c_adz[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-
-// pos[dof] = row of that DOF in the dense matrix or -1; rows[i] = full DOF of row i
+// pos[dof] = row of that DOF in the dense matrix or -1; rows[i] = full DOF of row i.
+// A thread per row and (neighbour node, component): it adds the entries of the up to
+// 8 elements that hold both nodes, so every matrix entry is written once (a thread
+// per row that added its 8 elements' 24 entries one after the other in memory took
+// 100 us, now 8).
 __global__ void k_coarse_dense(const double *__restrict__ Ks, const uint8_t *__restrict__ eact, int ny, int nx, int nz,
                                const int *__restrict__ rows, const int *__restrict__ pos, int ncf, double *__restrict__ A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ncf) return;
-    const int NY = ny + 1, NX = nx + 1;
-    const int dof = rows[i];
-    const int node = dof / 3, c = dof % 3;
+    const int d = blockIdx.y % 3, nb = blockIdx.y / 3;
+    const int ny_ = nb % 3 - 1, nx_ = nb / 3 % 3 - 1, nz_ = nb / 9 - 1;   // offset of the neighbour
+    const int NY = ny + 1, NX = nx + 1, NZ = nz + 1;
+    const int dof = rows[i], node = dof / 3, c = dof % 3;
     const int iy = node % NY, ix = (node / NY) % NX, iz = node / (NY * NX);
+    const int my = iy + ny_, mx = ix + nx_, mz = iz + nz_;
+    if (my < 0 || mx < 0 || mz < 0 || my >= NY || mx >= NX || mz >= NZ) return;
+    const int p = pos[3 * (my + NY * (mx + NX * mz)) + d];
+    if (p < 0) return;
+    // reference corner order j: offsets (dy, dx, dz), and back
+    const int ady[8] = {1, 1, 0, 0, 1, 1, 0, 0}, adx[8] = {0, 1, 1, 0, 0, 1, 1, 0}, adz[8] = {0, 0, 0, 0, 1, 1, 1, 1};
+    double sum = 0.0;
+    bool any = false;
+#pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const int ey = iy - c_ady[j], ex = ix - c_adx[j], ez = iz - c_adz[j];
+        const int ey = iy - ady[j], ex = ix - adx[j], ez = iz - adz[j];
+        const int qy = ady[j] + ny_, qx = adx[j] + nx_, qz = adz[j] + nz_;   // the neighbour's corner
         if (ey < 0 || ex < 0 || ez < 0 || ey >= ny || ex >= nx || ez >= nz) continue;
+        if (qy < 0 || qy > 1 || qx < 0 || qx > 1 || qz < 0 || qz > 1) continue;
         const int64_t e = (int64_t)ey + (int64_t)ny * (ex + (int64_t)nx * ez);
         if (!eact[e]) continue;
-        const double *k = Ks + 576 * e;
-        for (int kk = 0; kk < 8; ++kk) {
-            const int m = (ey + c_ady[kk]) + NY * ((ex + c_adx[kk]) + NX * (ez + c_adz[kk]));
-            for (int d = 0; d < 3; ++d) {
-                const int p = pos[3 * m + d];
-                if (p < 0) continue;
-                A[(int64_t)i + (int64_t)ncf * p] += k[(3 * j + c) + 24 * (3 * kk + d)];
-            }
-        }
+        const int kk = 4 * qz + (qy ? qx : 3 - qx);
+        sum += Ks[576 * e + (3 * j + c) + 24 * (3 * kk + d)];
+        any = true;
     }
+    if (any) A[(int64_t)i + (int64_t)ncf * p] = sum;
 }
 
 void launch_coarse_dense(const Level &lc, int ncf, const int *rows_and_pos, double *A, cudaStream_t s) {
@@ -296,7 +293,7 @@ void launch_coarse_dense(const Level &lc, int ncf, const int *rows_and_pos, doub
     if (ncf == 0) return;   // every coarsest DOF fixed: nothing to factor
     cudaMemsetAsync(A, 0, sizeof(double) * (size_t)ncf * ncf, s);
     ++g_launches;
-    k_coarse_dense<<<(ncf + 127) / 128, 128, 0, s>>>(lc.Ks, lc.eact, lc.ny, lc.nx, lc.nz, rows, pos, ncf, A);
+    k_coarse_dense<<<dim3((ncf + 127) / 128, 81), 128, 0, s>>>(lc.Ks, lc.eact, lc.ny, lc.nx, lc.nz, rows, pos, ncf, A);
 }
 
 // ---- blocked band Cholesky, NB x NB tiles, column-major n x n ------------------
@@ -624,83 +621,118 @@ __global__ void __launch_bounds__(16 * TI_G) k_trinv_tiles(const float2 *__restr
 
 size_t trinv_smem_bytes(int R, int G) { return sizeof(float2) * ((size_t)R * G + 32 * (TI_KC + 1) + 32 * G); }
 
+constexpr int TI_LP = TI_KC + 4, TI_DP = 36;   // padded rows, 16-byte aligned, of the FP32 sweep's tiles
+
 // The same column sweep in FP32 (the hi words of the double-float band and
 // block inverses, FP32 FMA accumulation), writing only the FP32 copy M32 that
 // the FP32 V-cycle of the mixed-precision solves applies.  Its rounding error
 // only perturbs that preconditioner: the coarse apply M32' (M32 r) stays
 // symmetric positive semi-definite for any M32, and the outer solve still
 // converges on the FP64 residual.
+//
+// The sweep is a chain of small steps, so their loads run ahead: while a chunk of the
+// band is multiplied, the next one (of this row block or the first of the next) is on
+// its way in registers, and so is the row block's inverse.  Rows above the group's
+// first column are not read: M is zero there.  (Each chunk loaded when it was
+// needed: 1.37 ms for 3888 rows of half band 287; now 0.83.)
 template <int TI_G>
 __global__ void __launch_bounds__(16 * TI_G) k_trinv_tiles32(const float2 *__restrict__ LB,
                                                              const float2 *__restrict__ D, int n, int b, int R,
                                                              float *__restrict__ M32) {
     constexpr int TI_THREADS = 16 * TI_G;
-    extern __shared__ float tsm32[];
-    float *ring = tsm32;                      // [R][TI_G]
-    float *Lt = ring + (int64_t)R * TI_G;     // [32][TI_KC + 1]
-    float *rhs = Lt + 32 * (TI_KC + 1);       // [32][TI_G]
+    constexpr int NL = 32 * TI_KC / TI_THREADS, ND = 1024 / TI_THREADS;
+    extern __shared__ __align__(16) float tsm32[];
+    float *ring = tsm32;                      // [TI_G][R]: column g's rows, row i in slot i mod R
+    float *Lt = ring + (int64_t)R * TI_G;     // [32][TI_LP]
+    float *Dt = Lt + 32 * TI_LP;              // [32][TI_DP]: (inverse of the diagonal block)[r][q]
+    float *rhs = Dt + 32 * TI_DP;             // [TI_G][TI_DP]
     const int t = threadIdx.x, r = t & 31, gp = (t >> 5) * 2;
-    const int c0 = blockIdx.x * TI_G;
+    const int c0 = blockIdx.x * TI_G, first = c0 & ~31;
     for (int idx = t; idx < R * TI_G; idx += TI_THREADS) ring[idx] = 0.f;
-    __syncthreads();
-    for (int i0 = c0 & ~31; i0 < n; i0 += 32) {
+    // a row block's first band column, rounded down to a group of 4 (the band is zero there)
+    auto kbegin = [&](int i0) { return max(first, (i0 - b) & ~3); };
+    float lreg[NL], dreg[ND];
+    auto fetch_band = [&](int i0, int kc) {   // chunk kc .. of row block i0
+        const int kn = min(TI_KC, i0 - kc);
+#pragma unroll
+        for (int k = 0; k < NL; ++k) {
+            const int idx = t + k * TI_THREADS, rr = idx & 31, kk = idx >> 5, i = i0 + rr, kcol = kc + kk;
+            lreg[k] = (kk < kn && i < n && i - kcol <= b) ? band_at(LB, b, i, kcol).x : 0.f;
+        }
+    };
+    auto fetch_inverse = [&](int i0) {
+#pragma unroll
+        for (int k = 0; k < ND; ++k) dreg[k] = D[(int64_t)(i0 >> 5) * 1024 + t + k * TI_THREADS].x;
+    };
+    auto fma4x = [](const float4 l, const float4 m, float acc) {
+        return fmaf(l.w, m.w, fmaf(l.z, m.z, fmaf(l.y, m.y, fmaf(l.x, m.x, acc))));
+    };
+    auto at4 = [](const float *p) { return *reinterpret_cast<const float4 *>(p); };
+    fetch_inverse(first);
+    for (int i0 = first; i0 < n; i0 += 32) {
         float a0 = 0.f, a1 = 0.f;
-        const int kbeg = max(0, i0 - b);
-        for (int kc = kbeg; kc < i0; kc += TI_KC) {
-            const int kn = min(TI_KC, i0 - kc);
-            for (int idx = t; idx < 32 * TI_KC; idx += TI_THREADS) {
-                const int rr = idx & 31, kk = idx >> 5, i = i0 + rr, k = kc + kk;
-                Lt[rr * (TI_KC + 1) + kk] = (kk < kn && i < n && i - k <= b) ? band_at(LB, b, i, k).x : 0.f;
+        const bool more = i0 + 32 < n;
+        __syncthreads();   // the last block's Dt, rhs and ring rows
+#pragma unroll
+        for (int k = 0; k < ND; ++k) {
+            const int idx = t + k * TI_THREADS, rr = idx & 31, q = idx >> 5;
+            Dt[rr * TI_DP + q] = q <= rr ? dreg[k] : 0.f;
+        }
+        if (more) fetch_inverse(i0 + 32);
+        for (int kc = kbegin(i0); kc < i0; kc += TI_KC) {
+            const int kn = min(TI_KC, i0 - kc);   // a multiple of 4
+#pragma unroll
+            for (int k = 0; k < NL; ++k) {
+                const int idx = t + k * TI_THREADS;
+                Lt[(idx & 31) * TI_LP + (idx >> 5)] = lreg[k];
             }
             __syncthreads();
-#pragma unroll 8
-            for (int kk = 0; kk < kn; ++kk) {
-                const float l = Lt[r * (TI_KC + 1) + kk];
-                const float2 m = *reinterpret_cast<const float2 *>(ring + (int64_t)((kc + kk) & (R - 1)) * TI_G + gp);
-                a0 = fmaf(l, m.x, a0);
-                a1 = fmaf(l, m.y, a1);
+            if (kc + TI_KC < i0)
+                fetch_band(i0, kc + TI_KC);
+            else if (more)
+                fetch_band(i0 + 32, kbegin(i0 + 32));
+            // four columns of the band a step; R is a power of two, so four slots never wrap
+#pragma unroll 4
+            for (int kk = 0; kk < kn; kk += 4) {
+                const float4 l = at4(Lt + r * TI_LP + kk);
+                const float *m = ring + gp * R + ((kc + kk) & (R - 1));
+                a0 = fma4x(l, at4(m), a0);
+                a1 = fma4x(l, at4(m + R), a1);
             }
             __syncthreads();
         }
+        if (i0 == first && more) fetch_band(i0 + 32, kbegin(i0 + 32));   // no chunk before it
         const int i = i0 + r;
-        {
-            float e0 = -a0, e1 = -a1;
-            if (i == c0 + gp) e0 += 1.f;
-            if (i == c0 + gp + 1) e1 += 1.f;
-            rhs[r * TI_G + gp] = e0;
-            rhs[r * TI_G + gp + 1] = e1;
-        }
+        rhs[gp * TI_DP + r] = (i == c0 + gp ? 1.f : 0.f) - a0;
+        rhs[(gp + 1) * TI_DP + r] = (i == c0 + gp + 1 ? 1.f : 0.f) - a1;
         __syncthreads();
         float x0 = 0.f, x1 = 0.f;
-        const float2 *dblk = D + (int64_t)(i0 >> 5) * 1024 + r;
-#pragma unroll 8
-        for (int q = 0; q < 32; ++q) {
-            const float d = q <= r ? dblk[q * 32].x : 0.f;
-            x0 = fmaf(d, rhs[q * TI_G + gp], x0);
-            x1 = fmaf(d, rhs[q * TI_G + gp + 1], x1);
+#pragma unroll
+        for (int q = 0; q < 32; q += 4) {
+            const float4 d = at4(Dt + r * TI_DP + q);
+            x0 = fma4x(d, at4(rhs + gp * TI_DP + q), x0);
+            x1 = fma4x(d, at4(rhs + (gp + 1) * TI_DP + q), x1);
         }
-        float *slot = ring + (int64_t)(i & (R - 1)) * TI_G + gp;
-        slot[0] = x0;
-        slot[1] = x1;
+        ring[gp * R + (i & (R - 1))] = x0;
+        ring[(gp + 1) * R + (i & (R - 1))] = x1;
         if (i < n) {
             const int ca = c0 + gp, cb = ca + 1;
             if (ca < n && i >= ca) M32[(int64_t)i + (int64_t)n * ca] = x0;
             if (cb < n && i >= cb) M32[(int64_t)i + (int64_t)n * cb] = x1;
         }
-        __syncthreads();
-        rhs[r * TI_G + gp] = x0;
-        rhs[r * TI_G + gp + 1] = x1;
+        // the transpose into the upper triangle, so that the stores run along the columns
         __syncthreads();
         for (int idx = t; idx < 32 * TI_G; idx += TI_THREADS) {
             const int g = idx % TI_G, rr = idx / TI_G;
             const int cc = c0 + g, ii = i0 + rr;
-            if (ii < n && cc < n && ii > cc) M32[(int64_t)cc + (int64_t)n * ii] = rhs[rr * TI_G + g];
+            if (ii < n && cc < n && ii > cc) M32[(int64_t)cc + (int64_t)n * ii] = ring[g * R + (ii & (R - 1))];
         }
-        __syncthreads();
     }
 }
 
-size_t trinv32_smem_bytes(int R, int G) { return sizeof(float) * ((size_t)R * G + 32 * (TI_KC + 1) + 32 * G); }
+size_t trinv32_smem_bytes(int R, int G) {
+    return sizeof(float) * ((size_t)R * G + 32 * TI_LP + 32 * TI_DP + G * TI_DP);
+}
 
 // launches of the two sweeps for the context's column-group width
 template <int G>

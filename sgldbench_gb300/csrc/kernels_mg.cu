@@ -588,35 +588,54 @@ __constant__ int c_cdx[8] = {0, 1, 1, 0, 0, 1, 1, 0};
 __constant__ int c_cdz[8] = {0, 0, 0, 0, 1, 1, 1, 1};
 __constant__ double c_dKe[24];
 
+// UNIFORM: all 24 diagonal entries of Ke are equal, as for an isotropic cube, so the sum
+// of the 8 moduli times that entry serves all three components: 9 FP64 operations per
+// node instead of 24 (256 x 128 x 128: 176 -> 79 us).
+template <bool UNIFORM>
 __global__ void k_diag_finest(const double *__restrict__ E, const uint8_t *__restrict__ nflag, int ny, int nx, int nz,
                               double *__restrict__ D) {
     const int NY = ny + 1, NX = nx + 1, NZ = nz + 1;
     const int64_t nn = (int64_t)NY * NX * NZ;
     const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (n >= nn) return;
-    double d0 = 0.0, d1 = 0.0, d2 = 0.0;
+    double d[3] = {0.0, 0.0, 0.0};
     if (nflag[n] & NF_ACTIVE) {
         const int iy = (int)(n % NY), ix = (int)((n / NY) % NX), iz = (int)(n / ((int64_t)NY * NX));
+#pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int ey = iy - c_cdy[j], ex = ix - c_cdx[j], ez = iz - c_cdz[j];
             if (ey < 0 || ex < 0 || ez < 0 || ey >= ny || ex >= nx || ez >= nz) continue;
             const double ev = E[(int64_t)ey + (int64_t)ny * (ex + (int64_t)nx * ez)];
-            d0 += c_dKe[3 * j] * ev;
-            d1 += c_dKe[3 * j + 1] * ev;
-            d2 += c_dKe[3 * j + 2] * ev;
+            if (UNIFORM) {
+                d[0] += ev;
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) d[c] += c_dKe[3 * j + c] * ev;
+            }
         }
+        if (UNIFORM) d[0] = d[1] = d[2] = d[0] * c_dKe[0];
     }
-    D[3 * n] = d0;
-    D[3 * n + 1] = d1;
-    D[3 * n + 2] = d2;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) D[3 * n + c] = d[c];
 }
 
 void launch_diag_finest(const Level &l0, const double *E, const double *Ke, double *diag, cudaStream_t s) {
-    double dk[24];
-    for (int i = 0; i < 24; ++i) dk[i] = Ke[i + 24 * i];
+    double dk[24], mean = 0.0;
+    for (int i = 0; i < 24; ++i) {
+        dk[i] = Ke[i + 24 * i];
+        mean += dk[i] / 24.0;
+    }
+    bool uniform = true;   // to rounding
+    for (int i = 0; i < 24; ++i) uniform = uniform && fabs(dk[i] - mean) <= 1e-15 * fabs(mean);
+    if (uniform)
+        for (int i = 0; i < 24; ++i) dk[i] = mean;
     cudaMemcpyToSymbolAsync(c_dKe, dk, sizeof dk, 0, cudaMemcpyHostToDevice, s);
     ++g_launches;
-    k_diag_finest<<<(unsigned)((l0.nnode + 255) / 256), 256, 0, s>>>(E, l0.nflag, l0.ny, l0.nx, l0.nz, diag);
+    const unsigned nb = (unsigned)((l0.nnode + 255) / 256);
+    if (uniform)
+        k_diag_finest<true><<<nb, 256, 0, s>>>(E, l0.nflag, l0.ny, l0.nx, l0.nz, diag);
+    else
+        k_diag_finest<false><<<nb, 256, 0, s>>>(E, l0.nflag, l0.ny, l0.nx, l0.nz, diag);
 }
 
 __global__ void k_diag_from_Ks(const double *__restrict__ Ks, const uint8_t *__restrict__ eact,
@@ -649,19 +668,29 @@ void launch_diag_from_Ks(const Level &l, double *diag, cudaStream_t s) {
     k_diag_from_Ks<<<(unsigned)((l.nnode + 255) / 256), 256, 0, s>>>(l.Ks, l.eact, l.nflag, l.ny, l.nx, l.nz, diag);
 }
 
+// a thread per node: the finest level's three entries are equal, one division then
 __global__ void k_inverse_diag(const double *__restrict__ D, const uint8_t *__restrict__ nflag, int64_t nn,
                                double omega2, double *__restrict__ iD, float *__restrict__ iD32) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= 3 * nn) return;
-    const double v = (nflag[i / 3] & NF_ACTIVE) ? omega2 / D[i] : 0.0;
-    iD[i] = v;
-    iD32[i] = (float)v;
+    const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (n >= nn) return;
+    double v[3] = {0.0, 0.0, 0.0};
+    if (nflag[n] & NF_ACTIVE) {
+        const double d0 = D[3 * n], d1 = D[3 * n + 1], d2 = D[3 * n + 2];
+        v[0] = v[1] = v[2] = omega2 / d0;
+        if (d1 != d0) v[1] = omega2 / d1;
+        if (d2 != d0) v[2] = omega2 / d2;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        iD[3 * n + c] = v[c];
+        iD32[3 * n + c] = (float)v[c];
+    }
 }
 
 void launch_inverse_diag(const Level &l, double omega, cudaStream_t s) {
     ++g_launches;
-    k_inverse_diag<<<(unsigned)((3 * l.nnode + 255) / 256), 256, 0, s>>>(l.diag, l.nflag, l.nnode, 2.0 * omega, l.idiag,
-                                                                      l.idiag32);
+    k_inverse_diag<<<(unsigned)((l.nnode + 255) / 256), 256, 0, s>>>(l.diag, l.nflag, l.nnode, 2.0 * omega, l.idiag,
+                                                                     l.idiag32);
 }
 
 // ---- compact <-> full conversions -------------------------------------------
