@@ -130,7 +130,7 @@ template <typename TIn>
 __global__ void __launch_bounds__(256, 1) k_conv_wgrad(const TIn *__restrict__ in, int cin,
                                                     const float *__restrict__ g, int cout, int taps, int ny, int nx,
                                                     int nz, int64_t vchunk, float *__restrict__ part,
-                                                    float *__restrict__ bpart) {
+                                                    int64_t pstride) {
     __shared__ __align__(16) float Xs[WG_BV * (CV_CMAX + 4)];
     __shared__ __align__(16) float Gs[WG_BV * (CV_CMAX + 4)];
     __shared__ float red[256 * 4];
@@ -188,7 +188,8 @@ __global__ void __launch_bounds__(256, 1) k_conv_wgrad(const TIn *__restrict__ i
         __syncthreads();
     }
     // sum the vsplit groups of each (ci, co) block: 16 + 4 values per thread
-    float *outw = part + ((int64_t)s * taps + t) * cin * cout;
+    float *outw = part + (int64_t)s * pstride + (int64_t)t * cin * cout;
+    float *bout = part + (int64_t)s * pstride + (int64_t)taps * cin * cout;
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
         __syncthreads();
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(256, 1) k_conv_wgrad(const TIn *__restrict__ i
                 if (q < 4)
                     outw[(4 * ci4 + q) * cout + co] = sum[j];
                 else if (centre && ci4 == 0)
-                    bpart[(int64_t)s * cout + co] = sum[j];
+                    bout[co] = sum[j];
             }
         }
     }
@@ -351,16 +352,26 @@ __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, 
 // loss = sum se / (C sum m); gy *= 2 / (C sum m)
 __global__ void k_mse_finish(const double *__restrict__ part, int nb, int C, int64_t n, float *__restrict__ gy,
                              double *__restrict__ loss) {
-    __shared__ double sc;
-    if (threadIdx.x == 0) {
-        double se = 0.0, sm = 0.0;
-        for (int b = 0; b < nb; ++b) {
-            se += part[2 * b];
-            sm += part[2 * b + 1];
+    __shared__ double sc, r1[256], r2[256];
+    double se = 0.0, sm = 0.0;
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+        se += part[2 * b];
+        sm += part[2 * b + 1];
+    }
+    r1[threadIdx.x] = se;
+    r2[threadIdx.x] = sm;
+    __syncthreads();
+    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+        if ((int)threadIdx.x < s) {
+            r1[threadIdx.x] += r1[threadIdx.x + s];
+            r2[threadIdx.x] += r2[threadIdx.x + s];
         }
-        const double den = (double)C * (sm > 0.0 ? sm : 1.0);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const double den = (double)C * (r2[0] > 0.0 ? r2[0] : 1.0);
         sc = 2.0 / den;
-        if (blockIdx.x == 0) *loss = se / den;
+        if (blockIdx.x == 0) *loss = r1[0] / den;
     }
     __syncthreads();
     const float f = (float)sc;
@@ -414,10 +425,12 @@ static bool net_cuda_cores() {
     return v;
 }
 
+bool net_on_tensor_cores(int cin, int cout) { return net_conv_tc_fits(cin, cout) && !net_cuda_cores(); }
+
 void net_conv_fwd(const bf16 *in, int cin, const bf16 *w, const float *b, int cout, int taps, int ny, int nx, int nz,
-                  bool relu_bf16_out, void *out, bf16 *wimg, int *err, cudaStream_t s) {
-    if (wimg && net_conv_tc_fits(cin, cout) && !net_cuda_cores()) {
-        net_conv_fwd_tc(in, cin, w, b, cout, taps, ny, nx, nz, relu_bf16_out, out, wimg, err, s);
+                  bool relu_bf16_out, void *out, const bf16 *wimg, int *err, cudaStream_t s) {
+    if (net_on_tensor_cores(cin, cout)) {
+        net_conv_fwd_tc(in, cin, wimg, b, cout, taps, ny, nx, nz, relu_bf16_out, out, err, s);
         return;
     }
     const int64_t V = (int64_t)ny * nx * nz;
@@ -432,17 +445,17 @@ void net_conv_fwd(const bf16 *in, int cin, const bf16 *w, const float *b, int co
 }
 
 // data gradient: gin (=/+=) mask(conv(gout, flipped w)); wt is scratch of taps*cin*cout
-void net_conv_bwd_data(const float *gout, int cout, const bf16 *w, bf16 *wt, int cin, int taps, int ny, int nx,
-                       int nz, const bf16 *mask, float *gin, bool accumulate, bf16 *wimg, int *err, cudaStream_t s) {
-    const int64_t V = (int64_t)ny * nx * nz;
-    const int64_t nw = (int64_t)taps * cin * cout;
-    ++g_launches;
-    k_wflip<<<nblk(nw), 256, 0, s>>>(w, taps, cin, cout, wt);
-    if (wimg && net_conv_tc_fits(cout, cin) && !net_cuda_cores()) {
-        net_conv_bwd_data_tc(gout, cout, wt, cin, taps, ny, nx, nz, mask, gin, accumulate, wimg, err, s);
+void net_conv_bwd_data(const float *gout, const bf16 *g16, int cout, const bf16 *w, bf16 *wt, int cin, int taps, int ny,
+                       int nx, int nz, const bf16 *mask, float *gin, bool accumulate, const bf16 *wimg, int *err,
+                       cudaStream_t s) {
+    if (net_on_tensor_cores(cout, cin)) {
+        net_conv_bwd_data_tc(g16, cout, wimg, cin, taps, ny, nx, nz, mask, gin, accumulate, err, s);
         return;
     }
-    ++g_launches;
+    const int64_t V = (int64_t)ny * nx * nz;
+    const int64_t nw = (int64_t)taps * cin * cout;
+    g_launches += 2;
+    k_wflip<<<nblk(nw), 256, 0, s>>>(w, taps, cin, cout, wt);
     const int threads = 32 * (((cin + 3) & ~3) / 4);
     k_conv<float, 2><<<nblk(V, CV_BM), threads, conv_smem(cout, cin), s>>>(gout, cout, wt, nullptr, cin, taps, ny, nx,
                                                                            nz, gin, mask, accumulate ? 1 : 0);
@@ -453,23 +466,21 @@ int net_wgrad_splits(int64_t V) {
     return (int)(s < 1 ? 1 : (s > 64 ? 64 : s));
 }
 
-// gw = dL/dw [taps][cin][cout], gb = dL/db [cout]; part holds S*(taps*cin*cout + cout) floats
-void net_conv_wgrad(const bf16 *in, int cin, const float *gout, int cout, int taps, int ny, int nx, int nz,
-                    float *part, float *gw, float *gb, int *err, cudaStream_t s) {
+// part holds S * (taps*cin*cout + cout) floats
+void net_conv_wgrad(const bf16 *in, int cin, const float *gout, const bf16 *g16, int cout, int taps, int ny, int nx,
+                    int nz, float *part, float *gwb, int *err, cudaStream_t s) {
     const int64_t V = (int64_t)ny * nx * nz;
     const int S = net_wgrad_splits(V);
     const int64_t vchunk = (V + S - 1) / S;
-    const int64_t nw = (int64_t)taps * cin * cout;
-    float *bpart = part + (int64_t)S * nw;
-    g_launches += 2;
-    if (err && net_wgrad_tc_fits(cin, cout) && !net_cuda_cores()) {
-        net_conv_wgrad_tc(in, cin, gout, cout, taps, ny, nx, nz, S, vchunk, part, bpart, err, s);
+    const int64_t nw = (int64_t)taps * cin * cout + cout;
+    if (net_on_tensor_cores(cin, cout) && net_wgrad_tc_fits(cin, cout)) {
+        net_conv_wgrad_tc(in, cin, g16, cout, taps, ny, nx, nz, S, vchunk, part, nw, err, s);
     } else {
         ++g_launches;
-        k_conv_wgrad<bf16><<<dim3(taps, S), 256, 0, s>>>(in, cin, gout, cout, taps, ny, nx, nz, vchunk, part, bpart);
+        k_conv_wgrad<bf16><<<dim3(taps, S), 256, 0, s>>>(in, cin, gout, cout, taps, ny, nx, nz, vchunk, part, nw);
     }
-    k_sum_parts<<<nblk(nw), 256, 0, s>>>(part, nw, S, gw);
-    k_sum_parts<<<nblk(cout), 256, 0, s>>>(bpart, cout, S, gb);
+    ++g_launches;
+    k_sum_parts<<<nblk(nw), 256, 0, s>>>(part, nw, S, gwb);
 }
 
 void net_pool(const bf16 *f, int C, const int fd[3], const int cd[3], bf16 *c, cudaStream_t s) {

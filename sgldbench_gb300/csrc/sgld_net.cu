@@ -42,24 +42,25 @@ const int *dim3_of(const Net &n, int l) { return n.dims[l]; }
 void conv_fwd(Net &n, int k, const bf16 *in, void *out, bool relu) {
     const NetConv &c = n.conv[k];
     const int *d = dim3_of(n, c.level);
-    net_conv_fwd(in, c.cin, n.wb + c.w, n.w + c.b, c.cout, c.taps, d[0], d[1], d[2], relu, out, n.wimg, n.tc_err,
-                 n.s);
+    net_conv_fwd(in, c.cin, n.wb + c.w, n.w + c.b, c.cout, c.taps, d[0], d[1], d[2], relu, out,
+                 n.wimg + n.images.at[k], n.tc_err, n.s);
 }
 
-// dW, db of convolution k from its input activation and the gradient of its output
+// dW, db of convolution k from its input activation and the gradient of its output,
+// which is left rounded to BF16 in n.g16 for conv_bwd
 void conv_wgrad(Net &n, int k, const bf16 *in, const float *gout) {
     const NetConv &c = n.conv[k];
     const int *d = dim3_of(n, c.level);
-    net_conv_wgrad(in, c.cin, gout, c.cout, c.taps, d[0], d[1], d[2], n.wpart, n.g + c.w, n.g + c.b, n.tc_err,
-                   n.s);
+    if (net_on_tensor_cores(c.cin, c.cout)) net_to_bf16(gout, n.g16, n.V[c.level] * c.cout, n.s);
+    net_conv_wgrad(in, c.cin, gout, n.g16, c.cout, c.taps, d[0], d[1], d[2], n.wpart, n.g + c.w, n.tc_err, n.s);
 }
 
-// gradient of convolution k's input: gin (=/+=) mask(conv^T(gout))
+// gradient of convolution k's input, after conv_wgrad of the same k: gin (=/+=) mask(conv^T(gout))
 void conv_bwd(Net &n, int k, const float *gout, const bf16 *mask, float *gin, bool acc) {
     const NetConv &c = n.conv[k];
     const int *d = dim3_of(n, c.level);
-    net_conv_bwd_data(gout, c.cout, n.wb + c.w, n.wt, c.cin, c.taps, d[0], d[1], d[2], mask, gin, acc, n.wimg,
-                      n.tc_err, n.s);
+    net_conv_bwd_data(gout, n.g16, c.cout, n.wb + c.w, n.wt, c.cin, c.taps, d[0], d[1], d[2], mask, gin, acc,
+                      n.wimg + n.images.at[k], n.tc_err, n.s);
 }
 
 int conv_a(int l) { return 2 * l; }
@@ -112,11 +113,20 @@ int net_init(Net &n, int ny, int nx, int nz, int cin, int cout, int L, const int
         add(n.width[l], n.width[l], 27, l);
     }
     add(n.width[0], cout, 1, 0);
-    int64_t wmax = 0, pmax = 0, imax = 0;
+    int64_t wmax = 0, pmax = 0, gmax = 0;
+    NetImages &im = n.images;
+    im.n = 0;
+    im.at[0] = 0;
     for (const NetConv &c : n.conv) {
         const int64_t nw = (int64_t)c.taps * c.cin * c.cout;
         wmax = std::max(wmax, nw);
-        imax = std::max(imax, (int64_t)c.taps * ((c.cin + 15) & ~15) * ((c.cout + 15) & ~15));
+        gmax = std::max(gmax, n.V[c.level] * c.cout);
+        im.taps[im.n] = c.taps;
+        im.cin[im.n] = c.cin;
+        im.cout[im.n] = c.cout;
+        im.w[im.n] = c.w;
+        im.at[im.n + 1] = im.at[im.n] + (int64_t)c.taps * ((c.cin + 15) & ~15) * ((c.cout + 15) & ~15);
+        ++im.n;
         pmax = std::max(pmax, (int64_t)net_wgrad_splits(n.V[c.level]) * (nw + c.cout));
     }
     cudaError_t e = cudaSuccess;
@@ -128,7 +138,8 @@ int net_init(Net &n, int ny, int nx, int nz, int cin, int cout, int L, const int
     NA(&n.g, n.nparam);
     NA(&n.wb, n.nparam);
     NA(&n.wt, wmax);
-    NA(&n.wimg, imax);
+    NA(&n.wimg, im.at[im.n]);
+    NA(&n.g16, gmax);
     NA(&n.tc_err, 1);
     if (e == cudaSuccess) e = cudaMemsetAsync(n.tc_err, 0, sizeof(int), s);
     NA(&n.wpart, pmax);
@@ -197,6 +208,7 @@ void net_free(Net &n) {
 
 void net_forward(Net &n) {
     const int L = n.L;
+    net_weight_images(n.wb, n.images, false, n.wimg, n.s);
     for (int l = 0; l < L; ++l) {
         conv_fwd(n, conv_a(l), l == 0 ? n.X.a : n.P[l].a, n.Ea[l].a, true);
         conv_fwd(n, conv_b(l), n.Ea[l].a, n.E[l].a, true);
@@ -218,6 +230,7 @@ void net_loss(Net &n, const float *T, const float *M) {
 
 void net_backward(Net &n) {
     const int L = n.L;
+    net_weight_images(n.wb, n.images, true, n.wimg, n.s);
     NetAct &last = L > 1 ? n.D[0] : n.E[0];
     conv_wgrad(n, conv_head(n), last.a, n.gY);
     conv_bwd(n, conv_head(n), n.gY, last.a, last.g, false);

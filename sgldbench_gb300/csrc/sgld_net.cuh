@@ -32,6 +32,13 @@ struct NetConv {
     int64_t w, b;   // offsets into the parameter vector
 };
 
+// the tensor-core operand images of all convolutions' weights (offsets in elements)
+struct NetImages {
+    int n = 0;
+    int taps[4 * NET_MAXL], cin[4 * NET_MAXL], cout[4 * NET_MAXL];
+    int64_t w[4 * NET_MAXL], at[4 * NET_MAXL + 1];   // weights, and image c at at[c] .. at[c + 1]
+};
+
 struct NetAct {
     int level = 0, C = 0;
     bf16 *a = nullptr;    // activation [V][C]
@@ -46,7 +53,10 @@ struct Net {
     int64_t nparam = 0;
     float *w = nullptr, *m = nullptr, *v = nullptr, *g = nullptr, *wpart = nullptr;
     bf16 *wb = nullptr, *wt = nullptr;
-    bf16 *wimg = nullptr;   // one convolution's weights as tensor-core operand images (all taps)
+    NetImages images;
+    bf16 *wimg = nullptr;   // all convolutions' weights as tensor-core operand images, of the last
+                            // forward pass, or flipped, of the last backward pass
+    bf16 *g16 = nullptr;    // the gradient in work, rounded to BF16 as an operand
     int *tc_err = nullptr;  // set by a tensor-core convolution whose MMA wait gave up
     NetAct X, Ea[NET_MAXL], E[NET_MAXL], P[NET_MAXL], Du[NET_MAXL], S[NET_MAXL], D[NET_MAXL];
     bf16 *x_own = nullptr;   // the network's own input buffer (X.a may point elsewhere)
@@ -70,25 +80,29 @@ bool net_take_error(Net &n);
 
 // kernels_net.cu
 void net_init_attributes();
-// wimg: scratch for the weight images of the tensor-core path (taps x pad16(cin) x
-// pad16(cout) BF16); err: device flag of that path
+// wimg: this convolution's weight images (tensor-core path; flipped ones for the data
+// gradient); g16: gout rounded to BF16 (tensor-core path); err: device flag of that path
+bool net_on_tensor_cores(int cin, int cout);
+void net_weight_images(const bf16 *w, const NetImages &im, bool flip, bf16 *out, cudaStream_t s);
 void net_conv_fwd(const bf16 *in, int cin, const bf16 *w, const float *b, int cout, int taps, int ny, int nx, int nz,
-                  bool relu_bf16_out, void *out, bf16 *wimg, int *err, cudaStream_t s);
-void net_conv_bwd_data(const float *gout, int cout, const bf16 *w, bf16 *wt, int cin, int taps, int ny, int nx,
-                       int nz, const bf16 *mask, float *gin, bool accumulate, bf16 *wimg, int *err, cudaStream_t s);
+                  bool relu_bf16_out, void *out, const bf16 *wimg, int *err, cudaStream_t s);
+void net_conv_bwd_data(const float *gout, const bf16 *g16, int cout, const bf16 *w, bf16 *wt, int cin, int taps, int ny,
+                       int nx, int nz, const bf16 *mask, float *gin, bool accumulate, const bf16 *wimg, int *err,
+                       cudaStream_t s);
 // kernels_net_tc.cu: the same convolutions on the tensor cores (tcgen05)
 bool net_conv_tc_fits(int cin, int cout);
 bool net_wgrad_tc_fits(int cin, int cout);
-void net_conv_wgrad_tc(const bf16 *in, int cin, const float *gout, int cout, int taps, int ny, int nx, int nz, int S,
-                       int64_t vchunk, float *part, float *bpart, int *err, cudaStream_t s);
+void net_conv_wgrad_tc(const bf16 *in, int cin, const bf16 *gout, int cout, int taps, int ny, int nx, int nz, int S,
+                       int64_t vchunk, float *part, int64_t pstride, int *err, cudaStream_t s);
 void net_tc_init_attributes();
-void net_conv_fwd_tc(const bf16 *in, int cin, const bf16 *w, const float *b, int cout, int taps, int ny, int nx,
-                     int nz, bool relu_bf16_out, void *out, bf16 *wimg, int *err, cudaStream_t s);
-void net_conv_bwd_data_tc(const float *gout, int cout, const bf16 *wt, int cin, int taps, int ny, int nx, int nz,
-                          const bf16 *mask, float *gin, bool accumulate, bf16 *wimg, int *err, cudaStream_t s);
+void net_conv_fwd_tc(const bf16 *in, int cin, const bf16 *wimg, const float *b, int cout, int taps, int ny, int nx,
+                     int nz, bool relu_bf16_out, void *out, int *err, cudaStream_t s);
+void net_conv_bwd_data_tc(const bf16 *gout, int cout, const bf16 *wimg, int cin, int taps, int ny, int nx, int nz,
+                          const bf16 *mask, float *gin, bool accumulate, int *err, cudaStream_t s);
 int net_wgrad_splits(int64_t V);
-void net_conv_wgrad(const bf16 *in, int cin, const float *gout, int cout, int taps, int ny, int nx, int nz,
-                    float *part, float *gw, float *gb, int *err, cudaStream_t s);
+// gwb: dL/dw [taps][cin][cout], then dL/db [cout]
+void net_conv_wgrad(const bf16 *in, int cin, const float *gout, const bf16 *g16, int cout, int taps, int ny, int nx,
+                    int nz, float *part, float *gwb, int *err, cudaStream_t s);
 void net_pool(const bf16 *f, int C, const int fd[3], const int cd[3], bf16 *c, cudaStream_t s);
 void net_pool_bwd(const float *gc, int C, const int fd[3], const int cd[3], const bf16 *maskf, float *gf,
                   bool accumulate, cudaStream_t s);

@@ -90,6 +90,10 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+// both operands MN-major instead (transpose bits of A and B): a core matrix is then 8 K rows
+// of 16 bytes, 8 elements along M or N; in the descriptor the stride byte offset leads
+// to the next core matrix along M or N, the leading byte offset to the next along K
+constexpr uint32_t IDESC_MN_MAJOR = (1u << 15) | (1u << 16);
 // D[tmem] (+)= A * B^T over K = 16; issued by one thread
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
