@@ -41,18 +41,58 @@ __device__ double msum_partials(const double *__restrict__ part, int nb) {
     return mblock_reduce((s0 + s1) + (s2 + s3));
 }
 
+// The vector updates of the inner CG sum up to ICG_FUSE_PARTS partials themselves, every
+// CTA for itself (the same sum in the same order, so the same value): alpha and beta
+// then cost no launch of their own.  An FP64 instruction holds an SM's scheduler for 64
+// clocks, so the sum is spread over one warp per scheduler and the updates run as few
+// large CTAs.  (Summed by 8 CTAs of 8 warps per SM, all warps taking part, the mixed
+// solve on 64 x 32 x 32 went from 5.67 to 6.47 ms; with this form to 5.25.)  Past
+// ICG_FUSE_PARTS k_icg_scalar's launch is the cheaper one: 192 x 96 x 96 blob shape, 1862
+// partials of z.s, load study 56.5 ms with them summed by the update, 50.8 by the launch.
+constexpr int UB = 512;   // threads of an update
+constexpr int UGRID = 152 * 2;
+constexpr int ICG_FUSE_PARTS = 1024;
+
+// the sum for thread 0
+__device__ __forceinline__ double usum_partials(const double *__restrict__ part, int nb) {
+    __shared__ double red[4];
+    const int i0 = threadIdx.x, w = i0 >> 5;
+    if (i0 < 128) {
+        double s0 = 0.0, s1 = 0.0;
+        int i = i0;
+#pragma unroll 4
+        for (; i + 128 < nb; i += 256) {
+            s0 += part[i];
+            s1 += part[i + 128];
+        }
+        if (i < nb) s0 += part[i];
+        s0 += s1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_down_sync(0xffffffffu, s0, o);
+        if ((i0 & 31) == 0) red[w] = s0;
+    }
+    __syncthreads();
+    return i0 == 0 ? (red[0] + red[1]) + (red[2] + red[3]) : 0.0;
+}
+
 // inner scalars (FP64 storage): rho = z.s of the last iteration, alpha, beta,
 // r0 = s.s at entry, the iteration count of this inner solve, the current
 // iteration cap, whether the last inner solve stopped at that cap short of
 // its tolerance, and (slot 8) the total over the outer solve (reset by the
 // host at the start of each solve)
-enum { IS_RHO = 0, IS_ALPHA = 1, IS_BETA = 2, IS_R0 = 3, IS_IT = 4, IS_KCAP = 5, IS_CAPHIT = 6, IS_TOT = 8 };
+enum { IS_RHO = 0, IS_ALPHA = 1, IS_BETA = 2, IS_R0 = 3, IS_IT = 4, IS_KCAP = 5, IS_CAPHIT = 6, IS_ZS = 7, IS_TOT = 8 };
+
+// alpha and beta of the inner CG.  z.s of an iteration goes to IS_ZS with beta and
+// to IS_RHO with alpha, so that no launch writes a scalar that another of its CTAs
+// may still have to read.
+__device__ __forceinline__ double icg_beta(double rho, double zs) { return rho != 0.0 ? zs / rho : 0.0; }
+__device__ __forceinline__ double icg_alpha(double zs, double dt) { return dt != 0.0 ? zs / dt : 0.0; }
 
 // op 0 (entry of an inner solve): r0 = sum, rho = 0, it = 0, and the cap:
 // kbase at the first inner solve of an outer solve, doubled (up to klimit)
 // after an inner solve that hit its cap without reaching its tolerance;
-// op 1: alpha = rho / sum;  op 2: beta = sum / rho (0 on the first iteration,
-// rho = 0), rho = sum
+// op 1: alpha = z.s / sum, rho = z.s;  op 2: beta = sum / rho (0 on the first
+// iteration, rho = 0), z.s = sum
 __global__ void k_icg_scalar(int op, double *__restrict__ sc, const double *__restrict__ part, int nb, int kbase,
                              int klimit) {
     const double s = msum_partials(part, nb);
@@ -69,11 +109,33 @@ __global__ void k_icg_scalar(int op, double *__restrict__ sc, const double *__re
         sc[IS_IT] = 0.0;
         sc[IS_ALPHA] = 0.0;   // the first d update adds alpha * d = 0 to e
     } else if (op == 1) {
-        sc[IS_ALPHA] = (s != 0.0) ? sc[IS_RHO] / s : 0.0;
+        const double zs = sc[IS_ZS];
+        sc[IS_ALPHA] = icg_alpha(zs, s);
+        sc[IS_RHO] = zs;
     } else {
-        sc[IS_BETA] = (sc[IS_RHO] != 0.0) ? s / sc[IS_RHO] : 0.0;
-        sc[IS_RHO] = s;
+        sc[IS_BETA] = icg_beta(sc[IS_RHO], s);
+        sc[IS_ZS] = s;
     }
+}
+
+// alpha (OP 1) or beta (OP 2) for all threads of a CTA, from the nsum partials of its
+// denominator or numerator, or as k_icg_scalar left it (nsum = 0)
+template <int OP>
+__device__ __forceinline__ float icg_coefficient(double *__restrict__ sc, const double *__restrict__ sum, int nsum) {
+    if (nsum == 0) return (float)sc[OP == 1 ? IS_ALPHA : IS_BETA];
+    const double other = sc[OP == 1 ? IS_ZS : IS_RHO];
+    const double s = usum_partials(sum, nsum);
+    __shared__ float coef;
+    if (threadIdx.x == 0) {
+        const double v = OP == 1 ? icg_alpha(other, s) : icg_beta(other, s);
+        if (blockIdx.x == 0) {
+            sc[OP == 1 ? IS_ALPHA : IS_BETA] = v;
+            sc[OP == 1 ? IS_RHO : IS_ZS] = OP == 1 ? other : s;
+        }
+        coef = (float)v;
+    }
+    __syncthreads();
+    return coef;
 }
 
 // end of an inner iteration: count it and keep iterating while it < kmax and
@@ -207,77 +269,91 @@ __device__ __forceinline__ float4 fma4(float a, float4 x, float4 y) {
     return make_float4(fmaf(a, x.x, y.x), fmaf(a, x.y, y.y), fmaf(a, x.z, y.z), fmaf(a, x.w, y.w));
 }
 
-// s -= alpha t; partial sums of s.s (new s) when part != null.  The matching
-// e += alpha d is deferred to the next d update (k_icg_dupdate), or, after the
-// last iteration, to k_widen_dots: d is read there anyway, which saves one
-// pass over e and d per iteration.
-__global__ void k_icg_update(float *__restrict__ e, float *__restrict__ s, const float *__restrict__ d,
-                             const float *__restrict__ t, int64_t n, const double *__restrict__ sc,
-                             double *__restrict__ part) {
-    (void)e;
-    (void)d;
-    const float a = (float)sc[IS_ALPHA];
-    const int64_t n4 = n >> 2, stride = (int64_t)gridDim.x * MB;
+// s -= alpha t; partial sums of s.s (new s).  The matching e += alpha d is deferred to
+// the next d update (k_icg_dupdate), or, after the last iteration, to k_widen_dots: d is
+// read there anyway, which saves one pass over e and d per iteration.  Bound by the
+// vectors' traffic on large grids and by latency on small ones, so a thread's first
+// words are on their way while its CTA sums the partials.
+__device__ __forceinline__ float sq4(float4 v, float acc) {
+    return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, acc))));
+}
+
+__device__ __forceinline__ void store_partial(float acc, double *__restrict__ part) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    __shared__ double wred[UB / 32];
+    if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = (double)acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int k = 0; k < UB / 32; ++k) t += wred[k];
+        part[blockIdx.x] = t;
+    }
+}
+
+__global__ void __launch_bounds__(UB, 4) k_icg_update(float *__restrict__ s, const float *__restrict__ t, int64_t n,
+                                                   double *__restrict__ sc, const double *__restrict__ sum, int nsum,
+                                                   double *__restrict__ part) {
+    const int64_t n4 = n >> 2, stride = (int64_t)gridDim.x * UB, i0 = blockIdx.x * (int64_t)UB + threadIdx.x;
     float4 *s4 = reinterpret_cast<float4 *>(s);
     const float4 *t4 = reinterpret_cast<const float4 *>(t);
+    float4 sv = make_float4(0.f, 0.f, 0.f, 0.f), tv = sv;
+    if (i0 < n4) {
+        sv = s4[i0];
+        tv = t4[i0];
+    }
+    const float a = icg_coefficient<1>(sc, sum, nsum);
     float acc = 0.f;
-    for (int64_t i = blockIdx.x * (int64_t)MB + threadIdx.x; i < n4; i += stride) {
+    if (i0 < n4) {
+        sv = fma4(-a, tv, sv);
+        s4[i0] = sv;
+        acc = sq4(sv, acc);
+    }
+#pragma unroll 2
+    for (int64_t i = i0 + stride; i < n4; i += stride) {
         const float4 v = fma4(-a, t4[i], s4[i]);
         s4[i] = v;
-        acc = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, acc))));
+        acc = sq4(v, acc);
     }
-    const int64_t i = 4 * n4 + blockIdx.x * (int64_t)MB + threadIdx.x;
+    const int64_t i = 4 * n4 + i0;
     if (i < n) {
         const float v = fmaf(-a, t[i], s[i]);
         s[i] = v;
         acc = fmaf(v, v, acc);
     }
-    if (part) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        __shared__ double wred[MB / 32];
-        if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = (double)acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double tt = 0.0;
-            for (int k = 0; k < MB / 32; ++k) tt += wred[k];
-            part[blockIdx.x] = tt;
-        }
-    }
+    store_partial(acc, part);
 }
 
-int launch_icg_update(float *e, float *s, const float *d, const float *t, int64_t n, const double *sc,
-                      double *part, cudaStream_t st) {
-    ++g_launches;
-    const int nb = reduce_blocks(n);
-    k_icg_update<<<nb, MB, 0, st>>>(e, s, d, t, n, sc, part);
-    return nb;
-}
-
-// e += alpha d (the previous iteration's step, alpha still in place); then
-// d = w + beta d
-__global__ void k_icg_dupdate(float *__restrict__ e, float *__restrict__ d, const float *__restrict__ w, int64_t n,
-                              const double *__restrict__ sc) {
-    const float a = (float)sc[IS_ALPHA], b = (float)sc[IS_BETA];
-    const int64_t n4 = n >> 2, stride = (int64_t)gridDim.x * MB;
+// e += alpha d (the previous iteration's step, alpha still in place); then d = w + beta d
+__global__ void __launch_bounds__(UB, 4) k_icg_dupdate(float *__restrict__ e, float *__restrict__ d,
+                                                    const float *__restrict__ w, int64_t n, double *__restrict__ sc,
+                                                    const double *__restrict__ sum, int nsum) {
+    const int64_t n4 = n >> 2, stride = (int64_t)gridDim.x * UB, i0 = blockIdx.x * (int64_t)UB + threadIdx.x;
     float4 *e4 = reinterpret_cast<float4 *>(e), *d4 = reinterpret_cast<float4 *>(d);
     const float4 *w4 = reinterpret_cast<const float4 *>(w);
-    for (int64_t i = blockIdx.x * (int64_t)MB + threadIdx.x; i < n4; i += stride) {
-        const float4 dv = d4[i];
-        e4[i] = fma4(a, dv, e4[i]);
-        d4[i] = fma4(b, dv, w4[i]);
+    float4 ev = make_float4(0.f, 0.f, 0.f, 0.f), dv = ev, wv = ev;
+    if (i0 < n4) {
+        dv = d4[i0];
+        ev = e4[i0];
+        wv = w4[i0];
     }
-    const int64_t i = 4 * n4 + blockIdx.x * (int64_t)MB + threadIdx.x;
+    const float a = (float)sc[IS_ALPHA], b = icg_coefficient<2>(sc, sum, nsum);
+    if (i0 < n4) {
+        e4[i0] = fma4(a, dv, ev);
+        d4[i0] = fma4(b, dv, wv);
+    }
+#pragma unroll 2
+    for (int64_t i = i0 + stride; i < n4; i += stride) {
+        const float4 v = d4[i];
+        e4[i] = fma4(a, v, e4[i]);
+        d4[i] = fma4(b, v, w4[i]);
+    }
+    const int64_t i = 4 * n4 + i0;
     if (i < n) {
-        const float dv = d[i];
-        e[i] = fmaf(a, dv, e[i]);
-        d[i] = fmaf(b, dv, w[i]);
+        const float v = d[i];
+        e[i] = fmaf(a, v, e[i]);
+        d[i] = fmaf(b, v, w[i]);
     }
-}
-
-void launch_icg_dupdate(float *e, float *d, const float *w, int64_t n, const double *sc, cudaStream_t st) {
-    ++g_launches;
-    k_icg_dupdate<<<reduce_blocks(n), MB, 0, st>>>(e, d, w, n, sc);
 }
 
 // ---- the same two updates over the active runs only -------------------------
@@ -287,109 +363,169 @@ void launch_icg_dupdate(float *e, float *d, const float *w, int64_t n, const dou
 // updates may visit only the active nodes' words.
 // The active y-runs (merged where they touch or lie a few nodes apart) are
 // cut into chunks of at most 2048 floats, each cut on a 16-byte boundary
-// (runs[i] = first DOF | floats << 40).  A warp takes a chunk: the words up to
-// the first 16-byte boundary one by one, then float4 groups, then the last
-// words.  Sums visit the chunks in a fixed order.
+// (runs[i] = first DOF | floats << 40).  A warp takes a chunk: float4 groups, and
+// the words before the first and after the last 16-byte boundary one by one.  A
+// chunk is mostly one or two groups a lane, so its time is the latency of its
+// loads: the single words and the first RUN_BATCH groups are loaded together, those of
+// the warp's first chunk before the partials are summed.  (Head words, groups
+// and tail words each with their own loads and stores: 58 and 37 us for the d and s update
+// of the 384 x 192 x 192 blob shape, now 49 and 28; 18.5 and 16.5 us on 192 x 96 x 96, now
+// 13 and 12.)  Sums visit the chunks in a fixed order.
 constexpr int RUN_SHIFT = 40;
 constexpr int64_t RUN_MASK = (int64_t(1) << RUN_SHIFT) - 1;
+constexpr int RUN_BATCH = 4, RUN_BATCH3 = 3;   // groups a lane loads at once, of two and of three vectors
 
-// the chunk's words [b, b + len): head words before a 16-byte boundary, the
-// float4 groups of the body, tail words; f(i) for single words, f4(i4) for a
-// float4 group at float index 4 * i4
-template <typename F1, typename F4>
-__device__ __forceinline__ void run_chunk(int64_t b, int len, int lane, F1 f1, F4 f4) {
-    const int head = min((int)((4 - (b & 3)) & 3), len);
-    if (lane < head) f1(b + lane);
-    const int64_t a4 = (b + head) >> 2;
-    const int n4 = (len - head) >> 2;
-    // unrolled so that several groups' loads are in flight at once
-#pragma unroll 4
-    for (int k = lane; k < n4; k += 32) f4(a4 + k);
-    const int rest = len - head - 4 * n4;
-    if (lane < rest) f1(b + head + 4 * (int64_t)n4 + lane);
-}
-
-__global__ void __launch_bounds__(MB) k_icg_update_runs(float *__restrict__ s, const float *__restrict__ t,
-                                                        const int64_t *__restrict__ runs, int64_t nruns,
-                                                        const double *__restrict__ sc, double *__restrict__ part) {
-    const float a = (float)sc[IS_ALPHA];
-    const int lane = threadIdx.x & 31;
-    const int64_t w0 = (int64_t)blockIdx.x * (MB / 32) + (threadIdx.x >> 5), nw = (int64_t)gridDim.x * (MB / 32);
-    float4 *s4 = reinterpret_cast<float4 *>(s);
-    const float4 *t4 = reinterpret_cast<const float4 *>(t);
-    float acc = 0.f;
-    for (int64_t r = w0; r < nruns; r += nw) {
-        const int64_t rv = runs[r];
-        run_chunk(
-            rv & RUN_MASK, (int)(rv >> RUN_SHIFT), lane,
-            [&](int64_t i) {
-                const float v = fmaf(-a, t[i], s[i]);
-                s[i] = v;
-                acc = fmaf(v, v, acc);
-            },
-            [&](int64_t i4) {
-                const float4 v = fma4(-a, t4[i4], s4[i4]);
-                s4[i4] = v;
-                acc = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, acc))));
-            });
+// a warp's chunk: word `single` of this lane (-1: none), n4 groups from group g4
+struct RunChunk {
+    int64_t single = -1, g4 = 0;
+    int n4 = 0;
+    __device__ __forceinline__ void take(int64_t rv, int lane) {
+        const int64_t b = rv & RUN_MASK;
+        const int len = (int)(rv >> RUN_SHIFT), head = min((int)((4 - (b & 3)) & 3), len);
+        g4 = (b + head) >> 2;
+        n4 = (len - head) >> 2;
+        const int rest = len - head - 4 * n4;
+        single = lane < head ? b + lane : lane >= 4 && lane < 4 + rest ? b + head + 4 * (int64_t)n4 + (lane - 4) : -1;
     }
-    if (part) {
+};
+
+// NV vectors' words of a chunk: the single word and a batch of groups
+template <int NV, int Q>
+struct RunWords {
+    float one[NV];
+    float4 four[Q][NV];
+    __device__ __forceinline__ void load(const RunChunk &c, int k0, const float *const (&v)[NV]) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        __shared__ double wred[MB / 32];
-        if (lane == 0) wred[threadIdx.x >> 5] = (double)acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double tt = 0.0;
-            for (int k = 0; k < MB / 32; ++k) tt += wred[k];
-            part[blockIdx.x] = tt;
-        }
+        for (int j = 0; j < NV; ++j) one[j] = k0 < 32 && c.single >= 0 ? v[j][c.single] : 0.f;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+            for (int j = 0; j < NV; ++j)
+                four[q][j] = k0 + 32 * q < c.n4 ? reinterpret_cast<const float4 *>(v[j])[c.g4 + k0 + 32 * q]
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-}
+};
 
-__global__ void __launch_bounds__(MB) k_icg_dupdate_runs(float *__restrict__ e, float *__restrict__ d,
-                                                         const float *__restrict__ w,
-                                                         const int64_t *__restrict__ runs, int64_t nruns,
-                                                         const double *__restrict__ sc) {
-    const float a = (float)sc[IS_ALPHA], bt = (float)sc[IS_BETA];
+__global__ void __launch_bounds__(UB, 2) k_icg_update_runs(float *s, const float *t, const int64_t *__restrict__ runs,
+                                                        int64_t nruns, double *__restrict__ sc,
+                                                        const double *__restrict__ sum, int nsum,
+                                                        double *__restrict__ part) {
     const int lane = threadIdx.x & 31;
-    const int64_t w0 = (int64_t)blockIdx.x * (MB / 32) + (threadIdx.x >> 5), nw = (int64_t)gridDim.x * (MB / 32);
-    float4 *e4 = reinterpret_cast<float4 *>(e), *d4 = reinterpret_cast<float4 *>(d);
-    const float4 *w4 = reinterpret_cast<const float4 *>(w);
-    for (int64_t r = w0; r < nruns; r += nw) {
-        const int64_t rv = runs[r];
-        run_chunk(
-            rv & RUN_MASK, (int)(rv >> RUN_SHIFT), lane,
-            [&](int64_t i) {
-                const float dv = d[i];
-                e[i] = fmaf(a, dv, e[i]);
-                d[i] = fmaf(bt, dv, w[i]);
-            },
-            [&](int64_t i4) {
-                const float4 dv = d4[i4];
-                e4[i4] = fma4(a, dv, e4[i4]);
-                d4[i4] = fma4(bt, dv, w4[i4]);
-            });
+    const int64_t w0 = (int64_t)blockIdx.x * (UB / 32) + (threadIdx.x >> 5), nw = (int64_t)gridDim.x * (UB / 32);
+    const float *const src[2] = {s, t};
+    RunChunk c;
+    RunWords<2, RUN_BATCH> x;
+    if (w0 < nruns) {
+        c.take(runs[w0], lane);
+        x.load(c, lane, src);
+    }
+    const float a = icg_coefficient<1>(sc, sum, nsum);
+    float acc = 0.f;
+    for (int64_t r = w0; r < nruns;) {
+        const int64_t rv = runs[min(r + nw, nruns - 1)];
+        if (c.single >= 0) {
+            const float v = fmaf(-a, x.one[1], x.one[0]);
+            s[c.single] = v;
+            acc = fmaf(v, v, acc);
+        }
+        for (int k0 = lane;;) {
+#pragma unroll
+            for (int q = 0; q < RUN_BATCH; ++q)
+                if (k0 + 32 * q < c.n4) {
+                    const float4 v = fma4(-a, x.four[q][1], x.four[q][0]);
+                    reinterpret_cast<float4 *>(s)[c.g4 + k0 + 32 * q] = v;
+                    acc = sq4(v, acc);
+                }
+            k0 += 32 * RUN_BATCH;
+            if (k0 - lane >= c.n4) break;
+            x.load(c, k0, src);
+        }
+        if ((r += nw) >= nruns) break;
+        c.take(rv, lane);
+        x.load(c, lane, src);
+    }
+    store_partial(acc, part);
+}
+
+__global__ void __launch_bounds__(UB, 2) k_icg_dupdate_runs(float *e, float *d, const float *w,
+                                                         const int64_t *__restrict__ runs, int64_t nruns,
+                                                         double *__restrict__ sc, const double *__restrict__ sum,
+                                                         int nsum) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w0 = (int64_t)blockIdx.x * (UB / 32) + (threadIdx.x >> 5), nw = (int64_t)gridDim.x * (UB / 32);
+    const float *const src[3] = {e, d, w};
+    RunChunk c;
+    RunWords<3, RUN_BATCH3> x;
+    if (w0 < nruns) {
+        c.take(runs[w0], lane);
+        x.load(c, lane, src);
+    }
+    const float a = (float)sc[IS_ALPHA], b = icg_coefficient<2>(sc, sum, nsum);
+    for (int64_t r = w0; r < nruns;) {
+        const int64_t rv = runs[min(r + nw, nruns - 1)];
+        if (c.single >= 0) {
+            e[c.single] = fmaf(a, x.one[1], x.one[0]);
+            d[c.single] = fmaf(b, x.one[1], x.one[2]);
+        }
+        for (int k0 = lane;;) {
+#pragma unroll
+            for (int q = 0; q < RUN_BATCH3; ++q)
+                if (k0 + 32 * q < c.n4) {
+                    reinterpret_cast<float4 *>(e)[c.g4 + k0 + 32 * q] = fma4(a, x.four[q][1], x.four[q][0]);
+                    reinterpret_cast<float4 *>(d)[c.g4 + k0 + 32 * q] = fma4(b, x.four[q][1], x.four[q][2]);
+                }
+            k0 += 32 * RUN_BATCH3;
+            if (k0 - lane >= c.n4) break;
+            x.load(c, k0, src);
+        }
+        if ((r += nw) >= nruns) break;
+        c.take(rv, lane);
+        x.load(c, lane, src);
     }
 }
 
-static int run_blocks(int64_t nruns) {
-    const int64_t b = (nruns + MB / 32 - 1) / (MB / 32);
-    return (int)(b < 1216 ? (b > 0 ? b : 1) : 1216);   // 152 SMs x 8 CTAs
+// CTAs over the chunks, a warp each, at most `most`: the s update runs best as the two CTAs
+// that an SM holds (384 x 192 x 192 blob shape: 28 us, 32 with 8 per SM), the d update,
+// whose traffic is 2.5 times that, with more, which the SMs take as they finish (49 us, 70 with two)
+static int run_blocks(int64_t nruns, int most) {
+    const int64_t b = (nruns + UB / 32 - 1) / (UB / 32);
+    return (int)(b < most ? (b > 0 ? b : 1) : most);
+}
+static int update_blocks(int64_t n) {
+    const int64_t b = (n / 4 + UB - 1) / UB;
+    return (int)(b < 2 * UGRID ? (b > 0 ? b : 1) : 2 * UGRID);
 }
 
-int launch_icg_update_runs(float *s, const float *t, const int64_t *runs, int64_t nruns, const double *sc,
-                           double *part, cudaStream_t st) {
-    ++g_launches;
-    const int nb = run_blocks(nruns);
-    k_icg_update_runs<<<nb, MB, 0, st>>>(s, t, runs, nruns, sc, part);
-    return nb;
+// the scalar of an update from nb partials: by the update itself, or by a launch before it
+static int icg_sum(int op, double *sc, const double *sum, int nb, cudaStream_t st) {
+    if (nb <= ICG_FUSE_PARTS) return nb;
+    launch_icg_scalar(op, sc, sum, nb, st, 0, 0);
+    return 0;
 }
 
-void launch_icg_dupdate_runs(float *e, float *d, const float *w, const int64_t *runs, int64_t nruns,
-                             const double *sc, cudaStream_t st) {
+void launch_icg_dupdate(float *e, float *d, const float *w, const Level &l0, double *sc, const double *sum, int nb,
+                        cudaStream_t st) {
+    const int nsum = icg_sum(2, sc, sum, nb, st);
     ++g_launches;
-    k_icg_dupdate_runs<<<run_blocks(nruns), MB, 0, st>>>(e, d, w, runs, nruns, sc);
+    if (l0.runs) {
+        k_icg_dupdate_runs<<<run_blocks(l0.nruns, 152 * 8), UB, 0, st>>>(e, d, w, l0.runs, l0.nruns, sc, sum, nsum);
+    } else {
+        const int64_t n = 3 * l0.nnode;
+        k_icg_dupdate<<<update_blocks(n), UB, 0, st>>>(e, d, w, n, sc, sum, nsum);
+    }
+}
+
+int launch_icg_update(float *s, const float *t, const Level &l0, double *sc, const double *sum, int nb, double *part,
+                      cudaStream_t st) {
+    const int nsum = icg_sum(1, sc, sum, nb, st);
+    ++g_launches;
+    const int64_t n = 3 * l0.nnode;
+    const int g = l0.runs ? run_blocks(l0.nruns, UGRID) : update_blocks(n);
+    if (l0.runs)
+        k_icg_update_runs<<<g, UB, 0, st>>>(s, t, l0.runs, l0.nruns, sc, sum, nsum, part);
+    else
+        k_icg_update<<<g, UB, 0, st>>>(s, t, n, sc, sum, nsum, part);
+    return g;
 }
 
 // z64 = e32 + alpha d32 (the last iteration's deferred step; masked at fixed

@@ -424,6 +424,18 @@ static cudaGraph_t capturing_graph(cudaStream_t s) {
 // iteration count (eta <= 0) keeps kmax.
 static int inner_cap_limit(int kmax, double eta) { return eta > 0.0 ? 16 * kmax : kmax; }
 
+// one inner iteration up to its stopping test; returns the number of partials of s.s,
+// which lie past the npart partials of the V-cycle and K*u
+static int inner_iteration(sgld_ctx *ctx, cudaStream_t s) {
+    Ctx &c = ctx->c;
+    const Level &l0 = c.lv[0];
+    int nb = 0;
+    vcycle_dev32(ctx, c.d_s32, c.d_z32, c.d_part2, &nb, s);
+    launch_icg_dupdate(c.d_e32, c.d_d32, c.d_z32, l0, c.d_isc, c.d_part2, nb, s);
+    launch_kbyu_f32(l0, c.d_E32, c.d_d32, c.d_t32, c.d_part2, &nb, s);
+    return launch_icg_update(c.d_s32, c.d_t32, l0, c.d_isc, c.d_part2, nb, c.d_part2 + c.npart, s);
+}
+
 static int capture_inner(sgld_ctx *ctx, cudaStream_t s, cudaStream_t sb, int kmax, double eta, int64_t *entry,
                          int64_t *body_n) {
     Ctx &c = ctx->c;
@@ -441,18 +453,8 @@ static int capture_inner(sgld_ctx *ctx, cudaStream_t s, cudaStream_t sb, int kma
     if (rc) return rc;
     before = g_launches;
     CK(cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    int nb = 0;
-    vcycle_dev32(ctx, c.d_s32, c.d_z32, c.d_part2, &nb, sb);
-    launch_icg_scalar(2, c.d_isc, c.d_part2, nb, sb, 0, 0);
-    if (l0.runs)
-        launch_icg_dupdate_runs(c.d_e32, c.d_d32, c.d_z32, l0.runs, l0.nruns, c.d_isc, sb);
-    else
-        launch_icg_dupdate(c.d_e32, c.d_d32, c.d_z32, nv, c.d_isc, sb);
-    launch_kbyu_f32(l0, c.d_E32, c.d_d32, c.d_t32, c.d_part2, &nb, sb);
-    launch_icg_scalar(1, c.d_isc, c.d_part2, nb, sb, 0, 0);
-    nb = l0.runs ? launch_icg_update_runs(c.d_s32, c.d_t32, l0.runs, l0.nruns, c.d_isc, c.d_part2, sb)
-                 : launch_icg_update(c.d_e32, c.d_s32, c.d_d32, c.d_t32, nv, c.d_isc, c.d_part2, sb);
-    launch_icg_cond(h, c.d_isc, c.d_part2, nb, kmax, eta, c.d_scal, c.d_isc + IS_TOTAL, sb);
+    const int nb = inner_iteration(ctx, sb);
+    launch_icg_cond(h, c.d_isc, c.d_part2 + c.npart, nb, kmax, eta, c.d_scal, c.d_isc + IS_TOTAL, sb);
     CK(cudaStreamEndCapture(sb, &body));
     *body_n = g_launches - before;
     return SGLD_OK;
@@ -495,18 +497,8 @@ static int inner_run_host(sgld_ctx *ctx, int kmax, double eta) {
     launch_icg_scalar(0, c.d_isc, c.d_part2, nbi, c.stream, kmax, inner_cap_limit(kmax, eta));
     const int kl = inner_cap_limit(kmax, eta);
     for (int it = 0; it < kl; ++it) {
-        int nb = 0;
-        vcycle_dev32(ctx, c.d_s32, c.d_z32, c.d_part2, &nb);
-        launch_icg_scalar(2, c.d_isc, c.d_part2, nb, c.stream, 0, 0);
-        if (l0.runs)
-            launch_icg_dupdate_runs(c.d_e32, c.d_d32, c.d_z32, l0.runs, l0.nruns, c.d_isc, c.stream);
-        else
-            launch_icg_dupdate(c.d_e32, c.d_d32, c.d_z32, nv, c.d_isc, c.stream);
-        launch_kbyu_f32(l0, c.d_E32, c.d_d32, c.d_t32, c.d_part2, &nb, c.stream);
-        launch_icg_scalar(1, c.d_isc, c.d_part2, nb, c.stream, 0, 0);
-        nb = l0.runs ? launch_icg_update_runs(c.d_s32, c.d_t32, l0.runs, l0.nruns, c.d_isc, c.d_part2, c.stream)
-                     : launch_icg_update(c.d_e32, c.d_s32, c.d_d32, c.d_t32, nv, c.d_isc, c.d_part2, c.stream);
-        launch_icg_cond_flag(d_flag, c.d_isc, c.d_part2, nb, kmax, eta, c.d_scal, c.d_isc + IS_TOTAL, c.stream);
+        const int nb = inner_iteration(ctx, c.stream);
+        launch_icg_cond_flag(d_flag, c.d_isc, c.d_part2 + c.npart, nb, kmax, eta, c.d_scal, c.d_isc + IS_TOTAL, c.stream);
         int more = 0;
         CK(cudaMemcpyAsync(&more, d_flag, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
         CK(cudaStreamSynchronize(c.stream));
@@ -956,7 +948,7 @@ int sgld_create(int resY, int resX, int resZ, const uint8_t *solid, const sgld_o
                                       (int64_t)(((l0.ny + 1) * (l0.nx + 1) + 255) / 256) * (l0.nz + 1),
                                       (int64_t)((l0.ny + 31) / 31 + 1) * ((l0.nx + 7) / 7 + 1) * ((l0.nz + 16) / 16 + 1)});
     CK(dalloc(&c.d_part, c.npart));
-    CK(dalloc(&c.d_part2, c.npart));
+    CK(dalloc(&c.d_part2, c.npart + 152 * 8));   // and the partials of the inner CG's update
     CK(dalloc(&c.d_scal, 64));
     CK(dalloc(&c.d_iflag, 64));
     CK(cudaMemset(c.d_iflag, 0, 64 * sizeof(int)));

@@ -211,8 +211,12 @@ void launch_kbyu_df(const Level &l0, const double *E, const double *u, double *y
 // op 0 also sets the inner iteration cap (kbase at an outer solve's first inner solve,
 // doubled up to klimit after a capped inner solve that missed its tolerance)
 void launch_icg_scalar(int op, double *sc, const double *part, int nb, cudaStream_t s, int kbase, int klimit);
-int launch_icg_update(float *e, float *s, const float *d, const float *t, int64_t n, const double *sc,
-                      double *part, cudaStream_t st);
+// s -= alpha t and the partials of s.s; e += alpha d, then d = w + beta d.  sum: the nb
+// partials of d.t and of z.s (not the area that update's own partials go to)
+int launch_icg_update(float *s, const float *t, const Level &l0, double *sc, const double *sum, int nb, double *part,
+                      cudaStream_t st);
+void launch_icg_dupdate(float *e, float *d, const float *w, const Level &l0, double *sc, const double *sum, int nb,
+                        cudaStream_t st);
 void launch_icg_cond(cudaGraphConditionalHandle h, double *sc, const double *part, int nb, int kmax,
                      double eta_min, const double *outer, double *total, cudaStream_t s);
 int launch_icg_init(const float *r, float *s, float *e, float *d, int64_t n, double *part, cudaStream_t st);
@@ -221,12 +225,6 @@ void launch_outer_cond(cudaGraphConditionalHandle hw, cudaGraphConditionalHandle
 void launch_set_cond(cudaGraphConditionalHandle h, unsigned v, cudaStream_t s);
 void launch_icg_cond_flag(int *flag, double *sc, const double *part, int nb, int kmax, double eta_min,
                           const double *outer, double *total, cudaStream_t s);
-void launch_icg_dupdate(float *e, float *d, const float *w, int64_t n, const double *sc, cudaStream_t st);
-// the same updates over the finest level's active runs (Level::runs)
-int launch_icg_update_runs(float *s, const float *t, const int64_t *runs, int64_t nruns, const double *sc,
-                           double *part, cudaStream_t st);
-void launch_icg_dupdate_runs(float *e, float *d, const float *w, const int64_t *runs, int64_t nruns,
-                             const double *sc, cudaStream_t st);
 void launch_widen_dots(const float *e, const float *d, const double *sc, double *z, const double *r,
                        const double *q, int64_t n, double *p1,
                        double *p2, int nb, cudaStream_t st);
