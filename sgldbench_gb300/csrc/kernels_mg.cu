@@ -17,6 +17,8 @@
 // 2 omega ./ D_l is formed once per assembly, so a fine node takes one
 // multiply-add, x_l = r_l (2 omega / D_l) + P x_{l+1}, which may differ from the
 // reference's sum in the last bit.
+#include <algorithm>
+
 #include "sgld_internal.cuh"
 
 namespace sgld {
@@ -580,6 +582,276 @@ template void launch_prolong_smooth<double>(const Level &, const Level &, const 
                                             const double *, double *, bool, double *, int *, cudaStream_t);
 template void launch_prolong_smooth<float>(const Level &, const Level &, const float *, const float *, const float *,
                                            float *, bool, double *, int *, cudaStream_t);
+
+// ---- the FP32 V-cycle's small levels -----------------------------------------
+// A launch on a level of a few thousand nodes costs a memory latency and its place in
+// the chain of launches, about 4 us, whatever it computes.  The cycle is additive and
+// its levels are nested by factors of 2, so the chains collapse:
+//   * the product of span-2 restrictions is the tent of span 4, 8, so that up to three
+//     coarser residuals are formed from one level's in one launch;
+//   * trilinear interpolation through the levels in between is trilinear interpolation
+//     on each level's own cell, so a thread that prolongates to 8 fine nodes carries
+//     the 8 corners of its cell down from the coarsest level, adding r (2 omega / D) on
+//     the way; the levels in between are not written at all.
+// The sums are those of the level-by-level launches in another order.  FP32 V-cycle, us:
+// 96 x 48 x 48 51 -> 37, 125 x 61 x 67 blob shape 55 -> 48, 192 x 96 x 96 65 -> 50, 384 x 192 x 192
+// 160 -> 140, 256 x 128 x 128 134 -> 123.
+
+// S-fold restriction at coarse node (I, J, K) by NT threads, one of which writes: taps are
+// read at clamped positions, those past the grid with weight 0
+template <int S, int NT>
+__device__ __forceinline__ void restrict_chain_taps(const float *__restrict__ rf, int I, int J, int K, int nyf, int nxf,
+                                                    int nzf, int t0, float (&a)[3]) {
+    constexpr int W = 2 * S - 1;
+#pragma unroll 9
+    for (int k = 0; k < (W * W * W + NT - 1) / NT; ++k) {
+        const int t = t0 + NT * k, dy = t % W - (S - 1), dx = t / W % W - (S - 1), dz = t / (W * W) - (S - 1);
+        const int y = S * I + dy, x = S * J + dx, z = S * K + dz;
+        const int fy = min(max(y, 0), nyf), fx = min(max(x, 0), nxf), fz = min(max(z, 0), nzf);
+        const bool in = fy == y && fx == x && fz == z;
+        const float w = in && t < W * W * W ? (float)((S - abs(dy)) * (S - abs(dx)) * (S - abs(dz))) : 0.f;
+        const float *r = rf + 3 * (fy + (nyf + 1) * (fx + (nxf + 1) * fz));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c] = fmaf(w, r[c], a[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) a[c] *= 1.f / (float)(S * S * S);
+}
+
+// targets k = 0, 1, 2 lie 1, 2, 3 levels below the base; CTAs in the order 2, 1, 0 (the
+// longest sums first)
+struct RestrictChain {
+    int n = 0;
+    int ny[4], nx[4], nz[4];           // [0] the base, [1 + k] target k
+    const uint8_t *flag[3];
+    float *out[3];
+    int first[3];                      // the target's first CTA
+};
+
+__global__ void __launch_bounds__(128) k_restrict_chain(const float *__restrict__ rf,
+                                                        const __grid_constant__ RestrictChain c) {
+    const int b = blockIdx.x, lane = threadIdx.x & 31;
+    int k = 0;
+    while (k + 1 < c.n && b < c.first[k]) ++k;
+    const int per = k == 0 ? 128 : k == 1 ? 4 : 1;   // coarse nodes per CTA: a thread, a warp, a CTA for each
+    const int i = (b - c.first[k]) * per + (k == 0 ? (int)threadIdx.x : k == 1 ? (int)(threadIdx.x >> 5) : 0);
+    const int NY = c.ny[1 + k] + 1, NX = c.nx[1 + k] + 1;
+    if (i >= NY * NX * (c.nz[1 + k] + 1)) return;
+    if (!(c.flag[k][i] & NF_ACTIVE)) return;          // holds 0 since it was allocated
+    const int I = i % NY, J = i / NY % NX, K = i / (NY * NX);
+    float a[3] = {0.f, 0.f, 0.f};
+    float *out = c.out[k] + 3 * i;
+    if (k == 0) {
+        restrict_chain_taps<2, 1>(rf, I, J, K, c.ny[0], c.nx[0], c.nz[0], 0, a);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) out[q] = a[q];
+        return;
+    }
+    if (k == 1)
+        restrict_chain_taps<4, 32>(rf, I, J, K, c.ny[0], c.nx[0], c.nz[0], lane, a);
+    else
+        restrict_chain_taps<8, 128>(rf, I, J, K, c.ny[0], c.nx[0], c.nz[0], (int)threadIdx.x, a);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
+    if (k == 1) {
+        if (lane < 3) out[lane] = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];
+        return;
+    }
+    __shared__ float red[4][3];
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) red[threadIdx.x >> 5][q] = a[q];
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        const int q = threadIdx.x;
+        out[q] = (red[0][q] + red[1][q]) + (red[2][q] + red[3][q]);
+    }
+}
+
+// levels by distance from the output's: [0] the next coarser one, [M] the coarsest, whose
+// solution x is given; r and D of the M levels in between
+template <int M>
+struct ProlongChain {
+    int ny[M + 1], nx[M + 1], nz[M + 1];
+    const float *r[M], *D[M], *x;
+};
+
+// corners of a cell's half along one axis: index bit `step` of v, half b
+__device__ __forceinline__ void half_cell(float (&v)[8], int step, int b) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (k & step) continue;
+        const float lo = v[k], hi = v[k | step], mid = 0.5f * (lo + hi);
+        v[k] = b ? mid : lo;
+        v[k | step] = b ? hi : mid;
+    }
+}
+
+// x_f = r_f .* D + P x_c as k_prolong_cells, a thread per node of the next coarser level
+template <int M, bool FINAL>
+__global__ void __launch_bounds__(128) k_prolong_chain(const __grid_constant__ ProlongChain<M> c,
+                                                       const float *__restrict__ rf, const float *__restrict__ D,
+                                                       const uint8_t *__restrict__ nflag, float *__restrict__ xf,
+                                                       double *__restrict__ partial) {
+    const int nyc = c.ny[0], nxc = c.nx[0], nzc = c.nz[0];
+    const int NYc = nyc + 1, NXc = nxc + 1, NYf = 2 * nyc + 1, NXf = 2 * nxc + 1;
+    const int pl = blockIdx.x * blockDim.x + threadIdx.x;
+    float dot = 0.f;
+    if (pl < NYc * NXc) {
+        const int I = pl % NYc, J = pl / NYc, K = blockIdx.y;
+        const int ly = I < nyc, lx = J < nxc, lz = K < nzc, fpl = NYf * NXf;
+        const int f00 = 2 * I + NYf * 2 * J + fpl * 2 * K;
+        // everything that this thread reads, before anything waits for it
+        float r[8][3], dg[8][3];
+        uint8_t fl[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int f = f00 + ((k & 1) && ly ? 1 : 0) + ((k & 2) && lx ? NYf : 0) + ((k & 4) && lz ? fpl : 0);
+            fl[k] = nflag[f];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                r[k][q] = rf[3 * f + q];
+                dg[k][q] = D[3 * f + q];
+            }
+        }
+        float cr[M][8][3], v[3][8];
+#pragma unroll
+        for (int l = 0; l <= M; ++l) {
+            const int y = I >> l, x = J >> l, z = K >> l, NY = c.ny[l] + 1, NP = NY * (c.nx[l] + 1);
+            const int n = y + NY * x + NP * z;
+            const int oy = y < c.ny[l] ? 1 : 0, ox = x < c.nx[l] ? NY : 0, oz = z < c.nz[l] ? NP : 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int m = 3 * (n + (k & 1 ? oy : 0) + (k & 2 ? ox : 0) + (k & 4 ? oz : 0));
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    if (l == M)
+                        v[q][k] = c.x[m + q];
+                    else
+                        cr[l][k][q] = c.r[l][m + q] * c.D[l][m + q];
+                }
+            }
+        }
+#pragma unroll
+        for (int l = M - 1; l >= 0; --l)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                half_cell(v[q], 1, I >> l & 1);
+                half_cell(v[q], 2, J >> l & 1);
+                half_cell(v[q], 4, K >> l & 1);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[q][k] += cr[l][k][q];
+            }
+        // v: x of the next coarser level at the cell's corners (a corner that no active fine
+        // node depends on may hold anything finite)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (((k & 1) && !ly) || ((k & 2) && !lx) || ((k & 4) && !lz)) continue;
+            const int f = f00 + (k & 1) + (k & 2 ? NYf : 0) + (k & 4 ? fpl : 0);
+            const bool act = (fl[k] & NF_ACTIVE) != 0;
+            float o[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                float p = 0.f;
+#pragma unroll
+                for (int m = 0; m < 8; ++m)
+                    if ((m & ~k) == 0) p += v[q][m];
+                const float scale = 1.f / (float)((k & 1 ? 2 : 1) * (k & 2 ? 2 : 1) * (k & 4 ? 2 : 1));
+                o[q] = fmaf(scale, p, r[k][q] * dg[k][q]);
+                if (FINAL && (fl[k] & (NF_FIXX << q))) o[q] = 0.f;
+            }
+            if (act) {   // inactive nodes hold 0
+                if (FINAL) dot += o[0] * r[k][0] + o[1] * r[k][1] + o[2] * r[k][2];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) xf[3 * f + q] = o[q];
+            }
+        }
+    }
+    if (FINAL && partial) {
+        __shared__ double red[4];
+        const double sum = warp_block_sum<float>(dot, red);
+        if (threadIdx.x == 0) partial[blockIdx.x + gridDim.x * blockIdx.y] = sum;
+    }
+}
+
+// Nodes of the level that a chained launch starts from (restriction) or ends on
+// (prolongation), at most; past them the extra taps and corners cost more than launches:
+// the 192 x 96 x 96 blob shape's cycle takes 50 us chained from its second level (233,000 nodes),
+// 58 from the third, 71 from the finest (1.8 million).
+constexpr int64_t CHAIN_NODES = 300000;
+
+static bool dyadic_below(const std::vector<Level> &lv, int l) {
+    for (size_t k = l + 1; k < lv.size(); ++k)
+        if (lv[k].span != 2) return false;
+    return true;
+}
+
+// Residuals of the levels below level b from b's: returns how many levels it did (0: use launch_restrict)
+int launch_restrict_chain(const std::vector<Level> &lv, int b, const float *rf, cudaStream_t st) {
+    const int n = std::min(3, (int)lv.size() - 1 - b);
+    if (n < 2 || lv[b].nnode > CHAIN_NODES || !dyadic_below(lv, b)) return 0;
+    RestrictChain c;
+    c.n = n;
+    int ctas = 0;
+    for (int k = n - 1; k >= 0; --k) {
+        const Level &l = lv[b + 1 + k];
+        const int per = k == 0 ? 128 : k == 1 ? 4 : 1;
+        c.flag[k] = l.nflag;
+        c.out[k] = l.r32;
+        c.first[k] = ctas;
+        ctas += (int)((l.nnode + per - 1) / per);
+    }
+    for (int k = 0; k <= n; ++k) {
+        c.ny[k] = lv[b + k].ny;
+        c.nx[k] = lv[b + k].nx;
+        c.nz[k] = lv[b + k].nz;
+    }
+    ++g_launches;
+    k_restrict_chain<<<ctas, 128, 0, st>>>(rf, c);
+    return n;
+}
+
+template <int M>
+static void prolong_chain(const std::vector<Level> &lv, int f, const float *rf, float *xf, double *partial, dim3 g,
+                          cudaStream_t st) {
+    ProlongChain<M> c;
+    for (int k = 0; k <= M; ++k) {
+        const Level &l = lv[f + 1 + k];
+        c.ny[k] = l.ny;
+        c.nx[k] = l.nx;
+        c.nz[k] = l.nz;
+        if (k < M) {
+            c.r[k] = l.r32;
+            c.D[k] = l.idiag32;
+        } else {
+            c.x = l.x32;
+        }
+    }
+    if (f == 0)
+        k_prolong_chain<M, true><<<g, 128, 0, st>>>(c, rf, lv[f].idiag32, lv[f].nflag, xf, partial);
+    else
+        k_prolong_chain<M, false><<<g, 128, 0, st>>>(c, rf, lv[f].idiag32, lv[f].nflag, xf, nullptr);
+}
+
+// x of level f straight from the coarsest level's; false: go level by level
+bool launch_prolong_chain(const std::vector<Level> &lv, int f, const float *rf, float *xf, double *partial, int *nblocks,
+                          cudaStream_t st) {
+    const int M = (int)lv.size() - 2 - f;
+    if (M < 1 || M > 3 || lv[f].nnode > CHAIN_NODES || !dyadic_below(lv, f)) return false;
+    const Level &l = lv[f + 1];
+    const dim3 g((unsigned)(((l.ny + 1) * (l.nx + 1) + 127) / 128), (unsigned)(l.nz + 1));
+    if (f == 0 && nblocks) *nblocks = (int)(g.x * g.y);
+    ++g_launches;
+    if (M == 1)
+        prolong_chain<1>(lv, f, rf, xf, partial, g, st);
+    else if (M == 2)
+        prolong_chain<2>(lv, f, rf, xf, partial, g, st);
+    else
+        prolong_chain<3>(lv, f, rf, xf, partial, g, st);
+    return true;
+}
 
 // ---- Jacobi diagonals (src/Solving_AssembleFEAstencil.m:82-121) -------------
 // reference corner order j = 1..8 as offsets (dy, dx, dz)

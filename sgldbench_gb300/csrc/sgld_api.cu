@@ -358,12 +358,21 @@ int vcycle_dev32(sgld_ctx *ctx, const float *r, float *z, double *partial, int *
     if (!st) st = c.stream;
     const int L = c.L;
     const float *rf = r;
-    for (int l = 1; l < L; ++l) {
-        launch_restrict<float>(c.lv[l - 1], c.lv[l], rf, c.lv[l].r32, st);
+    for (int l = 0; l < L - 1;) {
+        int n = launch_restrict_chain(c.lv, l, rf, st);
+        if (n == 0) {
+            launch_restrict<float>(c.lv[l], c.lv[l + 1], rf, c.lv[l + 1].r32, st);
+            n = 1;
+        }
+        l += n;
         rf = c.lv[l].r32;
     }
     launch_coarse_apply_f32(c, c.lv[L - 1].r32, c.lv[L - 1].x32, st);
-    for (int l = L - 2; l >= 0; --l) {
+    // the finest level that is reached from the coarsest in one launch, then level by level
+    int top = L - 1;
+    for (int f = 0; f < L - 2 && top == L - 1; ++f)
+        if (launch_prolong_chain(c.lv, f, f == 0 ? r : c.lv[f].r32, f == 0 ? z : c.lv[f].x32, partial, nb, st)) top = f;
+    for (int l = top - 1; l >= 0; --l) {
         const float *rl = (l == 0) ? r : c.lv[l].r32;
         float *xl = (l == 0) ? z : c.lv[l].x32;
         launch_prolong_smooth<float>(c.lv[l], c.lv[l + 1], c.lv[l + 1].x32, rl, c.lv[l].idiag32, xl,

@@ -320,6 +320,12 @@ void launch_mma_eval(const double *xv, const double *xmin, const double *xmax, c
 
 template <typename T>
 void launch_restrict(const Level &fine, const Level &coarse, const T *rf, T *rc, cudaStream_t s);
+// the FP32 V-cycle's small levels: the residuals of up to three levels below level b at once
+// (the number done; 0: take launch_restrict), and level f's x straight from the coarsest's
+// (false: take launch_prolong_smooth)
+int launch_restrict_chain(const std::vector<Level> &lv, int b, const float *rf, cudaStream_t st);
+bool launch_prolong_chain(const std::vector<Level> &lv, int f, const float *rf, float *xf, double *partial, int *nblocks,
+                          cudaStream_t st);
 template <typename T>
 void launch_prolong_smooth(const Level &fine, const Level &coarse, const T *xc, const T *rf, const T *diag,
                            T *xf, bool final_level, double *partial_dot, int *nblocks_out,
