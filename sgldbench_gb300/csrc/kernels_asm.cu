@@ -865,23 +865,46 @@ int coarse_factor_invert(Ctx &c) {
 //   lower (UPPER = false): y_i = sum_{j <= i} M[i + n j] v[rows[j]]
 //   upper (UPPER = true):  x[rows[j]] = sum_{i >= j} M[j + n i] v[i]   (= (M' v)_j)
 // A cluster of CL_CTAS CTAs covers 32 output rows.  Their columns are dealt to the
-// cluster's 64 warps in blocks of 32, so the triangle's short and long rows
+// cluster's 32 warps in blocks of 32, so the triangle's short and long rows
 // load all of them alike; lane l holds row i0 + l, and the 32 loads of a block
 // (one coalesced row segment per column) are in flight together.  The warps' sums
 // meet in shared memory, the CTAs' sums in the first CTA's through distributed
 // shared memory, where they are added in a fixed order.  Chunk partials in global
 // memory cost two more launches and a memset of x per apply: the FP32 V-cycle of
 // 384 x 192 x 192 blobs (1300 rows) went from 214 to 193 us, of 256 x 128 x 128
-// (3888 rows) from 151 to 136, of 96 x 48 x 48 from 63 to 53.
-constexpr int CL_WARPS = 8, CL_CTAS = 8;
+// (3888 rows) from 151 to 136, of 96 x 48 x 48 from 63 to 53.  An apply of a few thousand rows
+// is a chain of latencies: 4 CTAs per cluster are better than 8 (96 x 48 x 48: 30 us a cycle
+// instead of 33.5; 256 x 128 x 128: 117 and 119) and than 2, or 1 to 4 of 16 or 32 warps (34 to 36).
+constexpr int CL_WARPS = 8, CL_CTAS = 4;
+
+// the warps' sums are added in FP64, or for FP32 in pairs of FP32 numbers: an FP64
+// operation holds a warp's scheduler for 64 clocks, and a chain of 16 conversions and adds
+// was a good part of an FP32 apply
+template <typename T>
+struct WideSum;
+template <>
+struct WideSum<double> {
+    double v;
+    __device__ __forceinline__ static WideSum of(double a) { return {a}; }
+    __device__ __forceinline__ WideSum operator+(WideSum b) const { return {v + b.v}; }
+    __device__ __forceinline__ double value() const { return v; }
+};
+template <>
+struct WideSum<float> {
+    df v;
+    __device__ __forceinline__ static WideSum of(float a) { return {{a, 0.f}}; }
+    __device__ __forceinline__ WideSum operator+(WideSum b) const { return {df_add(v, b.v)}; }
+    __device__ __forceinline__ float value() const { return v.hi; }
+};
 
 template <typename T, bool UPPER>
 __global__ void __cluster_dims__(1, CL_CTAS, 1) __launch_bounds__(32 * CL_WARPS)
     k_coarse_gemv(const T *__restrict__ M, const int *__restrict__ rows, const int *__restrict__ pos, int ndof,
                   const T *__restrict__ v, int n, T *__restrict__ y) {
     namespace cg = cooperative_groups;
+    using S = WideSum<T>;
     __shared__ T red[CL_WARPS][32];
-    __shared__ double sums[CL_CTAS][32];
+    __shared__ S sums[CL_CTAS][32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i0 = blockIdx.x * 32, i = i0 + lane, ii = min(i, n - 1);
     auto cluster = cg::this_cluster();
@@ -907,18 +930,15 @@ __global__ void __cluster_dims__(1, CL_CTAS, 1) __launch_bounds__(32 * CL_WARPS)
     __syncthreads();
     cluster.barrier_wait(std::move(started));
     if (w == 0) {
-        double sum = 0.0;
+        S t[CL_WARPS];
 #pragma unroll
-        for (int k = 0; k < CL_WARPS; ++k) sum += (double)red[k][lane];
-        cluster.map_shared_rank(&sums[0][0], 0)[32 * blockIdx.y + lane] = sum;
+        for (int k = 0; k < CL_WARPS; ++k) t[k] = S::of(red[k][lane]);
+        cluster.map_shared_rank(&sums[0][0], 0)[32 * blockIdx.y + lane] =
+            ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
     }
     cluster.sync();
-    if (blockIdx.y == 0 && w == 0 && i < n) {
-        double sum = 0.0;
-#pragma unroll
-        for (int k = 0; k < CL_CTAS; ++k) sum += sums[k][lane];
-        y[UPPER ? rows[i] : i] = (T)sum;
-    }
+    if (blockIdx.y == 0 && w == 0 && i < n)
+        y[UPPER ? rows[i] : i] = ((sums[0][lane] + sums[1][lane]) + (sums[2][lane] + sums[3][lane])).value();
     // x is zero off the free DOFs
     if (UPPER && blockIdx.x == 0 && blockIdx.y == 1)
         for (int d = threadIdx.x; d < ndof; d += 32 * CL_WARPS)

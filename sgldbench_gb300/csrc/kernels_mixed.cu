@@ -142,26 +142,43 @@ __device__ __forceinline__ float icg_coefficient(double *__restrict__ sc, const 
 // ||s|| > eta ||s_0||, eta = max(eta_min, tol / (2 relres)) with the outer
 // solve's tolerance and current relative residual (outer[15], outer[3]): the
 // inner solve of the last outer step only goes as far as the outer tolerance
-// needs.  eta_min <= 0: exactly kmax iterations.  Sets the condition of the
-// graph's while node.
-__global__ void k_icg_cond(cudaGraphConditionalHandle h, double *__restrict__ sc, const double *__restrict__ part,
-                           int nb, int kmax, double eta_min, const double *__restrict__ outer,
-                           double *__restrict__ total) {
-    const double ss = msum_partials(part, nb);
-    if (threadIdx.x != 0) return;
-    const double it = sc[IS_IT] + 1.0;
-    sc[IS_IT] = it;
-    *total += 1.0;
-    const double cap = eta_min > 0.0 ? sc[IS_KCAP] : (double)kmax;
-    bool more = it < cap;
+// needs.  eta_min <= 0: exactly kmax iterations.  For thread 0: whether to go on.
+// The threshold is formed beside the sum, by a thread of a warp that takes no part in it:
+// a launch of one CTA is all latency, and its FP64 division alone a good part of it.
+__device__ __forceinline__ bool icg_more(double *__restrict__ sc, const double *__restrict__ part, int nb, int kmax,
+                                         double eta_min, const double *__restrict__ outer, double *__restrict__ total) {
+    __shared__ double limit;
+    __shared__ int below;   // under the cap
+    if (threadIdx.x == 128) {
+        const double it = sc[IS_IT] + 1.0, cap = eta_min > 0.0 ? sc[IS_KCAP] : (double)kmax;
+        double l = 0.0;
+        if (eta_min > 0.0) {
+            const double relres = outer[3], tol = outer[15];
+            const double eta = (relres > 0.0) ? fmax(eta_min, 0.5 * tol / relres) : eta_min;
+            l = eta * eta * sc[IS_R0];
+        }
+        sc[IS_IT] = it;
+        *total += 1.0;
+        limit = l;
+        below = it < cap;
+    }
+    const double ss = usum_partials(part, nb);   // ends with a barrier
+    if (threadIdx.x != 0) return false;
+    bool more = below != 0;
     if (eta_min > 0.0) {
-        const double relres = outer[3], tol = outer[15];
-        const double eta = (relres > 0.0) ? fmax(eta_min, 0.5 * tol / relres) : eta_min;
-        const bool above = ss > eta * eta * sc[IS_R0];
+        const bool above = ss > limit;
         if (!more && above) sc[IS_CAPHIT] = 1.0;
         more = more && above;
     }
-    cudaGraphSetConditional(h, more ? 1u : 0u);
+    return more;
+}
+
+// sets the condition of the graph's while node
+__global__ void k_icg_cond(cudaGraphConditionalHandle h, double *__restrict__ sc, const double *__restrict__ part,
+                           int nb, int kmax, double eta_min, const double *__restrict__ outer,
+                           double *__restrict__ total) {
+    const bool more = icg_more(sc, part, nb, kmax, eta_min, outer, total);
+    if (threadIdx.x == 0) cudaGraphSetConditional(h, more ? 1u : 0u);
 }
 
 // sets a conditional handle: a handle's default value is applied when the
@@ -198,21 +215,8 @@ void launch_outer_cond(cudaGraphConditionalHandle hw, cudaGraphConditionalHandle
 __global__ void k_icg_cond_flag(int *flag, double *__restrict__ sc, const double *__restrict__ part, int nb,
                                 int kmax, double eta_min, const double *__restrict__ outer,
                                 double *__restrict__ total) {
-    const double ss = msum_partials(part, nb);
-    if (threadIdx.x != 0) return;
-    const double it = sc[IS_IT] + 1.0;
-    sc[IS_IT] = it;
-    *total += 1.0;
-    const double cap = eta_min > 0.0 ? sc[IS_KCAP] : (double)kmax;
-    bool more = it < cap;
-    if (eta_min > 0.0) {
-        const double relres = outer[3], tol = outer[15];
-        const double eta = (relres > 0.0) ? fmax(eta_min, 0.5 * tol / relres) : eta_min;
-        const bool above = ss > eta * eta * sc[IS_R0];
-        if (!more && above) sc[IS_CAPHIT] = 1.0;
-        more = more && above;
-    }
-    *flag = more ? 1 : 0;
+    const bool more = icg_more(sc, part, nb, kmax, eta_min, outer, total);
+    if (threadIdx.x == 0) *flag = more ? 1 : 0;
 }
 
 void launch_icg_cond_flag(int *flag, double *sc, const double *part, int nb, int kmax, double eta_min,
