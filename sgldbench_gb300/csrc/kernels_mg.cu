@@ -591,8 +591,9 @@ template void launch_prolong_smooth<float>(const Level &, const Level &, const f
 // ---- the FP32 V-cycle's small levels -----------------------------------------
 // A launch on a level of a few thousand nodes costs a memory latency and its place in
 // the chain of launches, about 4 us, whatever it computes.  The cycle is additive and
-// its levels are nested by factors of 2, so the chains collapse:
-//   * the product of span-2 restrictions is the tent of span 4, 8, so that up to three
+// its levels are nested by factors of 2 (4 below the finest of a non-dyadic hierarchy), so
+// the chains collapse:
+//   * the product of restrictions is the tent of span 4, 8, so that up to three
 //     coarser residuals are formed from one level's in one launch;
 //   * trilinear interpolation through the levels in between is trilinear interpolation
 //     on each level's own cell, so a thread that prolongates to 8 fine nodes carries
@@ -600,7 +601,7 @@ template void launch_prolong_smooth<float>(const Level &, const Level &, const f
 //     the way; the levels in between are not written at all.
 // The sums are those of the level-by-level launches in another order.  FP32 V-cycle, us:
 // 96 x 48 x 48 51 -> 37, 125 x 61 x 67 blob shape 55 -> 48, 192 x 96 x 96 65 -> 50, 384 x 192 x 192
-// 160 -> 140, 256 x 128 x 128 134 -> 123.
+// 160 -> 140, 256 x 128 x 128 134 -> 123; non-dyadic 64 x 32 x 32 33 -> 25.
 
 // S-fold restriction at coarse node (I, J, K) by 2 S NX threads: 2 S lanes along y (one
 // idle), NX groups along x, each of which takes 2 S / NX columns through z.  Taps are read at
@@ -637,10 +638,10 @@ __device__ __forceinline__ void restrict_chain_taps(const float *__restrict__ rf
     for (int c = 0; c < 3; ++c) a[c] *= 1.f / (float)(S * S * S);
 }
 
-// targets k = 0, 1, 2 lie 1, 2, 3 levels below the base; CTAs in the order 2, 1, 0 (the
-// longest sums first)
+// target k is the level 2, 4, 8 times coarser than the base (k = 0, 1, 2; a base whose next
+// level is 4 times coarser has no target 0); CTAs in the order 2, 1, 0 (the longest sums first)
 struct RestrictChain {
-    int n = 0;
+    int k0, k1;                        // the first and the last target
     int ny[4], nx[4], nz[4];           // [0] the base, [1 + k] target k
     const uint8_t *flag[3];
     float *out[3];
@@ -650,8 +651,8 @@ struct RestrictChain {
 __global__ void __launch_bounds__(128) k_restrict_chain(const float *__restrict__ rf,
                                                         const __grid_constant__ RestrictChain c) {
     const int b = blockIdx.x, lane = threadIdx.x & 31;
-    int k = 0;
-    while (k + 1 < c.n && b < c.first[k]) ++k;
+    int k = c.k0;
+    while (k < c.k1 && b < c.first[k]) ++k;
     const int per = k == 0 ? 128 : k == 1 ? 4 : 1;   // coarse nodes per CTA: a thread, a warp, a CTA for each
     const int i = (b - c.first[k]) * per + (k == 0 ? (int)threadIdx.x : k == 1 ? (int)(threadIdx.x >> 5) : 0);
     const int NY = c.ny[1 + k] + 1, NX = c.nx[1 + k] + 1;
@@ -708,6 +709,41 @@ __device__ __forceinline__ void half_cell(float (&v)[8], int step, int b) {
     }
 }
 
+// v: x of the next coarser level at the corners of its cell (I, J, K), component q, corner
+// k = y | x << 1 | z << 2; positions past the grid repeat the last node.  A corner that no
+// active fine node depends on may hold anything finite.
+template <int M>
+__device__ __forceinline__ void chain_corners(const ProlongChain<M> &c, int I, int J, int K, float (&v)[3][8]) {
+    float cr[M][8][3];
+#pragma unroll
+    for (int l = 0; l <= M; ++l) {
+        const int y = I >> l, x = J >> l, z = K >> l, NY = c.ny[l] + 1, NP = NY * (c.nx[l] + 1);
+        const int n = y + NY * x + NP * z;
+        const int oy = y < c.ny[l] ? 1 : 0, ox = x < c.nx[l] ? NY : 0, oz = z < c.nz[l] ? NP : 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int m = 3 * (n + (k & 1 ? oy : 0) + (k & 2 ? ox : 0) + (k & 4 ? oz : 0));
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                if (l == M)
+                    v[q][k] = c.x[m + q];
+                else
+                    cr[l][k][q] = c.r[l][m + q] * c.D[l][m + q];
+            }
+        }
+    }
+#pragma unroll
+    for (int l = M - 1; l >= 0; --l)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            half_cell(v[q], 1, I >> l & 1);
+            half_cell(v[q], 2, J >> l & 1);
+            half_cell(v[q], 4, K >> l & 1);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[q][k] += cr[l][k][q];
+        }
+}
+
 // x_f = r_f .* D + P x_c as k_prolong_cells, a thread per node of the next coarser level
 template <int M, bool FINAL>
 __global__ void __launch_bounds__(128) k_prolong_chain(const __grid_constant__ ProlongChain<M> c,
@@ -735,36 +771,8 @@ __global__ void __launch_bounds__(128) k_prolong_chain(const __grid_constant__ P
                 dg[k][q] = D[3 * f + q];
             }
         }
-        float cr[M][8][3], v[3][8];
-#pragma unroll
-        for (int l = 0; l <= M; ++l) {
-            const int y = I >> l, x = J >> l, z = K >> l, NY = c.ny[l] + 1, NP = NY * (c.nx[l] + 1);
-            const int n = y + NY * x + NP * z;
-            const int oy = y < c.ny[l] ? 1 : 0, ox = x < c.nx[l] ? NY : 0, oz = z < c.nz[l] ? NP : 0;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int m = 3 * (n + (k & 1 ? oy : 0) + (k & 2 ? ox : 0) + (k & 4 ? oz : 0));
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    if (l == M)
-                        v[q][k] = c.x[m + q];
-                    else
-                        cr[l][k][q] = c.r[l][m + q] * c.D[l][m + q];
-                }
-            }
-        }
-#pragma unroll
-        for (int l = M - 1; l >= 0; --l)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                half_cell(v[q], 1, I >> l & 1);
-                half_cell(v[q], 2, J >> l & 1);
-                half_cell(v[q], 4, K >> l & 1);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v[q][k] += cr[l][k][q];
-            }
-        // v: x of the next coarser level at the cell's corners (a corner that no active fine
-        // node depends on may hold anything finite)
+        float v[3][8];
+        chain_corners<M>(c, I, J, K, v);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             if (((k & 1) && !ly) || ((k & 2) && !lx) || ((k & 4) && !lz)) continue;
@@ -795,6 +803,63 @@ __global__ void __launch_bounds__(128) k_prolong_chain(const __grid_constant__ P
     }
 }
 
+// the same for a finest level 4 times finer than the next: threads as in k_prolong_rows4
+template <int M>
+__global__ void __launch_bounds__(128) k_prolong_chain4(const __grid_constant__ ProlongChain<M> c,
+                                                        const float *__restrict__ rf, const float *__restrict__ D,
+                                                        const uint8_t *__restrict__ nflag, float *__restrict__ xf,
+                                                        double *__restrict__ partial) {
+    constexpr int S = 4;
+    const int nyc = c.ny[0], NYc = nyc + 1, NYf = S * nyc + 1, NXf = S * c.nx[0] + 1;
+    const int pl = blockIdx.x * blockDim.x + threadIdx.x;
+    float dot = 0.f;
+    if (pl < NYc * NXf) {
+        const int I = pl % NYc, fx = pl / NYc, fz = blockIdx.y, rx = fx % S, rz = fz % S;
+        const int f0 = S * I + NYf * (fx + NXf * fz), ly = I < nyc ? S : 1;
+        uint8_t fl[S];
+        float r[S][3], dg[S][3];
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            const int f = f0 + (k < ly ? k : 0);
+            fl[k] = nflag[f];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                r[k][q] = rf[3 * f + q];
+                dg[k][q] = D[3 * f + q];
+            }
+        }
+        float v[3][8];
+        chain_corners<M>(c, I, fx / S, fz / S, v);
+        float qa[2][3] = {};
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+            const float w = (float)((k & 4 ? rz : S - rz) * (k & 2 ? rx : S - rx)) * (1.f / (S * S));
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                qa[0][q] = fmaf(w, v[q][k], qa[0][q]);
+                qa[1][q] = fmaf(w, v[q][k + 1], qa[1][q]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            if (k >= ly || !(fl[k] & NF_ACTIVE)) continue;   // inactive nodes hold 0
+            float o[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                o[q] = r[k][q] * dg[k][q] + ((float)(S - k) / S * qa[0][q] + (float)k / S * qa[1][q]);
+                if (fl[k] & (NF_FIXX << q)) o[q] = 0.f;
+                xf[3 * (f0 + k) + q] = o[q];
+            }
+            dot += o[0] * r[k][0] + o[1] * r[k][1] + o[2] * r[k][2];
+        }
+    }
+    if (partial) {
+        __shared__ double red[4];
+        const double sum = warp_block_sum<float>(dot, red);
+        if (threadIdx.x == 0) partial[blockIdx.x + gridDim.x * blockIdx.y] = sum;
+    }
+}
+
 // Nodes of the level that a chained launch starts from (restriction) or ends on
 // (prolongation), at most; past them the extra taps and corners cost more than launches:
 // the 192 x 96 x 96 blob shape's cycle takes 50 us chained from its second level (233,000 nodes),
@@ -809,27 +874,30 @@ static bool dyadic_below(const std::vector<Level> &lv, int l) {
 
 // Residuals of the levels below level b from b's: returns how many levels it did (0: use launch_restrict)
 int launch_restrict_chain(const std::vector<Level> &lv, int b, const float *rf, cudaStream_t st) {
-    const int n = std::min(3, (int)lv.size() - 1 - b);
-    if (n < 2 || lv[b].nnode > CHAIN_NODES || !dyadic_below(lv, b)) return 0;
+    const int L = (int)lv.size();
+    if (L - 1 - b < 2 || lv[b].nnode > CHAIN_NODES || !dyadic_below(lv, b + 1)) return 0;
     RestrictChain c;
-    c.n = n;
+    c.k0 = lv[b + 1].span == 2 ? 0 : 1;
+    if (lv[b + 1].span != 2 << c.k0) return 0;
+    c.k1 = std::min(2, c.k0 + L - 2 - b);
     int ctas = 0;
-    for (int k = n - 1; k >= 0; --k) {
-        const Level &l = lv[b + 1 + k];
+    for (int k = c.k1; k >= c.k0; --k) {
+        const Level &l = lv[b + 1 + k - c.k0];
         const int per = k == 0 ? 128 : k == 1 ? 4 : 1;
         c.flag[k] = l.nflag;
         c.out[k] = l.r32;
         c.first[k] = ctas;
         ctas += (int)((l.nnode + per - 1) / per);
+        c.ny[1 + k] = l.ny;
+        c.nx[1 + k] = l.nx;
+        c.nz[1 + k] = l.nz;
     }
-    for (int k = 0; k <= n; ++k) {
-        c.ny[k] = lv[b + k].ny;
-        c.nx[k] = lv[b + k].nx;
-        c.nz[k] = lv[b + k].nz;
-    }
+    c.ny[0] = lv[b].ny;
+    c.nx[0] = lv[b].nx;
+    c.nz[0] = lv[b].nz;
     ++g_launches;
     k_restrict_chain<<<ctas, 128, 0, st>>>(rf, c);
-    return n;
+    return c.k1 - c.k0 + 1;
 }
 
 template <int M>
@@ -848,7 +916,9 @@ static void prolong_chain(const std::vector<Level> &lv, int f, const float *rf, 
             c.x = l.x32;
         }
     }
-    if (f == 0)
+    if (lv[f + 1].span == 4)
+        k_prolong_chain4<M><<<g, 128, 0, st>>>(c, rf, lv[f].idiag32, lv[f].nflag, xf, partial);
+    else if (f == 0)
         k_prolong_chain<M, true><<<g, 128, 0, st>>>(c, rf, lv[f].idiag32, lv[f].nflag, xf, partial);
     else
         k_prolong_chain<M, false><<<g, 128, 0, st>>>(c, rf, lv[f].idiag32, lv[f].nflag, xf, nullptr);
@@ -858,9 +928,11 @@ static void prolong_chain(const std::vector<Level> &lv, int f, const float *rf, 
 bool launch_prolong_chain(const std::vector<Level> &lv, int f, const float *rf, float *xf, double *partial, int *nblocks,
                           cudaStream_t st) {
     const int M = (int)lv.size() - 2 - f;
-    if (M < 1 || M > 3 || lv[f].nnode > CHAIN_NODES || !dyadic_below(lv, f)) return false;
+    if (M < 1 || M > 3 || lv[f].nnode > CHAIN_NODES || !dyadic_below(lv, f + 1)) return false;
     const Level &l = lv[f + 1];
-    const dim3 g((unsigned)(((l.ny + 1) * (l.nx + 1) + 127) / 128), (unsigned)(l.nz + 1));
+    if (l.span != 2 && (l.span != 4 || f != 0)) return false;
+    const dim3 g = l.span == 4 ? dim3((unsigned)(((l.ny + 1) * (lv[f].nx + 1) + 127) / 128), (unsigned)(lv[f].nz + 1))
+                               : dim3((unsigned)(((l.ny + 1) * (l.nx + 1) + 127) / 128), (unsigned)(l.nz + 1));
     if (f == 0 && nblocks) *nblocks = (int)(g.x * g.y);
     ++g_launches;
     if (M == 1)

@@ -1216,7 +1216,9 @@ int sgld_set_modulus(sgld_ctx *ctx, const double *E) {
 // lv[0].kx_tx / kx_zc.  Runs once per context, at the first assembly (never
 // during a graph capture); SGLD_AUTOTUNE=0 keeps the default tile.  Width
 // and chunk trade halo work (one extra element column / layer per CTA)
-// against the number of CTAs in flight.
+// against the number of CTAs in flight: 3 node layers per stream are best on 64 x 32 x 32
+// (8.4 us, 8.9 with 4), 3 or 5 on 96 x 48 x 48 (10.3, 11.0 with 4 or 6), 10 on the 384 x 192 x 192
+// blob shape (99, 101 with 8).
 static int tune_kbyu_f32(sgld_ctx *ctx) {
     Ctx &c = ctx->c;
     Level &l0 = c.lv[0];
@@ -1229,7 +1231,7 @@ static int tune_kbyu_f32(sgld_ctx *ctx) {
     }
     const int NZ = l0.nz + 1;
     std::vector<int> cand;
-    for (int zc : {4, 6, 8, 12, 16, 24})   // node layers per stream, two streams per CTA
+    for (int zc : {3, 4, 5, 6, 8, 10, 12, 16, 24})   // node layers per stream, two streams per CTA
         if (2 * zc <= NZ + 1) cand.push_back(zc);
     cand.push_back(0);   // the default rule
     CK(cudaMemsetAsync(c.d_r32, 0, sizeof(float) * 3 * (size_t)l0.nnode, c.stream));

@@ -39,3 +39,27 @@ def test_vcycle_fp32_chained_levels(built_lib, shape, levels, fill):
     # scratch vectors keep zeros at inactive nodes from one cycle to the next
     assert np.array_equal(z, s.Solving_Vcycle(r, "mixed"))
     s.close()
+
+
+@pytest.mark.parametrize("shape,levels,fill", [((8, 40, 24), 4, 1.0), ((16, 48, 32), 5, 0.6), ((32, 64, 32), 6, 1.0)])
+def test_vcycle_fp32_chained_levels_non_dyadic(built_lib, shape, levels, fill):
+    """The first level 4 times coarser: one to three levels below it."""
+    from sgldbench_gb300 import VoxelSolver
+
+    rng = np.random.default_rng(sum(shape) + levels)
+    vox = rng.random(shape) < fill
+    vox[:, 0, :] = True
+    m = G.build_model(vox, non_dyadic=1, omega=0.6, num_levels=levels)
+    s = VoxelSolver(vox, num_levels=levels, non_dyadic=1, omega=0.6, pad=False)
+    E = rng.uniform(0.05, 1.0, s.numElements)
+    G.set_modulus(m, E)
+    s.set_fixed_dofs(m.levels[0].fixedDOFs)
+    s.set_modulus(E)
+    G.assemble_stencil(m)
+    s.Solving_AssembleFEAstencil()
+    r = rng.standard_normal(m.levels[0].numDOFs)
+    r[m.levels[0].fixedDOFs] = 0.0
+    z = s.Solving_Vcycle(r, "mixed")
+    assert _rel(z, G.vcycle(m, r)) <= 1e-4
+    assert np.array_equal(z, s.Solving_Vcycle(r, "mixed"))
+    s.close()
