@@ -1,6 +1,6 @@
 // Element-stencil kernels on the finest level: the FP32 matrix-free K*u, unit
-// compliance and the stress recovery of the solution.  (FP64 K*u:
-// kernels_kbyu64.cu; double-float K*u: kernels_df.cu.)
+// compliance and the stress recovery of the solution.  (FP64 and double-float K*u:
+// kernels_kbyu64.cu.)
 //
 // The element product uses the 8-corner Hadamard basis in which the
 // isotropic hexahedral Ke has 45 nonzeros (instead of 576).
@@ -173,8 +173,7 @@ __device__ __forceinline__ T block_sum(T v, T *red) {
     return s;
 }
 
-constexpr int KT_Y = 32, KT_X = 8;
-constexpr int KT_ZC = 16;                        // node layers per CTA
+constexpr int KT_Y = 32;
 
 // Active-tile map of a z-marching K*u grid g whose CTAs own (TY-1) x (TX-1)
 // node columns and zc node layers: a CTA is active iff an element of its box
@@ -626,10 +625,6 @@ static dim3 kbyu_f32_grid(const Level &l) {
     return dim3((l.ny + 1 + KT_Y - 2) / (KT_Y - 1), (l.nx + 1 + tx - 2) / (tx - 1), (NZ + zl - 1) / zl);
 }
 
-static dim3 kbyu_grid(const Level &l) {
-    return dim3((l.ny + 1 + KT_Y - 2) / (KT_Y - 1), (l.nx + 1 + KT_X - 2) / (KT_X - 1), (l.nz + 1 + KT_ZC - 1) / KT_ZC);
-}
-
 template <int TX, bool DOT, bool CUBIC>
 static void tma_attributes() {
     cudaFuncSetAttribute(k_kbyu_tma<TX, DOT, CUBIC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -722,12 +717,6 @@ int launch_kbyu_f32(const Level &l0, const float *E, const float *u, float *y, d
 
 int update_kbyu_tiles(Level &l0, cudaStream_t s) {
     cudaError_t e = cudaSuccess;
-    const dim3 g16 = kbyu_grid(l0);
-    if (!l0.tiles16) {
-        e = cudaMalloc((void **)&l0.tiles16, (size_t)g16.x * g16.y * g16.z);
-        if (e != cudaSuccess) return (int)e;
-        make_tile_map(l0, KT_Y, KT_X, KT_ZC, g16, l0.tiles16, s);
-    }
     if (!l0.tiles64) {
         const dim3 g = kbyu64_grid(l0);
         e = cudaMalloc((void **)&l0.tiles64, (size_t)g.x * g.y * g.z);

@@ -763,7 +763,6 @@ int bind_ctx(sgld_ctx *ctx) {
     if (g_kh_valid[c.device] && !same) CK(cudaDeviceSynchronize());
     g_kh_valid[c.device] = false;
     upload_kh(c.Kh, c.stream);
-    upload_kh_df(c.Kh, c.stream);
     CK(cudaStreamSynchronize(c.stream));
     memcpy(g_kh_held[c.device], c.Kh, sizeof c.Kh);
     g_kh_valid[c.device] = true;
@@ -948,7 +947,6 @@ int sgld_create(int resY, int resX, int resZ, const uint8_t *solid, const sgld_o
     CK(cudaMemset(c.d_t32, 0, sizeof(float) * nv));
     CK(dalloc(&c.d_isc, 16));
     init_kernel_attributes();
-    init_kbyu_df_attributes();
     kbyu64_pick_tile(c.lv[0]);
     const dim3 g64 = kbyu64_grid(l0);
     // partial-sum slots: the largest grid of any kernel that writes per-CTA partials
@@ -975,7 +973,7 @@ void sgld_destroy(sgld_ctx *ctx) {
         cudaSetDevice(c.device);
     for (Level &l : c.lv) {
         for (void *p : {(void *)l.eact, (void *)l.nflag, (void *)l.diag, (void *)l.idiag, (void *)l.idiag32, (void *)l.Ks, (void *)l.r,
-                        (void *)l.x, (void *)l.r32, (void *)l.x32, (void *)l.tiles64, (void *)l.tiles16, (void *)l.tiles_f32,
+                        (void *)l.x, (void *)l.r32, (void *)l.x32, (void *)l.tiles64, (void *)l.tiles_f32,
                         (void *)l.runs, (void *)l.kerr})
             if (p) cudaFree(p);
     }

@@ -52,10 +52,9 @@ struct Level {
     uint8_t *eact = nullptr;      // [nel] element non-empty
     // active-tile maps of the finest level's K*u launches (one byte per CTA:
     // 0 = no active element in the CTA's element box, so every node it owns
-    // is inactive and its result is zero): the FP64 kernel's grid, the 32 x 8 x
-    // 16-layer grid of the double-float kernel, and the FP32 kernel's grid for
-    // the tile (tiles_f32_tx, tiles_f32_zc) it was made for
-    uint8_t *tiles64 = nullptr, *tiles16 = nullptr, *tiles_f32 = nullptr;
+    // is inactive and its result is zero): the grid of the FP64 and double-float kernel, and
+    // the FP32 kernel's grid for the tile (tiles_f32_tx, tiles_f32_zc) it was made for
+    uint8_t *tiles64 = nullptr, *tiles_f32 = nullptr;
     // finest level: the words of the active nodes as chunks of contiguous
     // floats (runs of active nodes along y, gaps of a few nodes bridged), each
     // first DOF | floats << 40, in address order; empty when nearly every node
@@ -202,9 +201,7 @@ void init_kernel_attributes();
 int kbyu_f32_zc(const Level &l0);   // node layers per CTA the FP32 K*u uses on this level
 int kbyu_f32_tx(const Level &l0);   // x width (elements) of the FP32 K*u tile on this level
 int kbyu_f32_cta_layers(const Level &l0);   // node layers one CTA of the FP32 K*u covers
-// double-float K*u (kernels_df.cu)
-void upload_kh_df(const double *Kh, cudaStream_t s);
-void init_kbyu_df_attributes();
+// the same in double-float arithmetic (kernels_kbyu64.cu)
 void launch_kbyu_df(const Level &l0, const double *E, const double *u, double *y, double *partial_dot,
                     int *nblocks_out, cudaStream_t s);
 // mixed-precision solve (kernels_mixed.cu)
