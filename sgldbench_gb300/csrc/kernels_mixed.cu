@@ -41,39 +41,9 @@ __device__ double msum_partials(const double *__restrict__ part, int nb) {
     return mblock_reduce((s0 + s1) + (s2 + s3));
 }
 
-// The vector updates of the inner CG sum up to ICG_FUSE_PARTS partials themselves, every
-// CTA for itself (the same sum in the same order, so the same value): alpha and beta
-// then cost no launch of their own.  An FP64 instruction holds an SM's scheduler for 64
-// clocks, so the sum is spread over one warp per scheduler and the updates run as few
-// large CTAs.  (Summed by 8 CTAs of 8 warps per SM, all warps taking part, the mixed
-// solve on 64 x 32 x 32 went from 5.67 to 6.47 ms; with this form to 5.25.)  Past
-// ICG_FUSE_PARTS k_icg_scalar's launch is the cheaper one: 192 x 96 x 96 blob shape, 1862
-// partials of z.s, load study 56.5 ms with them summed by the update, 50.8 by the launch.
+// The vector updates of the inner CG sum up to FUSE_PARTS partials themselves (usum_partials).
 constexpr int UB = 512;   // threads of an update
 constexpr int UGRID = 152 * 2;
-constexpr int ICG_FUSE_PARTS = 1024;
-
-// the sum for thread 0
-__device__ __forceinline__ double usum_partials(const double *__restrict__ part, int nb) {
-    __shared__ double red[4];
-    const int i0 = threadIdx.x, w = i0 >> 5;
-    if (i0 < 128) {
-        double s0 = 0.0, s1 = 0.0;
-        int i = i0;
-#pragma unroll 4
-        for (; i + 128 < nb; i += 256) {
-            s0 += part[i];
-            s1 += part[i + 128];
-        }
-        if (i < nb) s0 += part[i];
-        s0 += s1;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_down_sync(0xffffffffu, s0, o);
-        if ((i0 & 31) == 0) red[w] = s0;
-    }
-    __syncthreads();
-    return i0 == 0 ? (red[0] + red[1]) + (red[2] + red[3]) : 0.0;
-}
 
 // inner scalars (FP64 storage): rho = z.s of the last iteration, alpha, beta,
 // r0 = s.s at entry, the iteration count of this inner solve, the current
@@ -502,7 +472,7 @@ static int update_blocks(int64_t n) {
 
 // the scalar of an update from nb partials: by the update itself, or by a launch before it
 static int icg_sum(int op, double *sc, const double *sum, int nb, cudaStream_t st) {
-    if (nb <= ICG_FUSE_PARTS) return nb;
+    if (nb <= FUSE_PARTS) return nb;
     launch_icg_scalar(op, sc, sum, nb, st, 0, 0);
     return 0;
 }

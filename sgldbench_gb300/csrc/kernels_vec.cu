@@ -58,11 +58,12 @@ void launch_finalize_sum(const double *partial, int nb, double *out, cudaStream_
 }
 
 // scalar slots
-enum { S_NORMB = 0, S_X1 = 1, S_LAM = 2, S_RES = 3, S_BETA = 4, S_PQ = 5, S_RR = 6, S_TOL = 15 };
+enum { S_NORMB = 0, S_X1 = 1, S_LAM = 2, S_RES = 3, S_BETA = 4, S_PQ = 5, S_RR = 6, S_ZR = 8, S_TOL = 15 };
 enum { I_ITS = 0, I_DONE = 1, I_STOP = 2 };
 
 // op: 0 normB = sqrt(sum); 1 x1 = sum; 2 lambda = x1 / sum;
-//     3 residual test; 4 beta = sum / x1, x1 = sum; 5 reset iteration state
+//     3 residual test; 4 beta = sum / x1, x1 = sum; 5 reset iteration state;
+//     6 x1 = zr, lambda = x1 / sum (zr: z.r as op 1, op 4 or k_pcg_pupdate_sum left it)
 __global__ void k_pcg_scalar(int op, double *__restrict__ scal, int *__restrict__ iflag,
                              const double *__restrict__ part, int nb, double tol, int maxit) {
     double s = 0.0;
@@ -73,7 +74,16 @@ __global__ void k_pcg_scalar(int op, double *__restrict__ scal, int *__restrict_
             scal[S_NORMB] = sqrt(s);
             scal[S_TOL] = tol;
             break;
-        case 1: scal[S_X1] = s; break;
+        case 1:
+            scal[S_X1] = s;
+            scal[S_ZR] = s;
+            break;
+        case 6:
+            if (iflag[I_STOP]) return;
+            scal[S_X1] = scal[S_ZR];
+            scal[S_PQ] = s;
+            scal[S_LAM] = scal[S_ZR] / s;
+            break;
         case 2:
             if (iflag[I_STOP]) return;
             scal[S_PQ] = s;
@@ -98,6 +108,7 @@ __global__ void k_pcg_scalar(int op, double *__restrict__ scal, int *__restrict_
             if (iflag[I_STOP]) return;
             scal[S_BETA] = s / scal[S_X1];
             scal[S_X1] = s;
+            scal[S_ZR] = s;
             break;
         case 5:
             iflag[I_ITS] = 0;
@@ -149,6 +160,120 @@ __global__ void k_pcg_pupdate(double *__restrict__ p, const double *__restrict__
 void launch_pcg_pupdate(double *p, const double *z, int64_t n, const double *scal, const int *iflag, cudaStream_t s) {
     ++g_launches;
     k_pcg_pupdate<<<reduce_blocks(n), VB, 0, s>>>(p, z, n, scal, iflag);
+}
+
+// The two updates with lambda and beta from partials: z.r goes to S_ZR with beta and to S_X1
+// with lambda, so that no launch writes a scalar that another of its CTAs may still have to
+// read.  A thread's first words are on their way while its CTA sums.
+constexpr int UB = 512, UGRID = 152 * 4;
+static int update_blocks(int64_t n) {
+    const int64_t b = (n + UB - 1) / UB;
+    return (int)(b < UGRID ? (b > 0 ? b : 1) : UGRID);
+}
+
+__global__ void __launch_bounds__(UB, 4) k_pcg_update_sum(double *__restrict__ x, double *__restrict__ r,
+                                                          const double *__restrict__ p, const double *__restrict__ q,
+                                                          int64_t n, double *__restrict__ scal,
+                                                          const int *__restrict__ iflag, const double *__restrict__ sum,
+                                                          int nsum, double *__restrict__ part) {
+    const int64_t i0 = blockIdx.x * (int64_t)UB + threadIdx.x, stride = (int64_t)gridDim.x * UB;
+    const int stop = iflag[I_STOP];
+    const double zr = scal[S_ZR];
+    double xv = 0.0, pv = 0.0, rv = 0.0, qv = 0.0;
+    if (i0 < n) {
+        xv = x[i0];
+        pv = p[i0];
+        rv = r[i0];
+        qv = q[i0];
+    }
+    __shared__ double coef, red[UB / 32];
+    const double pq = usum_partials(sum, nsum);
+    if (stop) return;
+    if (threadIdx.x == 0) {
+        coef = zr / pq;
+        if (blockIdx.x == 0) {
+            scal[S_PQ] = pq;
+            scal[S_LAM] = coef;
+            scal[S_X1] = zr;
+        }
+    }
+    __syncthreads();
+    const double lam = coef;
+    double s = 0.0;
+    if (i0 < n) {
+        x[i0] = xv + lam * pv;
+        const double ri = rv - lam * qv;
+        r[i0] = ri;
+        s = ri * ri;
+    }
+    for (int64_t i = i0 + stride; i < n; i += stride) {
+        x[i] = x[i] + lam * p[i];
+        const double ri = r[i] - lam * q[i];
+        r[i] = ri;
+        s += ri * ri;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < UB / 32; ++i) t[i & 3] += red[i];
+        part[blockIdx.x] = (t[0] + t[1]) + (t[2] + t[3]);
+    }
+}
+
+__global__ void __launch_bounds__(UB, 4) k_pcg_pupdate_sum(double *__restrict__ p, const double *__restrict__ z, int64_t n,
+                                                           double *__restrict__ scal, const int *__restrict__ iflag,
+                                                           const double *__restrict__ sum, int nsum) {
+    const int64_t i0 = blockIdx.x * (int64_t)UB + threadIdx.x, stride = (int64_t)gridDim.x * UB;
+    const int stop = iflag[I_STOP];
+    const double x1 = scal[S_X1];
+    double pv = 0.0, zv = 0.0;
+    if (i0 < n) {
+        pv = p[i0];
+        zv = z[i0];
+    }
+    __shared__ double coef;
+    const double zr = usum_partials(sum, nsum);
+    if (stop) return;
+    if (threadIdx.x == 0) {
+        coef = zr / x1;
+        if (blockIdx.x == 0) {
+            scal[S_BETA] = coef;
+            scal[S_ZR] = zr;
+        }
+    }
+    __syncthreads();
+    const double beta = coef;
+    if (i0 < n) p[i0] = zv + beta * pv;
+    for (int64_t i = i0 + stride; i < n; i += stride) p[i] = z[i] + beta * p[i];
+}
+
+int launch_pcg_update_sum(double *x, double *r, const double *p, const double *q, int64_t n, double *scal, int *iflag,
+                          const double *sum, int nb, double *partial, cudaStream_t s) {
+    int g = reduce_blocks(n);
+    if (nb <= FUSE_PARTS) {
+        g = update_blocks(n);
+        ++g_launches;
+        k_pcg_update_sum<<<g, UB, 0, s>>>(x, r, p, q, n, scal, iflag, sum, nb, partial);
+    } else {
+        launch_pcg_scalar(6, scal, iflag, sum, nb, 0.0, 0, s);
+        launch_pcg_update(x, r, p, q, n, scal, iflag, partial, g, s);
+    }
+    return g;
+}
+
+void launch_pcg_pupdate_sum(double *p, const double *z, int64_t n, double *scal, int *iflag, const double *sum, int nb,
+                            cudaStream_t s) {
+    if (nb <= FUSE_PARTS) {
+        ++g_launches;
+        k_pcg_pupdate_sum<<<update_blocks(n), UB, 0, s>>>(p, z, n, scal, iflag, sum, nb);
+    } else {
+        launch_pcg_scalar(4, scal, iflag, sum, nb, 0.0, 0, s);
+        launch_pcg_pupdate(p, z, n, scal, iflag, s);
+    }
 }
 
 // r = b - Ax

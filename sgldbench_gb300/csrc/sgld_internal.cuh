@@ -349,11 +349,50 @@ void launch_coarse_apply_f64(const Ctx &c, const double *rc, double *xc, cudaStr
 void launch_coarse_apply_f32(const Ctx &c, const float *rc, float *xc, cudaStream_t s);
 
 // vector ops (FP64 PCG)
+// A CG's vector updates sum up to FUSE_PARTS partials themselves, every CTA for itself
+// (the same sum in the same order, so the same value): alpha and beta then cost no
+// launch of their own.  An FP64 instruction holds an SM's scheduler for 64 clocks, so the
+// sum is spread over one warp per scheduler and the updates run as few large CTAs.
+// (Summed by 8 CTAs of 8 warps per SM, all warps taking part, the mixed solve on 64 x 32 x
+// 32 went from 5.67 to 6.47 ms; with this form to 5.25.)  Past FUSE_PARTS a launch for the
+// scalar is the cheaper one: 192 x 96 x 96 blob shape, 1862 partials of z.s, load study
+// 56.5 ms with them summed by the update, 50.8 by a launch.
+constexpr int FUSE_PARTS = 1024;
+
+// the sum for thread 0 of a CTA of at least 128 threads; ends with a barrier
+__device__ __forceinline__ double usum_partials(const double *__restrict__ part, int nb) {
+    __shared__ double red[4];
+    const int i0 = threadIdx.x, w = i0 >> 5;
+    if (i0 < 128) {
+        double s0 = 0.0, s1 = 0.0;
+        int i = i0;
+#pragma unroll 4
+        for (; i + 128 < nb; i += 256) {
+            s0 += part[i];
+            s1 += part[i + 128];
+        }
+        if (i < nb) s0 += part[i];
+        s0 += s1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_down_sync(0xffffffffu, s0, o);
+        if ((i0 & 31) == 0) red[w] = s0;
+    }
+    __syncthreads();
+    return i0 == 0 ? (red[0] + red[1]) + (red[2] + red[3]) : 0.0;
+}
+
 int reduce_blocks(int64_t n);
 void launch_dot(const double *a, const double *b, int64_t n, double *partial, int nb, cudaStream_t s);
 void launch_finalize_sum(const double *partial, int nb, double *out, cudaStream_t s);
 void launch_pcg_update(double *x, double *r, const double *p, const double *q, int64_t n, const double *scal,
                        int *iflag, double *partial, int nb, cudaStream_t s);
+// the same updates with their scalar from the nb partials of p.q and of z.r (lambda and beta
+// without a launch of their own up to FUSE_PARTS); not in the area of update's own partials.
+// Returns the number of those.
+int launch_pcg_update_sum(double *x, double *r, const double *p, const double *q, int64_t n, double *scal, int *iflag,
+                          const double *sum, int nb, double *partial, cudaStream_t s);
+void launch_pcg_pupdate_sum(double *p, const double *z, int64_t n, double *scal, int *iflag, const double *sum, int nb,
+                            cudaStream_t s);
 void launch_pcg_pupdate(double *p, const double *z, int64_t n, const double *scal, const int *iflag,
                         cudaStream_t s);
 void launch_residual(double *r, const double *b, const double *Ax, int64_t n, cudaStream_t s);
