@@ -331,14 +331,16 @@ __device__ __forceinline__ df df_rcp(df d) {
 //     taken for all columns at once afterwards.  (With the tile in shared memory, a
 //     square root in the chain, branches around the updates and two barriers a step
 //     the launch took 30 us; now 15);
-//   * CTA 0 writes the factored tile back;
+//   * CTA 0 writes the factored tile back, unless other CTAs of the launch still have to
+//     read the tile as it was (they may start late, beside another stream's work): then it
+//     goes to `diag`, and the trailing update's launch puts it in its place;
 //   * CTA b > 0 solves CP_RS rows of the band below against it (X = A L^-T):
 //     16 lanes per row, two columns per lane in registers, x_q broadcast by a
 //     16-wide shuffle.
 constexpr int CP_THREADS = 128;
 constexpr int CP_RS = 8;
 
-__global__ void __launch_bounds__(CP_THREADS) k_chol_panel(double *A, int n, int k0, int rend, int *info) {
+__global__ void __launch_bounds__(CP_THREADS) k_chol_panel(double *A, int n, int k0, int rend, double *diag, int *info) {
     __shared__ float2 T[NB][NB + 1];     // the factor
     __shared__ float2 rd[NB], ld[NB];    // 1 / L[j][j], L[j][j]
     const int t = threadIdx.x, r = t & 31, w = t >> 5;
@@ -400,9 +402,11 @@ __global__ void __launch_bounds__(CP_THREADS) k_chol_panel(double *A, int n, int
     if (blockIdx.x == 0) {
         for (int idx = t; idx < NB * NB; idx += CP_THREADS) {
             const int rr = idx & 31, cc = idx >> 5;
-            if (rr < m && cc < m)
-                A[(int64_t)(k0 + rr) + (int64_t)n * (k0 + cc)] =
-                    rr > cc ? df_to(get(T[rr][cc])) : (rr == cc ? df_to(get(ld[rr])) : 0.0);
+            const double v = rr > cc ? df_to(get(T[rr][cc])) : (rr == cc ? df_to(get(ld[rr])) : 0.0);
+            if (gridDim.x > 1)
+                diag[idx] = v;
+            else if (rr < m && cc < m)
+                A[(int64_t)(k0 + rr) + (int64_t)n * (k0 + cc)] = v;
         }
         return;
     }
@@ -435,7 +439,11 @@ __global__ void __launch_bounds__(CP_THREADS) k_chol_panel(double *A, int n, int
 // products are summed in double-float; A stays FP64.
 constexpr int SY_RS = 8;
 
-__global__ void __launch_bounds__(256) k_syrk_update(double *A, int n, int k0, int jb0, int nbt) {
+__global__ void __launch_bounds__(256) k_syrk_update(double *A, int n, int k0, int jb0, int nbt,
+                                                     const double *__restrict__ diag) {
+    if (blockIdx.x == 0 && blockIdx.y == 0)   // the panel's diagonal tile, which this launch does not read
+        for (int idx = threadIdx.x; idx < NB * NB; idx += 256)
+            A[(int64_t)(k0 + (idx & 31)) + (int64_t)n * (k0 + (idx >> 5))] = diag[idx];
     int p = blockIdx.x, ii = 0;
     while (p > ii) {
         p -= ii + 1;
@@ -767,11 +775,11 @@ static void factor_enqueue(Ctx &c, int *d_info) {
         const int rend = min(n, (kend + 1) * NB);
         const int ntrsm = rend > k0 + NB ? (rend - k0 - NB + CP_RS - 1) / CP_RS : 0;
         ++g_launches;
-        k_chol_panel<<<1 + ntrsm, CP_THREADS, 0, c.stream>>>(A, n, k0, rend, d_info);
+        k_chol_panel<<<1 + ntrsm, CP_THREADS, 0, c.stream>>>(A, n, k0, rend, c.d_LB, d_info);   // d_LB: scratch until the factor is done
         if (nbelow > 0) {
             const int npairs = nbelow * (nbelow + 1) / 2;
             ++g_launches;
-            k_syrk_update<<<dim3(npairs, NB / SY_RS), 256, 0, c.stream>>>(A, n, k0, kb + 1, nbelow);
+            k_syrk_update<<<dim3(npairs, NB / SY_RS), 256, 0, c.stream>>>(A, n, k0, kb + 1, nbelow, c.d_LB);
         }
     }
     const int b = c.cband;
