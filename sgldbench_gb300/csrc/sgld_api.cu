@@ -950,10 +950,11 @@ int sgld_create(int resY, int resX, int resZ, const uint8_t *solid, const sgld_o
     kbyu64_pick_tile(c.lv[0]);
     const dim3 g64 = kbyu64_grid(l0);
     // partial-sum slots: the largest grid of any kernel that writes per-CTA partials
-    // (prolongation: ceil(NY*NX/256) CTAs per node plane)
+    // (prolongation: ceil(NY*NX/256) CTAs per node plane; FP32 K*u: its smallest tile)
     c.npart = (int)std::max<int64_t>({(int64_t)152 * 8, (l0.nel + 255) / 256 + 1, (int64_t)g64.x * g64.y * g64.z,
                                       (int64_t)(((l0.ny + 1) * (l0.nx + 1) + 255) / 256) * (l0.nz + 1),
-                                      (int64_t)((l0.ny + 31) / 31 + 1) * ((l0.nx + 7) / 7 + 1) * ((l0.nz + 16) / 16 + 1)});
+                                      (int64_t)((l0.ny + 31) / 31 + 1) * ((l0.nx + 7) / 7 + 1) *
+                                          ((l0.nz + 2 * KX_ZC_MIN) / (2 * KX_ZC_MIN) + 1)});
     CK(dalloc(&c.d_part, c.npart));
     CK(dalloc(&c.d_part2, c.npart + 152 * 8));   // and the partials of the inner CG's update
     CK(dalloc(&c.d_scal, 64));
@@ -1229,7 +1230,7 @@ static int tune_kbyu_f32(sgld_ctx *ctx) {
     }
     const int NZ = l0.nz + 1;
     std::vector<int> cand;
-    for (int zc : {3, 4, 5, 6, 8, 10, 12, 16, 24})   // node layers per stream, two streams per CTA
+    for (int zc : {KX_ZC_MIN, 4, 5, 6, 8, 10, 12, 16, 24})   // node layers per stream, two streams per CTA
         if (2 * zc <= NZ + 1) cand.push_back(zc);
     cand.push_back(0);   // the default rule
     CK(cudaMemsetAsync(c.d_r32, 0, sizeof(float) * 3 * (size_t)l0.nnode, c.stream));

@@ -37,6 +37,10 @@ enum : uint8_t { NF_ACTIVE = 1, NF_FIXX = 2, NF_FIXY = 4, NF_FIXZ = 8 };
 // sit in constant memory in the same order (row-major within each block).
 constexpr int KH_NNZ = 45;
 
+// node layers per z stream of the FP32 K*u, the fewest that its tuner tries (a CTA covers two
+// streams); the partial-sum slots of a context are counted for it
+constexpr int KX_ZC_MIN = 3;
+
 struct Level {
     int nx = 0, ny = 0, nz = 0;   // elements
     int span = 1;                 // coarsening factor from the next finer level
