@@ -251,6 +251,19 @@ int fail(sgld_ctx *ctx, int code, const std::string &msg) {
         if (e_ != cudaSuccess) return fail(ctx, SGLD_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e_)); \
     } while (0)
 
+// an event that goes with its scope, whichever way that is left
+struct ScopedEvent {
+    cudaEvent_t e = nullptr;
+    cudaError_t make(unsigned flags = cudaEventDefault) { return cudaEventCreateWithFlags(&e, flags); }
+    operator cudaEvent_t() const { return e; }
+    ScopedEvent() = default;
+    ScopedEvent(const ScopedEvent &) = delete;
+    ScopedEvent &operator=(const ScopedEvent &) = delete;
+    ~ScopedEvent() {
+        if (e) cudaEventDestroy(e);
+    }
+};
+
 // The finest level's active runs (Level::runs): the y-runs of every brick of
 // 32 (y) x 8 (x) x 8 (z) nodes that holds an active node, in address order.
 // Left empty when more than 85 % of the bricks are active (a solid box),
@@ -579,6 +592,7 @@ int download_nodes(sgld_ctx *ctx, const double *d_full, double *h) {
 // GB300 host a copy into memory that no CPU has touched yet (a fresh numpy array) takes its page
 // faults from the GPU's side: the first
 // stress recovery of a 192 x 96 x 96 blob model (35 MB) took 23 ms, with the touch 1.7 ms.
+// The buffer may overlap the call's input, so only once the input's copy has landed.
 void touch_pages(void *p, size_t bytes) {
     volatile char *c = static_cast<volatile char *>(p);
     static const size_t page = (size_t)std::max(sysconf(_SC_PAGESIZE), 4096l);
@@ -1630,7 +1644,10 @@ int sgld_stress(sgld_ctx *ctx, const double *U, double *nodal, double *vmn, doub
         CK(dalloc(&ctx->d_vmn, (size_t)l0.nnode));
         CK(dalloc(&ctx->d_vme, (size_t)l0.nel));
     }
+    ScopedEvent uploaded;
+    CK(uploaded.make(cudaEventDisableTiming));
     if ((rc = upload_nodes(ctx, U, c.d_z))) return rc;
+    CK(cudaEventRecord(uploaded, c.stream));
     double M[48 * 24];
     stress_matrix(c.nu, c.cell, M);
     launch_stress(l0, c.E, c.d_z, M, c.nu, c.cell, c.d_nodemap, (int64_t)c.h_nodemap.size(), c.d_iflag + 16, ctx->d_s6,
@@ -1638,6 +1655,7 @@ int sgld_stress(sgld_ctx *ctx, const double *U, double *nodal, double *vmn, doub
     const int64_t nn = (int64_t)c.h_nodemap.size(), ne = (int64_t)c.h_elemap.size();
     if (vme) launch_elem_vm(l0, ctx->d_s6, c.d_elemap, ne, ctx->d_vme, c.stream);
     CKL();
+    CK(cudaEventSynchronize(uploaded));   // U is not read any more
     if (nodal && (rc = download_rows(ctx, c.d_nodemap, nn, 6, ctx->d_s6, nodal))) return rc;
     if (vmn) {
         touch_pages(vmn, sizeof(double) * nn);
@@ -1662,11 +1680,16 @@ int sgld_principal_stress(sgld_ctx *ctx, const double *U, double *ps_node, doubl
         CK(dalloc(&ctx->d_vmn, (size_t)l0.nnode));
         CK(dalloc(&ctx->d_vme, (size_t)l0.nel));
     }
+    ScopedEvent uploaded;
+    CK(uploaded.make(cudaEventDisableTiming));
     if ((rc = upload_nodes(ctx, U, c.d_z))) return rc;
+    CK(cudaEventRecord(uploaded, c.stream));
     double M[48 * 24];
     stress_matrix(c.nu, c.cell, M);
     launch_stress(l0, c.E, c.d_z, M, c.nu, c.cell, c.d_nodemap, (int64_t)c.h_nodemap.size(), c.d_iflag + 16, ctx->d_s6,
                   ctx->d_vmn, c.stream);
+    CKL();
+    CK(cudaEventSynchronize(uploaded));   // U is not read any more
     // one output at a time through a temporary full-grid buffer (12 doubles
     // per node or 3 per element), gathered to the compact order on the device
     auto fetch = [&](int per, int64_t count, const int64_t *d_map, int64_t n, double *out, bool nodes) -> int {
