@@ -1805,9 +1805,9 @@ int pcg_dev(sgld_ctx *ctx, const sgld_solve_opts *o, sgld_solve_info *info) {
     const int nbv = reduce_blocks(nv);
     const double tol = o->tol;
     const int maxit = o->maxit;
-    cudaEvent_t e0, e1;
-    CK(cudaEventCreate(&e0));
-    CK(cudaEventCreate(&e1));
+    ScopedEvent e0, e1, tested;
+    CK(e0.make());
+    CK(e1.make());
     CK(cudaEventRecord(e0, c.stream));
     int nb = 0;
     launch_pcg_scalar(5, c.d_scal, c.d_iflag, c.d_part, 1, tol, maxit, c.stream);
@@ -1831,12 +1831,11 @@ int pcg_dev(sgld_ctx *ctx, const sgld_solve_opts *o, sgld_solve_info *info) {
     // V-cycle at the end instead of a gap of 20 us in every iteration (64 x 32 x 32: 163 us an
     // iteration with it, 143 without).  On a large grid that V-cycle would cost more than the gaps.
     const bool ahead = !prof && !o->history && l0.nnode <= 2000000;
-    cudaEvent_t tested = nullptr;
-    if (ahead) CK(cudaEventCreateWithFlags(&tested, cudaEventDisableTiming));
+    if (ahead) CK(tested.make(cudaEventDisableTiming));
     double *rr_part = c.d_part2;   // partials of r.r: the update reads those of p.q in d_part
-    cudaEvent_t pe[4] = {nullptr, nullptr, nullptr, nullptr};   // K*u start/end, precond start/end
+    ScopedEvent pe[4];   // K*u start/end, precond start/end
     if (prof)
-        for (auto &e : pe) CK(cudaEventCreate(&e));
+        for (auto &e : pe) CK(e.make());
     double kb_ms = 0.0, pc_ms = 0.0;
     int kb_n = 0;
     bool pc_pending = false;
@@ -1881,7 +1880,6 @@ int pcg_dev(sgld_ctx *ctx, const sgld_solve_opts *o, sgld_solve_info *info) {
             if (h_flag[2]) break;
         }
     }
-    if (tested) cudaEventDestroy(tested);
     CK(cudaEventRecord(e1, c.stream));
     if (prof) {
         CK(cudaStreamSynchronize(c.stream));
@@ -1890,7 +1888,6 @@ int pcg_dev(sgld_ctx *ctx, const sgld_solve_opts *o, sgld_solve_info *info) {
             cudaEventElapsedTime(&t, pe[2], pe[3]);
             pc_ms += t;
         }
-        for (auto &e : pe) cudaEventDestroy(e);
     }
     CK(cudaMemcpyAsync(h_flag, c.d_iflag, sizeof(int) * 4, cudaMemcpyDeviceToHost, c.stream));
     double sc[8];
@@ -1898,8 +1895,6 @@ int pcg_dev(sgld_ctx *ctx, const sgld_solve_opts *o, sgld_solve_info *info) {
     CK(cudaStreamSynchronize(c.stream));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     its = h_flag[0];
     // true residual in FP64
     launch_kbyu_f64(l0, c.E, c.d_x, c.d_q, nullptr, nullptr, c.stream);
