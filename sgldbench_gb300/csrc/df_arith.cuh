@@ -24,6 +24,11 @@ __device__ __forceinline__ df quick_two_sum(float a, float b) {
     const float s = __fadd_rn(a, b);
     return {s, __fsub_rn(b, __fsub_rn(s, a))};
 }
+// a + b exactly, as the rounded sum and its error (Knuth's TwoSum)
+__device__ __forceinline__ df two_sum(float a, float b) {
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
+}
 __device__ __forceinline__ df df_add(df a, df b) {
     const float s = __fadd_rn(a.hi, b.hi);
     const float bb = __fsub_rn(s, a.hi);

@@ -23,6 +23,7 @@
 
 #include "sgld_internal.cuh"
 #include "df_arith.cuh"
+#include "wide_sum.cuh"
 
 namespace sgld {
 
@@ -885,40 +886,20 @@ int coarse_factor_invert(Ctx &c) {
 // instead of 33.5; 256 x 128 x 128: 117 and 119) and than 2, or 1 to 4 of 16 or 32 warps (34 to 36).
 constexpr int CL_WARPS = 8, CL_CTAS = 4;
 
-// the warps' sums are added in FP64, or for FP32 in pairs of FP32 numbers: an FP64
-// operation holds a warp's scheduler for 64 clocks, and a chain of 16 conversions and adds
-// was a good part of an FP32 apply
-template <typename T>
-struct WideSum;
-template <>
-struct WideSum<double> {
-    double v;
-    __device__ __forceinline__ static WideSum of(double a) { return {a}; }
-    __device__ __forceinline__ WideSum operator+(WideSum b) const { return {v + b.v}; }
-    __device__ __forceinline__ double value() const { return v; }
-};
-template <>
-struct WideSum<float> {
-    df v;
-    __device__ __forceinline__ static WideSum of(float a) { return {{a, 0.f}}; }
-    __device__ __forceinline__ WideSum operator+(WideSum b) const { return {df_add(v, b.v)}; }
-    __device__ __forceinline__ float value() const { return v.hi; }
-};
-
 template <typename T, bool UPPER>
 __global__ void __cluster_dims__(1, CL_CTAS, 1) __launch_bounds__(32 * CL_WARPS)
     k_coarse_gemv(const T *__restrict__ M, const int *__restrict__ rows, const int *__restrict__ pos, int ndof,
                   const T *__restrict__ v, int n, T *__restrict__ y) {
     namespace cg = cooperative_groups;
     using S = WideSum<T>;
-    __shared__ T red[CL_WARPS][32];
+    __shared__ S red[CL_WARPS][32];
     __shared__ S sums[CL_CTAS][32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i0 = blockIdx.x * 32, i = i0 + lane, ii = min(i, n - 1);
     auto cluster = cg::this_cluster();
     auto started = cluster.barrier_arrive();   // every CTA of the cluster runs before its memory is written
     const int first = UPPER ? i0 : 0, last = UPPER ? n : min(n, i0 + 32);
-    T acc = T(0);
+    S acc = {};
     for (int jb = first + 32 * (w + CL_WARPS * (int)blockIdx.y); jb < last; jb += 32 * CL_WARPS * CL_CTAS) {
         const int jl = jb + lane;
         const T vl = (jl < n) ? (UPPER ? v[jl] : v[rows[jl]]) : T(0);
@@ -932,7 +913,7 @@ __global__ void __cluster_dims__(1, CL_CTAS, 1) __launch_bounds__(32 * CL_WARPS)
             // the other triangle holds the transpose
             if (UPPER ? jb + q >= i : jb + q <= i) a[q & 3] += m[q] * vq;
         }
-        acc += (a[0] + a[1]) + (a[2] + a[3]);
+        acc.add((a[0] + a[1]) + (a[2] + a[3]));
     }
     red[w][lane] = acc;
     __syncthreads();
@@ -940,7 +921,7 @@ __global__ void __cluster_dims__(1, CL_CTAS, 1) __launch_bounds__(32 * CL_WARPS)
     if (w == 0) {
         S t[CL_WARPS];
 #pragma unroll
-        for (int k = 0; k < CL_WARPS; ++k) t[k] = S::of(red[k][lane]);
+        for (int k = 0; k < CL_WARPS; ++k) t[k] = red[k][lane];
         cluster.map_shared_rank(&sums[0][0], 0)[32 * blockIdx.y + lane] =
             ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
     }
