@@ -252,11 +252,16 @@ __device__ __forceinline__ float sq4(float4 v, float acc) {
     return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, acc))));
 }
 
-__device__ __forceinline__ void store_partial(float acc, double *__restrict__ part) {
+__device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// v: lane 0's is the warp's
+__device__ __forceinline__ void store_partial(double v, double *__restrict__ part) {
     __shared__ double wred[UB / 32];
-    if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = (double)acc;
+    if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0.0;
@@ -295,7 +300,7 @@ __global__ void __launch_bounds__(UB, 4) k_icg_update(float *__restrict__ s, con
         s[i] = v;
         acc = fmaf(v, v, acc);
     }
-    store_partial(acc, part);
+    store_partial((double)warp_sum(acc), part);
 }
 
 // e += alpha d (the previous iteration's step, alpha still in place); then d = w + beta d
@@ -394,7 +399,9 @@ __global__ void __launch_bounds__(UB, 2) k_icg_update_runs(float *s, const float
         x.load(c, lane, src);
     }
     const float a = icg_coefficient<1>(sc, sum, nsum);
-    float acc = 0.f;
+    // a warp's even and odd chunks apart: 9728 sums over the grid, as long a chain in FP32 as with
+    // twice the warps
+    float acc = 0.f, other = 0.f;
     for (int64_t r = w0; r < nruns;) {
         const int64_t rv = runs[min(r + nw, nruns - 1)];
         if (c.single >= 0) {
@@ -414,11 +421,14 @@ __global__ void __launch_bounds__(UB, 2) k_icg_update_runs(float *s, const float
             if (k0 - lane >= c.n4) break;
             x.load(c, k0, src);
         }
+        const float last = acc;
+        acc = other;
+        other = last;
         if ((r += nw) >= nruns) break;
         c.take(rv, lane);
         x.load(c, lane, src);
     }
-    store_partial(acc, part);
+    store_partial((double)warp_sum(acc) + (double)warp_sum(other), part);
 }
 
 __global__ void __launch_bounds__(UB, 2) k_icg_dupdate_runs(float *e, float *d, const float *w,
