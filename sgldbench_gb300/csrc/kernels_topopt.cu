@@ -146,8 +146,8 @@ __global__ void k_topo_q(const double *__restrict__ x, const double *__restrict_
         q[e] = eact[e] ? x[e] * sqrt(-dc[e] / dv[e]) + 0.0 : 0.0;
 }
 
-// bisection state (device): [0] lo [1] hi [2] lmid [3] g [4] done [5] steps
-enum { OC_LO = 0, OC_HI = 1, OC_MID = 2, OC_G = 3, OC_DONE = 4, OC_STEPS = 5 };
+// bisection state (device): [0] lo [1] hi [2] lmid [3] g
+enum { OC_LO = 0, OC_HI = 1, OC_MID = 2, OC_G = 3 };
 
 // element flags of level 1: bit 0 active, bit 1 passive (kept solid by the
 // SIMP loop; TopOpti_GlobalVolumeConstraint.m:162,179)
@@ -159,8 +159,6 @@ __global__ void k_oc_init(double *__restrict__ st, const double *__restrict__ su
     st[OC_G] = sum_v[0] / nact - volfrac;
     st[OC_LO] = 0.0;
     st[OC_HI] = 1e9;
-    st[OC_DONE] = 0.0;
-    st[OC_STEPS] = 0.0;
     st[OC_MID] = 0.5e9;
 }
 
@@ -180,7 +178,7 @@ __global__ void __launch_bounds__(TB) k_oc_bisect(const double *__restrict__ x, 
                                                   int64_t n, double move, double *st, double *part0, double *part1,
                                                   int max_steps) {
     auto grid = cooperative_groups::this_grid();
-    __shared__ double lo, hi, mid, next, rs, steps;
+    __shared__ double lo, hi, mid, next, rs;
     __shared__ bool done;
     const int tid = threadIdx.x;
     const double g = st[OC_G];
@@ -188,7 +186,6 @@ __global__ void __launch_bounds__(TB) k_oc_bisect(const double *__restrict__ x, 
         lo = st[OC_LO];
         hi = st[OC_HI];
         mid = st[OC_MID];
-        steps = 0.0;
         done = false;
     }
     bool plain = true;
@@ -227,7 +224,6 @@ __global__ void __launch_bounds__(TB) k_oc_bisect(const double *__restrict__ x, 
                 lo = mid;
             else
                 hi = mid;
-            steps += 1.0;
         }
         __syncthreads();
     }
@@ -235,8 +231,6 @@ __global__ void __launch_bounds__(TB) k_oc_bisect(const double *__restrict__ x, 
         st[OC_LO] = lo;
         st[OC_HI] = hi;
         st[OC_MID] = mid;
-        st[OC_STEPS] = steps;
-        st[OC_DONE] = done ? 1.0 : 0.0;
     }
 }
 

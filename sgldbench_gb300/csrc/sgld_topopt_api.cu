@@ -26,7 +26,7 @@ int tfail(sgld_ctx *ctx, int code, const std::string &m) {
         if (e_ != cudaSuccess) return tfail(ctx, SGLD_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-enum { OC_MID = 2, OC_G = 3, OC_DONE = 4, OC_STEPS = 5, T_SHARP = 8, T_C = 9, T_CHANGE = 10, T_VOL = 11 };
+enum { OC_G = 3, T_SHARP = 8, T_C = 9, T_CHANGE = 10, T_VOL = 11 };
 
 int ensure_topo(sgld_ctx *ctx) {
     Ctx &c = ctx->c;
