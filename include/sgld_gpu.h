@@ -446,7 +446,7 @@ int sgld_topopt_projected(sgld_ctx *ctx, const sgld_topopt_projected_opts *opts,
 /* FEA_StressAnalysis.m:17-60 and FEA_ComputePerElementVonMisesStress.m:10-19:
  * nodal Cartesian stress (numNodes x 6, row-major [xx yy zz yz zx xy]), nodal
  * von Mises and per-element von Mises with the reference's final .^(1/2).
- * Any output may be NULL. */
+ * Any output may be NULL, and an output may overlap U. */
 int sgld_stress(sgld_ctx *ctx, const double *U, double *nodal_stress, double *vm_node, double *vm_elem);
 /* The von Mises part of sgld_stress alone (FEA_ComputePerElementVonMisesStress.m:10-19,
  * FEA_ComputeVonMisesStress.m:1-7): per element (numElements) and per node
@@ -460,7 +460,7 @@ int sgld_vonmises(sgld_ctx *ctx, const double *U, double *vm_elem, double *vm_no
  * dir_elem (numElements x 3, row-major): per element, the principal direction
  * of largest |l| of the centroid stress
  * (Common_ExtractDominantDirectionsFromPrincipalStressDirections.m:9-38).
- * Either output may be NULL. */
+ * Either output may be NULL, and an output may overlap U. */
 int sgld_principal_stress(sgld_ctx *ctx, const double *U, double *ps_node, double *dir_elem);
 
 /* ---- the learned warm start's network on its own ------------------------------

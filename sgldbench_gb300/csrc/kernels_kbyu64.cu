@@ -429,7 +429,10 @@ __global__ void __launch_bounds__(k64::MAX_THREADS, 1)
 // tile, and the last one to start decides: there the cost is the active share of
 // the work, spread evenly, plus one whole CTA.  (With the solid grid's rule the 384 x
 // 192 x 192 blob shape took 3.69 ms, with this one 2.01; the fixed 32 x 8 x 16 tile
-// 3.28.)  At most SGLD_NOALLOC_MAX_CTAS CTAs, the scratch of the allocation-free
+// 3.28.)  The double-float form takes the same tile and map, although latency binds it rather
+// than the FP64 pipe: the rule's choice is the best of a sweep for it too on 256 x 128 x 128 (523 us),
+// on the 384 x 192 x 192 blob shape another tile would be 10 % faster (18 x 7 x 13: 850 us, the choice
+// 16 x 12 x 15: 951).  At most SGLD_NOALLOC_MAX_CTAS CTAs, the scratch of the allocation-free
 // call, where the grid allows it.
 void kbyu64_pick_tile(Level &l) {
     const int NY = l.ny + 1, NX = l.nx + 1, NZ = l.nz + 1;

@@ -333,7 +333,7 @@ __global__ void k_prolong_smooth(const T *__restrict__ xc, const T *__restrict__
 // a plane are the lower 4 of the next (a CTA marches through zp planes), and the
 // interpolation is sums of 1, 2, 4 or 8 corners, axis by axis, scaled once.
 // Indices are 32-bit.  Same result as k_prolong_smooth up to the order of the sums.
-// All of a batch's loads (r, 1/D and flags of the cell's 8 fine nodes in FP32, of
+// All of a batch's loads (r, 2 omega / D and flags of the cell's 8 fine nodes in FP32, of
 // 4 in FP64) are issued before the first is used, at clamped positions for the
 // nodes past the grid; with a branch around each fine node they went out node by
 // node, eight memory latencies per cell.  Finest level: FP32 384 x 192 x 192 blobs 76 ->

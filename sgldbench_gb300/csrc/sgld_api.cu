@@ -1828,8 +1828,11 @@ int pcg_dev(sgld_ctx *ctx, const sgld_solve_opts *o, sgld_solve_info *info) {
     const bool prof = o->profile != 0;
     // The stopping test's flags come over a stream of their own while this one goes on with
     // the V-cycle and the new direction, which a solve that has stopped does not need: one
-    // V-cycle at the end instead of a gap of 20 us in every iteration (64 x 32 x 32: 163 us an
-    // iteration with it, 143 without).  On a large grid that V-cycle would cost more than the gaps.
+    // V-cycle at the end instead of a gap of 12 us in every iteration.  From zero to 1e-9, ms
+    // without and with: 64 x 32 x 32 10.2 and 9.6 (53 iterations), 192 x 96 x 96 90.1 and 88.9 (93),
+    // and on larger grids as much in all (256 x 128 x 128 183.0 and 181.9, 95).  But a V-cycle costs
+    // 0.06, 0.18 and 0.35 ms there, the gaps of 5, 15 and 29 iterations, so a warm-started
+    // solve of fewer would lose: the limit is set where that is 15.
     const bool ahead = !prof && !o->history && l0.nnode <= 2000000;
     if (ahead) CK(tested.make(cudaEventDisableTiming));
     double *rr_part = c.d_part2;   // partials of r.r: the update reads those of p.q in d_part
