@@ -882,8 +882,8 @@ int coarse_factor_invert(Ctx &c) {
 // memory cost two more launches and a memset of x per apply: the FP32 V-cycle of
 // 384 x 192 x 192 blobs (1300 rows) went from 214 to 193 us, of 256 x 128 x 128
 // (3888 rows) from 151 to 136, of 96 x 48 x 48 from 63 to 53.  An apply of a few thousand rows
-// is a chain of latencies: 4 CTAs per cluster are better than 8 (96 x 48 x 48: 30 us a cycle
-// instead of 33.5; 256 x 128 x 128: 117 and 119) and than 2, or 1 to 4 of 16 or 32 warps (34 to 36).
+// is a chain of latencies: 4 CTAs per cluster are better than 8 (96 x 48 x 48: 3.5 us less
+// a cycle, 256 x 128 x 128: 2) and than 2, or 1 to 4 of 16 or 32 warps (4 to 6 less on 96 x 48 x 48).
 constexpr int CL_WARPS = 8, CL_CTAS = 4;
 
 template <typename T, bool UPPER>
