@@ -599,17 +599,19 @@ void touch_pages(void *p, size_t bytes) {
     for (size_t i = 0; i < bytes; i += page) c[i] = 0;
 }
 
-// rows of `per` doubles of a full-grid array at map's entries -> the compact host array h,
-// gathered on the device through d_tmp (3 nnode doubles) piece by piece
-int download_rows(sgld_ctx *ctx, const int64_t *d_map, int64_t n, int per, const double *d_full, double *h) {
+// rows of `per` doubles of a full-grid array of `rows` rows at map's n entries -> the compact
+// host array h, gathered on the device through d_tmp (3 nnode doubles) piece by piece; as they
+// are where every row is one of them
+int download_rows(sgld_ctx *ctx, const int64_t *d_map, int64_t n, int64_t rows, int per, const double *d_full, double *h) {
     Ctx &c = ctx->c;
-    const int64_t most = std::max<int64_t>(1, 3 * c.lv[0].nnode / per);
+    const bool all = n == rows;
+    const int64_t most = all ? n : std::max<int64_t>(1, 3 * c.lv[0].nnode / per);
     touch_pages(h, sizeof(double) * per * n);   // while the kernels run
     for (int64_t i = 0; i < n; i += most) {
         const int64_t k = std::min(most, n - i);
-        launch_gather_rows(d_map + i, k, per, d_full, c.d_tmp, c.stream);
+        if (!all) launch_gather_rows(d_map + i, k, per, d_full, c.d_tmp, c.stream);
         CKL();
-        CK(cudaMemcpyAsync(h + per * i, c.d_tmp, sizeof(double) * per * k, cudaMemcpyDeviceToHost, c.stream));
+        CK(cudaMemcpyAsync(h + per * i, all ? d_full : c.d_tmp, sizeof(double) * per * k, cudaMemcpyDeviceToHost, c.stream));
     }
     CK(cudaStreamSynchronize(c.stream));
     return SGLD_OK;
@@ -1656,7 +1658,7 @@ int sgld_stress(sgld_ctx *ctx, const double *U, double *nodal, double *vmn, doub
     if (vme) launch_elem_vm(l0, ctx->d_s6, c.d_elemap, ne, ctx->d_vme, c.stream);
     CKL();
     CK(cudaEventSynchronize(uploaded));   // U is not read any more
-    if (nodal && (rc = download_rows(ctx, c.d_nodemap, nn, 6, ctx->d_s6, nodal))) return rc;
+    if (nodal && (rc = download_rows(ctx, c.d_nodemap, nn, l0.nnode, 6, ctx->d_s6, nodal))) return rc;
     if (vmn) {
         touch_pages(vmn, sizeof(double) * nn);
         CK(cudaMemcpyAsync(vmn, ctx->d_vmn, sizeof(double) * nn, cudaMemcpyDeviceToHost, c.stream));
@@ -1690,22 +1692,23 @@ int sgld_principal_stress(sgld_ctx *ctx, const double *U, double *ps_node, doubl
                   ctx->d_vmn, c.stream);
     CKL();
     CK(cudaEventSynchronize(uploaded));   // U is not read any more
-    // one output at a time through a temporary full-grid buffer (12 doubles
+    // one output after the other through a temporary full-grid buffer (12 doubles
     // per node or 3 per element), gathered to the compact order on the device
-    auto fetch = [&](int per, int64_t count, const int64_t *d_map, int64_t n, double *out, bool nodes) -> int {
-        double *d_buf = nullptr;
-        CK(dalloc(&d_buf, (size_t)per * count));
-        if (nodes)
-            launch_principal(l0, ctx->d_s6, d_buf, nullptr, c.stream);
-        else
-            launch_principal(l0, ctx->d_s6, nullptr, d_buf, c.stream);
-        const int r = download_rows(ctx, d_map, n, per, d_buf, out);
-        if (r) cudaStreamSynchronize(c.stream);
-        cudaFree(d_buf);
-        return r;
-    };
-    if (ps_node && (rc = fetch(12, l0.nnode, c.d_nodemap, (int64_t)c.h_nodemap.size(), ps_node, true))) return rc;
-    if (dir_elem && (rc = fetch(3, l0.nel, c.d_elemap, (int64_t)c.h_elemap.size(), dir_elem, false))) return rc;
+    struct Buffer {
+        double *p = nullptr;
+        ~Buffer() {
+            if (p) cudaFree(p);
+        }
+    } buf;
+    CK(dalloc(&buf.p, std::max(ps_node ? 12 * (size_t)l0.nnode : 0, dir_elem ? 3 * (size_t)l0.nel : 0)));
+    if (ps_node) {
+        launch_principal(l0, ctx->d_s6, buf.p, nullptr, c.stream);
+        if ((rc = download_rows(ctx, c.d_nodemap, (int64_t)c.h_nodemap.size(), l0.nnode, 12, buf.p, ps_node))) return rc;
+    }
+    if (dir_elem) {
+        launch_principal(l0, ctx->d_s6, nullptr, buf.p, c.stream);
+        if ((rc = download_rows(ctx, c.d_elemap, (int64_t)c.h_elemap.size(), l0.nel, 3, buf.p, dir_elem))) return rc;
+    }
     return SGLD_OK;
 }
 
